@@ -68,10 +68,11 @@ LaplaceEngine::LaplaceEngine(const LaplaceSpec& spec, int max_batch, cudaStream_
     return it - spec_.rowidx.begin();
   };
   std::vector<unsigned char> pdiag(nnz_, 0);
-  std::vector<int> qri(nnz_);
+  std::vector<int> qri(nnz_), qci(nnz_);
   for (int64_t c = 0; c < n; ++c)
     for (int64_t p = spec_.colptr[c]; p < spec_.colptr[c + 1]; ++p) {
       qri[p] = (int)spec_.rowidx[p];
+      qci[p] = (int)c;
       if (spec_.rowidx[p] == c) pdiag[p] = 1;
     }
   for (int64_t c = 0; c < n; ++c)
@@ -146,6 +147,16 @@ LaplaceEngine::LaplaceEngine(const LaplaceSpec& spec, int max_batch, cudaStream_
         atv[fill[aci[a]]++] = av[a];
       }
   }
+  // columns summed by a CTA of their own (k_newton_rhs, k_spmv_at), lanes per other column: a warp
+  // where a column has more than 48 entries on average (the dense augmented form), else 8 lanes
+  wide_cols_ = nnz_ + (int64_t)aci.size() > 48 * n;
+  std::vector<int> longc;
+  for (int64_t j = 0; j < n; ++j)
+    if ((spec_.colptr[j + 1] - spec_.colptr[j]) + (spec_.identity_a ? 0 : atp[j + 1] - atp[j]) >
+        long_col(wide_cols_ ? 32 : 8))
+      longc.push_back((int)j);
+  nlong_ = (int)longc.size();
+  if (!longc.empty()) longc_.upload(longc, stream_);
 
   const auto t4 = std::chrono::steady_clock::now();
   comp_.upload(spec_.comp, stream_);
@@ -154,6 +165,7 @@ LaplaceEngine::LaplaceEngine(const LaplaceSpec& spec, int max_batch, cudaStream_
   if (!spec_.p2.empty()) p2_.upload(spec_.p2, stream_);
   qcp_.upload(spec_.colptr, stream_);
   qri_.upload(qri, stream_);
+  qci_.upload(qci, stream_);
   pdiag_.upload(pdiag, stream_);
   cptr_.upload(cptr, stream_);
   cobs_.upload(cobs, stream_);
@@ -190,8 +202,7 @@ LaplaceEngine::LaplaceEngine(const LaplaceSpec& spec, int max_batch, cudaStream_
   sig_.alloc(B * nnz_);
   red_.alloc(B * 4 * (spec_.ncomp + 1) + B * 8);
   {
-    const int64_t maxch = std::max<int64_t>({1, (nnz_ + kRedChunk - 1) / kRedChunk, (nobs + kRedChunk - 1) / kRedChunk,
-                                             (n + kColChunk - 1) / kColChunk});
+    const int64_t maxch = std::max<int64_t>({1, (nnz_ + kRedChunk - 1) / kRedChunk, (nobs + kRedChunk - 1) / kRedChunk});
     gpart_.alloc(B * maxch * 9);
     gtick_.alloc(B);
     INLA_CUDA(cudaMemsetAsync(gtick_.p, 0, sizeof(unsigned) * B, stream_));
@@ -468,6 +479,33 @@ void LaplaceEngine::fill_factor(int B, bool posterior, double diag_add) {
                    posterior ? w_.p : nullptr, spec_.nobs, B, posterior ? 0 : B, diag_add);
 }
 
+void LaplaceEngine::newton_rhs(int B, const double* d_x) {
+  const int64_t n = spec_.n;
+  const int64_t* atp = spec_.identity_a ? nullptr : atp_.p;
+  const unsigned nb = cdiv(B, kColB);
+  auto go = [&](auto kern, unsigned ctas, int threads) {
+    kern<<<dim3(ctas, nb), threads, 0, stream_>>>((int)n, spec_.ncomp, 1, nullptr, qcp_.p, qri_.p, comp_.p, nnz_,
+                                                  coef_.p, atp, ati_.p, atv_.p, spec_.nobs, grad_.p, d_x, step_.p, B,
+                                                  longc_.p);
+    ++launches_;
+  };
+  if (wide_cols_) go(k_newton_rhs<32, 256>, cdiv(n, 256 / 32), 256);
+  else go(k_newton_rhs<8, 256>, cdiv(n, 256 / 8), 256);
+  if (nlong_ > 0) go(k_newton_rhs<0, kLongThreads>, nlong_, kLongThreads);
+}
+
+void LaplaceEngine::spmv_at(int B, const double* d_v, double* d_u) {
+  const int64_t n = spec_.n;
+  auto go = [&](auto kern, unsigned ctas, int threads) {
+    kern<<<dim3(ctas, B), threads, 0, stream_>>>((int)n, spec_.identity_a ? nullptr : atp_.p, ati_.p, atv_.p,
+                                                 spec_.nobs, d_v, d_u, qcp_.p, longc_.p);
+    ++launches_;
+  };
+  if (wide_cols_) go(k_spmv_at<32, 256>, cdiv(n, 256 / 32), 256);
+  else go(k_spmv_at<8, 256>, cdiv(n, 256 / 8), 256);
+  if (nlong_ > 0) go(k_spmv_at<0, kLongThreads>, nlong_, kLongThreads);
+}
+
 void LaplaceEngine::eval_lik(int B, const double* d_xsrc) {
   const int64_t nobs = spec_.nobs;
   k_spmv_a<<<dim3(grid1(nobs), B), 256, 0, stream_>>>(nobs, (int)spec_.n, spec_.identity_a ? nullptr : acp_.p, aci_.p,
@@ -594,17 +632,13 @@ void LaplaceEngine::eval(int B, const double* coef, const double* p1scale, int f
   // ---- mode --------------------------------------------------------------------
   std::vector<int> prior_status(B);
   INLA_CUDA(cudaMemsetAsync(x_.p, 0, sizeof(double) * B * n, stream_));
-  const int64_t at_null = 0;
-  (void)at_null;
-  const int64_t* atp = spec_.identity_a ? nullptr : atp_.p;
   auto newton_system = [&](const double* d_x) {
     eval_lik(B, d_x);
     fill_factor(B, true, 0.0);
-    k_newton_rhs<<<dim3(grid1(n), B), 256, 0, stream_>>>((int)n, T, qcp_.p, qri_.p, comp_.p, nnz_, coef_.p, atp,
-                                                         ati_.p, atv_.p, nobs, grad_.p, d_x, step_.p);
+    newton_rhs(B, d_x);
     F_->solve(step_.p, n, B);
-    k_step_stats<256><<<B, 256, 0, stream_>>>((int)n_, n, step_.p, stats_.p);
-    launches_ += 2;
+    k_step_stats<1024><<<B, 1024, 0, stream_>>>((int)n_, n, step_.p, stats_.p);
+    ++launches_;
   };
   std::vector<double> st(2 * B);
   std::vector<int> bad(B), pst(B);
@@ -626,11 +660,10 @@ void LaplaceEngine::eval(int B, const double* coef, const double* p1scale, int f
                      Bp + B, Bp, 0.0);
     INLA_CUDA(cudaMemcpyAsync(ldp_.p, F_->d_logdet(), sizeof(double) * Bp, cudaMemcpyDeviceToDevice, stream_));
     INLA_CUDA(cudaMemcpyAsync(stp_.p, F_->d_status(), sizeof(int) * Bp, cudaMemcpyDeviceToDevice, stream_));
-    k_newton_rhs<<<dim3(grid1(n), B), 256, 0, stream_>>>((int)n, T, qcp_.p, qri_.p, comp_.p, nnz_, coef_.p, atp,
-                                                         ati_.p, atv_.p, nobs, grad_.p, x_.p, step_.p);
+    newton_rhs(B, x_.p);
     F_->solve(step_.p, n, B, post0);
-    k_step_stats<256><<<B, 256, 0, stream_>>>((int)n_, n, step_.p, stats_.p);
-    launches_ += 2;
+    k_step_stats<1024><<<B, 1024, 0, stream_>>>((int)n_, n, step_.p, stats_.p);
+    ++launches_;
     INLA_CUDA(cudaMemcpyAsync(x_.p, step_.p, sizeof(double) * B * n, cudaMemcpyDeviceToDevice, stream_));
     project(B, x_.p, true);  // inference.rs:867-869
     fetch();
@@ -698,7 +731,7 @@ void LaplaceEngine::eval(int B, const double* coef, const double* p1scale, int f
       ++launches_;
       project(B, xt_.p);
       // max |x_trial - x| of the accepted (projected) point (inference.rs:917-922)
-      k_max_abs_diff<256><<<B, 256, 0, stream_>>>((int)n_, n, xt_.p, x_.p, mdiff_.p);
+      k_max_abs_diff<1024><<<B, 1024, 0, stream_>>>((int)n_, n, xt_.p, x_.p, mdiff_.p);
       ++launches_;
       INLA_CUDA(cudaMemcpyAsync(x_.p, xt_.p, sizeof(double) * B * n, cudaMemcpyDeviceToDevice, stream_));
       std::vector<double> mdiff(B);
@@ -725,7 +758,7 @@ void LaplaceEngine::eval(int B, const double* coef, const double* p1scale, int f
   // ---- marginal likelihood pieces (inference.rs:953-972) ------------------------
   eval_lik(B, x_.p);
   k_row_sum_g<<<dim3(nchunks(nobs, kRedChunk), B), 256, 0, stream_>>>(nobs, logp_.p, gpart_.p, gtick_.p, d_scal);
-  k_quad_forms_g<<<dim3(nchunks(n, kColChunk), B), 256, 0, stream_>>>((int)n, T, qcp_.p, qri_.p, comp_.p, nnz_,
+  k_quad_forms_g<<<dim3(nchunks(nnz_, kRedChunk), B), 256, 0, stream_>>>((int)n, T, qri_.p, qci_.p, comp_.p, nnz_,
                                                                       coef_.p, nullptr, x_.p, gpart_.p, gtick_.p,
                                                                       d_xMx);
   launches_ += 2;
@@ -758,11 +791,11 @@ void LaplaceEngine::eval(int B, const double* coef, const double* p1scale, int f
         k_predictor_var<<<dim3(grid1(nobs), B), 256, 0, stream_>>>(nobs, acp_.p, av_.p, oppos_.p, opptr_.p, sig_.p,
                                                                    nnz_, tmp_o_.p);
         k_mul<<<dim3(grid1(nobs), B), 256, 0, stream_>>>(nobs, tmp_o_.p, dw_.p, tmp_o_.p);
-        k_spmv_at<<<dim3(grid1(n), B), 256, 0, stream_>>>((int)n, atp, ati_.p, atv_.p, nobs, tmp_o_.p, tmp_n_.p);
+        spmv_at(B, tmp_o_.p, tmp_n_.p);
         F_->solve(tmp_n_.p, n, B);
-        k_quad_forms_g<<<dim3(nchunks(n, kColChunk), B), 256, 0, stream_>>>(
-            (int)n, T, qcp_.p, qri_.p, comp_.p, nnz_, coef_.p, tmp_n_.p, x_.p, gpart_.p, gtick_.p, d_zMx);
-        launches_ += 4;
+        k_quad_forms_g<<<dim3(nchunks(nnz_, kRedChunk), B), 256, 0, stream_>>>(
+            (int)n, T, qri_.p, qci_.p, comp_.p, nnz_, coef_.p, tmp_n_.p, x_.p, gpart_.p, gtick_.p, d_zMx);
+        launches_ += 3;
       }
     }
   }

@@ -116,6 +116,8 @@ class LaplaceEngine {
  private:
   void fill_factor(int B, bool posterior, double diag_add);
   void eval_lik(int B, const double* d_xsrc);
+  void newton_rhs(int B, const double* d_x);               // step_ <- A^T grad_ - Q x
+  void spmv_at(int B, const double* d_v, double* d_u);     // u <- A^T v
   void augment_constraints();         // host, once: C, C^T, (C C^T)^-1, then one of
   void augment_dense();               //   widen the pattern by supp(C^T C), append kappa C^T C
   void augment_bordered();            //   border the pattern with C and -I/kappa (order n + k)
@@ -141,7 +143,9 @@ class LaplaceEngine {
   // static device data
   DBuf<double> comp_, y_, p1_, p2_, av_, atv_, cprod_;
   DBuf<int64_t> qcp_, acp_, atp_, opptr_, oppos_;
-  DBuf<int> qri_, aci_, ati_, cptr_, cobs_;
+  DBuf<int> qri_, qci_, aci_, ati_, cptr_, cobs_, longc_;
+  int nlong_ = 0;           // columns of more than long_col(lanes) entries (longc_)
+  bool wide_cols_ = false;  // a warp per column in the Newton right-hand side (8 lanes otherwise)
   DBuf<unsigned char> pdiag_;
   // per-batch work
   DBuf<double> coef_, p1s_, x_, xt_, step_, eta_, logp_, grad_, w_, dw_, var_, sig_, red_, stats_, alpha_, tmp_n_,

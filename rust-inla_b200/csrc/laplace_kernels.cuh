@@ -62,48 +62,144 @@ __global__ void k_eval_lik(int fam, int64_t nobs, const double* __restrict__ eta
   if (flag) atomicOr(bad + b, flag);
 }
 
-// rhs[b][j] = sum_a A[a, j] g[b][a] - (Q x)[b][j]; Q values = sum_t coef[b][t] comp[t][p]
-// on the full symmetric pattern (column j of Q = row j). A^T in CSR (atp, ati, atv).
-__global__ void k_newton_rhs(int n, int ncomp, const int64_t* __restrict__ qcp, const int* __restrict__ qri,
-                             const double* __restrict__ comp, int64_t nnz, const double* __restrict__ coef,
-                             const int64_t* __restrict__ atp, const int* __restrict__ ati,
-                             const double* __restrict__ atv, int64_t nobs, const double* __restrict__ g,
-                             const double* __restrict__ x, double* __restrict__ rhs) {
-  const int b = blockIdx.y;
-  const double* xb = x + (int64_t)b * n;
-  const double* gb = g + (int64_t)b * nobs;
-  const double* cb = coef + (int64_t)b * ncomp;
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-    double s = 0.0;
-    if (atp) {
-      for (int64_t a = atp[j]; a < atp[j + 1]; ++a) s += atv[a] * gb[ati[a]];
-    } else {
-      s = gb[j];
+// Column-wise sums of the Newton right-hand side and of A^T v. Latent models carry a few columns
+// that every observation touches (intercept, covariates, constraint borders): with one thread per
+// column such a column of 24 000 entries took 10 ms while the rest of the kernel took 0.05 ms. So
+// short columns are summed by L lanes each (strided entries, shuffle tree; NT = 256) and a column of
+// more than long_col(L) entries (host list `longc`) by a CTA of kLongThreads in a launch of its own
+// (L = 0). The split of a column depends on its own length only, so its sum does not depend on the
+// batch or on the other columns. What bounds a long column is the chain index -> x per entry, hence
+// 1024 threads for it (256: 105 us for group 24x24x14); two entries in flight per thread, four spill. With 8 lanes the
+// line lies at 128 entries: at 1024 the intercepts of models with 200 to 340 observations (600 to
+// 1024 entries) stayed with 8 lanes and set the kernel's time (226 us).
+// Group 24x24x14, B = 2: 10.4 ms -> 57 us; 96 uneven models, B = 2: 5.0 ms -> 96 us; SPDE 200^2, B = 7
+// (no long column: 8 lanes per column instead of one thread, components read once per four
+// problems): 82 -> 37 us.
+constexpr int kLongThreads = 1024;
+__host__ __device__ constexpr int wide_red(int lanes, int nt) { return lanes == 0 ? nt : 1; }
+__host__ __device__ constexpr int long_col(int lanes) { return lanes <= 8 ? 16 * lanes : 1024; }
+constexpr int kColB = 4;  // problems per CTA: an entry's component values are read once for all of them
+
+// Sum of v over the L lanes of a group (L a power of two <= 32); every lane of the warp takes part.
+template <int L>
+__device__ __forceinline__ double lane_sum(double v) {
+#pragma unroll
+  for (int o = L / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+template <int NT>
+__device__ __forceinline__ double block_sum(double v, double* red);
+
+// rhs[b][j] = sum_a A[a, j] g[b][a] - (Q x)[b][j]; Q values = sum_t coef[b][seg(j)][t] comp[t][p]
+// on the full symmetric pattern (column j of Q = row j; seg == nullptr: one model, G = 1).
+// A^T in CSR (atp, ati, atv; atp == nullptr: identity).
+template <int L, int NT>
+__global__ void __launch_bounds__(NT) k_newton_rhs(int n, int ncomp, int G, const int* __restrict__ segc,
+                                                    const int64_t* __restrict__ qcp, const int* __restrict__ qri,
+                                                    const double* __restrict__ comp, int64_t nnz,
+                                                    const double* __restrict__ coef, const int64_t* __restrict__ atp,
+                                                    const int* __restrict__ ati, const double* __restrict__ atv,
+                                                    int64_t nobs, const double* __restrict__ g,
+                                                    const double* __restrict__ x, double* __restrict__ rhs, int B,
+                                                    const int* __restrict__ longc) {
+  __shared__ double red[wide_red(L, NT)];
+  const int b0 = blockIdx.y * kColB, nb = min(kColB, B - b0);
+  constexpr bool wide = L == 0;
+  constexpr int GL = wide ? NT : L;  // threads per column
+  constexpr int U = wide ? 2 : 1;    // entries of Q in flight per thread
+  const int lane = threadIdx.x & (GL - 1);
+  const int j = wide ? longc[blockIdx.x] : (int)(blockIdx.x * (NT / GL) + threadIdx.x / GL);
+  double acc[kColB] = {0.0, 0.0, 0.0, 0.0};
+  bool mine = j < n;
+  if (mine) {
+    const int64_t p0 = qcp[j], p1 = qcp[j + 1];
+    const int64_t a0 = atp ? atp[j] : 0, a1 = atp ? atp[j + 1] : 0;
+    if (!wide && (p1 - p0) + (a1 - a0) > long_col(L)) mine = false;  // left to a CTA of its own
+    if (mine) {
+      const double* gb = g + (int64_t)b0 * nobs;
+      const double* xb = x + (int64_t)b0 * n;
+      const double* cb = coef + ((int64_t)b0 * G + (segc ? segc[j] : 0)) * ncomp;
+      if (!atp && lane == 0) {
+#pragma unroll
+        for (int q = 0; q < kColB; ++q)
+          if (q < nb) acc[q] = gb[(int64_t)q * nobs + j];
+      }
+#pragma unroll 4
+      for (int64_t a = a0 + lane; a < a1; a += GL) {
+        const double v = atv[a];
+        const int i = ati[a];
+#pragma unroll
+        for (int q = 0; q < kColB; ++q)
+          if (q < nb) acc[q] += v * gb[(int64_t)q * nobs + i];
+      }
+      for (int64_t p = p0 + lane; p < p1; p += U * GL) {
+        int r[U];
+        double v[U][kColB];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          r[u] = p + u * GL < p1 ? qri[p + u * GL] : -1;
+#pragma unroll
+          for (int q = 0; q < kColB; ++q) v[u][q] = 0.0;
+        }
+#pragma unroll 2
+        for (int t = 0; t < ncomp; ++t) {
+          double c[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u) c[u] = r[u] >= 0 ? comp[(int64_t)t * nnz + p + u * GL] : 0.0;
+#pragma unroll
+          for (int q = 0; q < kColB; ++q)
+            if (q < nb) {
+              const double w = cb[(int64_t)q * G * ncomp + t];
+#pragma unroll
+              for (int u = 0; u < U; ++u) v[u][q] += w * c[u];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (r[u] >= 0) {
+#pragma unroll
+            for (int q = 0; q < kColB; ++q)
+              if (q < nb) acc[q] -= v[u][q] * xb[(int64_t)q * n + r[u]];
+          }
+      }
     }
-    double qx = 0.0;
-    for (int64_t p = qcp[j]; p < qcp[j + 1]; ++p) {
-      double v = 0.0;
-      for (int t = 0; t < ncomp; ++t) v += cb[t] * comp[(int64_t)t * nnz + p];
-      qx += v * xb[qri[p]];
-    }
-    rhs[(int64_t)b * n + j] = s - qx;
+  }
+#pragma unroll
+  for (int q = 0; q < kColB; ++q) {
+    if (q >= nb) break;  // uniform over the CTA
+    const double s = wide ? block_sum<NT>(acc[q], red) : lane_sum<wide ? 32 : L>(acc[q]);
+    if (mine && lane == 0) rhs[(int64_t)(b0 + q) * n + j] = s;
   }
 }
 
-// u[b][j] = sum_a A[a,j] v[b][a]   (A^T in CSR)
-__global__ void k_spmv_at(int n, const int64_t* __restrict__ atp, const int* __restrict__ ati,
-                          const double* __restrict__ atv, int64_t nobs, const double* __restrict__ v,
-                          double* __restrict__ u) {
+// u[b][j] = sum_a A[a,j] v[b][a]   (A^T in CSR; atp == nullptr: identity)
+template <int L, int NT>
+__global__ void __launch_bounds__(NT) k_spmv_at(int n, const int64_t* __restrict__ atp, const int* __restrict__ ati,
+                                                 const double* __restrict__ atv, int64_t nobs,
+                                                 const double* __restrict__ v, double* __restrict__ u,
+                                                 const int64_t* __restrict__ qcp, const int* __restrict__ longc) {
+  __shared__ double red[wide_red(L, NT)];
   const int b = blockIdx.y;
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-    double s = 0.0;
-    if (atp) {
-      for (int64_t a = atp[j]; a < atp[j + 1]; ++a) s += atv[a] * v[(int64_t)b * nobs + ati[a]];
-    } else {
-      s = v[(int64_t)b * nobs + j];
+  const double* vb = v + (int64_t)b * nobs;
+  constexpr bool wide = L == 0;
+  constexpr int GL = wide ? NT : L;  // threads per column
+  const int lane = threadIdx.x & (GL - 1);
+  const int j = wide ? longc[blockIdx.x] : (int)(blockIdx.x * (NT / GL) + threadIdx.x / GL);
+  double s = 0.0;
+  bool mine = j < n;
+  if (mine && atp) {
+    const int64_t a0 = atp[j], a1 = atp[j + 1];
+    if (!wide && (qcp[j + 1] - qcp[j]) + (a1 - a0) > long_col(L)) mine = false;
+    if (mine) {
+#pragma unroll 4
+      for (int64_t a = a0 + lane; a < a1; a += GL) s += atv[a] * vb[ati[a]];
     }
-    u[(int64_t)b * n + j] = s;
+  } else if (mine && lane == 0) {
+    s = vb[j];  // a long column of Q is written by both launches, with the same value
   }
+  s = wide ? block_sum<NT>(s, red) : lane_sum<wide ? 32 : L>(s);
+  if (mine && lane == 0) u[(int64_t)b * n + j] = s;
 }
 
 __global__ void k_mul(int64_t len, const double* a, const double* b, double* c) {  // c may alias a
@@ -221,12 +317,13 @@ __global__ void __launch_bounds__(256) k_gauss_dll_g(int64_t nobs, const double*
   grid_reduce_store<1>(a, 1, false, part, ticket, out, 1, 0);
 }
 
-// x^T M_t x (t < ncomp) and x^T Q x = sum_t coef_t x^T M_t x, columns in chunks of
-// kColChunk: out[b][0] = x^T Q x, out[b][1+t] = x^T M_t x. With z != nullptr the
-// bilinear forms z^T M_t x go to out[b][t] (no total).
-constexpr int kColChunk = 1024;  // 256 threads x 4 columns
-__global__ void __launch_bounds__(256) k_quad_forms_g(int n, int ncomp, const int64_t* __restrict__ qcp,
-                                                      const int* __restrict__ qri, const double* __restrict__ comp,
+// x^T M_t x (t < ncomp) and x^T Q x = sum_t coef_t x^T M_t x over the pattern's entries (qri, qci:
+// row and column of every entry) in chunks of kRedChunk: out[b][0] = x^T Q x, out[b][1+t] =
+// x^T M_t x. With z != nullptr the bilinear forms z^T M_t x go to out[b][t] (no total). Entries, not
+// columns, are dealt out: coalesced, and a dense column costs what its entries cost (one thread per
+// column: 84 us for SPDE 200^2 at B = 7 and 7.9 ms for group 24x24x14; now 52 and 26 us).
+__global__ void __launch_bounds__(256) k_quad_forms_g(int n, int ncomp, const int* __restrict__ qri,
+                                                      const int* __restrict__ qci, const double* __restrict__ comp,
                                                       int64_t nnz, const double* __restrict__ coef,
                                                       const double* __restrict__ z, const double* __restrict__ x,
                                                       double* part, unsigned* ticket, double* __restrict__ out) {
@@ -236,17 +333,14 @@ __global__ void __launch_bounds__(256) k_quad_forms_g(int n, int ncomp, const in
   double acc[9];
 #pragma unroll
   for (int t = 0; t < 9; ++t) acc[t] = 0.0;
+#pragma unroll 4
+  for (int u = 0; u < 8; ++u) {
+    const int64_t p = (int64_t)blockIdx.x * kRedChunk + threadIdx.x + 256 * u;
+    if (p >= nnz) continue;
+    const double zx = zb[qci[p]] * xb[qri[p]];
 #pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const int j = blockIdx.x * kColChunk + threadIdx.x + 256 * u;
-    if (j >= n) continue;
-    const double zj = zb[j];
-    for (int64_t p = qcp[j]; p < qcp[j + 1]; ++p) {
-      const double zx = zj * xb[qri[p]];
-#pragma unroll
-      for (int t = 0; t < 8; ++t)
-        if (t < ncomp) acc[t] += comp[(int64_t)t * nnz + p] * zx;
-    }
+    for (int t = 0; t < 8; ++t)
+      if (t < ncomp) acc[t] += comp[(int64_t)t * nnz + p] * zx;
   }
   const int nc = ncomp < 8 ? ncomp : 8;
   if (z) {
@@ -257,6 +351,30 @@ __global__ void __launch_bounds__(256) k_quad_forms_g(int n, int ncomp, const in
       if (t < nc) acc[8] += coef[(int64_t)b * ncomp + t] * acc[t];
     grid_reduce_store<9>(acc, nc, true, part, ticket, out + 1, ncomp + 1, -1);
   }
+}
+
+// sum_q w[obs_q] prod_q over the contributions [q0, q1) of the lane's entry. A lane's list of more
+// than 32 is summed by the whole warp, one such lane after the other (an intercept's diagonal entry
+// has one contribution per observation). Every lane of the warp takes part.
+__device__ __forceinline__ double obs_sum_warp(int q0, int q1, const int* __restrict__ cobs,
+                                               const double* __restrict__ cprod, const double* __restrict__ w) {
+  const int lane = threadIdx.x & 31;
+  const bool wide = q1 - q0 > 32;
+  double a = 0.0;
+  if (!wide)
+    for (int q = q0; q < q1; ++q) a += w[cobs[q]] * cprod[q];
+  unsigned todo = __ballot_sync(0xffffffffu, wide);
+  while (todo) {
+    const int src = __ffs(todo) - 1;
+    todo &= todo - 1;
+    const int s0 = __shfl_sync(0xffffffffu, q0, src), s1 = __shfl_sync(0xffffffffu, q1, src);
+    double c = 0.0;
+#pragma unroll 4
+    for (int q = s0 + lane; q < s1; q += 32) c += w[cobs[q]] * cprod[q];
+    c = lane_sum<32>(c);
+    if (lane == src) a = c;
+  }
+  return a;
 }
 
 // Trace contractions of a selected inverse given on the full pattern (both
@@ -276,15 +394,14 @@ __global__ void __launch_bounds__(256) k_trace_contract_g(int64_t nnz, int ncomp
 #pragma unroll
   for (int u = 0; u < 8; ++u) {
     const int64_t p = (int64_t)blockIdx.x * kRedChunk + threadIdx.x + 256 * u;
-    if (p >= nnz) continue;
-    const double sv = sb[p];
+    const bool in = p < nnz;
+    const double sv = in ? sb[p] : 0.0;
 #pragma unroll
     for (int t = 0; t < 8; ++t)
-      if (t < ncomp) acc[t] += sv * comp[(int64_t)t * nnz + p];
+      if (in && t < ncomp) acc[t] += sv * comp[(int64_t)t * nnz + p];
     if (w2) {
-      double a = 0.0;
-      for (int q = cptr[p]; q < cptr[p + 1]; ++q) a += w2[(int64_t)b * nobs + cobs[q]] * cprod[q];
-      acc[8] += sv * a;
+      const double a = obs_sum_warp(in ? cptr[p] : 0, in ? cptr[p + 1] : 0, cobs, cprod, w2 + (int64_t)b * nobs);
+      if (in) acc[8] += sv * a;
     }
   }
   const int nc = ncomp < 8 ? ncomp : 8;

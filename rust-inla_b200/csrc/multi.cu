@@ -21,6 +21,8 @@ inline unsigned grid1(int64_t n, int threads = 256, int cap = 2048) {
   return (unsigned)std::max(1, std::min<int>(cdiv(n, threads), cap));
 }
 
+constexpr int kLanes = 4;  // lanes per column in the Newton right-hand side and A^T v
+
 // Fill-reducing order of one model's block (perm[new] = old, local indices).
 std::vector<int64_t> block_order(int64_t nb, const std::vector<int64_t>& cp, const std::vector<int64_t>& ri,
                                  int ordering) {
@@ -72,7 +74,7 @@ MultiLaplace::MultiLaplace(const MultiSpec& spec, int max_batch, cudaStream_t st
   }
   std::vector<int> pseg(nnz_);
   std::vector<unsigned char> pdiag(nnz_, 0);
-  std::vector<int> qri(nnz_);
+  std::vector<int> qri(nnz_), qci(nnz_);
   for (int64_t c = 0; c < n; ++c) {
     if (!std::is_sorted(spec_.rowidx.begin() + spec_.colptr[c], spec_.rowidx.begin() + spec_.colptr[c + 1]))
       throw std::runtime_error("multi: pattern row indices must be sorted");
@@ -81,6 +83,7 @@ MultiLaplace::MultiLaplace(const MultiSpec& spec, int max_batch, cudaStream_t st
       const int64_t r = spec_.rowidx[p];
       if (r < 0 || r >= n || segc[r] != segc[c]) throw std::runtime_error("multi: pattern is not block-diagonal");
       qri[p] = (int)r;
+      qci[p] = (int)c;
       pseg[p] = segc[c];
       if (r == c) pdiag[p] = 1, diag = true;
     }
@@ -198,6 +201,11 @@ MultiLaplace::MultiLaplace(const MultiSpec& spec, int max_batch, cudaStream_t st
         atv[fill[aci[a]]++] = spec_.av[a];
       }
   }
+  std::vector<int> longc;  // columns summed by a CTA of their own (k_newton_rhs, k_spmv_at)
+  for (int64_t j = 0; j < n; ++j)
+    if ((spec_.colptr[j + 1] - spec_.colptr[j]) + (atp[j + 1] - atp[j]) > long_col(kLanes)) longc.push_back((int)j);
+  nlong_ = (int)longc.size();
+  if (!longc.empty()) longc_.upload(longc, stream_);
 
   comp_.upload(spec_.comp, stream_);
   y_.upload(spec_.y.empty() ? std::vector<double>(1, 0.0) : spec_.y, stream_);
@@ -205,6 +213,7 @@ MultiLaplace::MultiLaplace(const MultiSpec& spec, int max_batch, cudaStream_t st
   if (!spec_.p2.empty()) p2_.upload(spec_.p2, stream_);
   qcp_.upload(spec_.colptr, stream_);
   qri_.upload(qri, stream_);
+  qci_.upload(qci, stream_);
   pdiag_.upload(pdiag, stream_);
   cptr_.upload(cptr, stream_);
   cobs_.upload(cobs, stream_);
@@ -255,6 +264,29 @@ MultiLaplace::MultiLaplace(const MultiSpec& spec, int max_batch, cudaStream_t st
 }
 
 MultiLaplace::~MultiLaplace() = default;
+
+// 4 lanes per column (AR1 and iid columns have 3 to 6 entries) whatever the models are: a model's
+// sums do not depend on the other models.
+void MultiLaplace::newton_rhs(int B, const double* d_x) {
+  auto go = [&](auto kern, unsigned ctas, int threads) {
+    kern<<<dim3(ctas, cdiv(B, kColB)), threads, 0, stream_>>>(
+        (int)spec_.n, spec_.ncomp, spec_.G, segc_.p, qcp_.p, qri_.p, comp_.p, nnz_, coef_.p, atp_.p, ati_.p, atv_.p,
+        spec_.nobs, grad_.p, d_x, step_.p, B, longc_.p);
+    ++launches_;
+  };
+  go(k_newton_rhs<kLanes, 256>, cdiv(spec_.n, 256 / kLanes), 256);
+  if (nlong_ > 0) go(k_newton_rhs<0, kLongThreads>, nlong_, kLongThreads);
+}
+
+void MultiLaplace::spmv_at(int B, const double* d_v, double* d_u) {
+  auto go = [&](auto kern, unsigned ctas, int threads) {
+    kern<<<dim3(ctas, B), threads, 0, stream_>>>((int)spec_.n, atp_.p, ati_.p, atv_.p, spec_.nobs, d_v, d_u, qcp_.p,
+                                                 longc_.p);
+    ++launches_;
+  };
+  go(k_spmv_at<kLanes, 256>, cdiv(spec_.n, 256 / kLanes), 256);
+  if (nlong_ > 0) go(k_spmv_at<0, kLongThreads>, nlong_, kLongThreads);
+}
 
 void MultiLaplace::eval_lik(int B, const double* d_xsrc) {
   const int64_t nobs = spec_.nobs;
@@ -317,7 +349,7 @@ void MultiLaplace::eval(int B, const double* coef, const double* p1scale, int fl
     F_->selinv(B);
     k_pattern_full<<<dim3(grid1(nnz_), B), 256, 0, stream_>>>(nnz_, F_->d_spos_full(), F_->d_sigma(0),
                                                               F_->front_total(), sig_.p);
-    k_seg_trace<256><<<dim3(G, B), 256, 0, stream_>>>(eoff_.p, G, nnz_, T, comp_.p, sig_.p, cptr_.p, cobs_.p,
+    k_seg_trace<1024><<<dim3(G, B), 1024, 0, stream_>>>(eoff_.p, G, nnz_, T, comp_.p, sig_.p, cptr_.p, cobs_.p,
                                                       cprod_.p, nullptr, nobs, d_trP);
     launches_ += 2;
   }
@@ -333,11 +365,10 @@ void MultiLaplace::eval(int B, const double* coef, const double* p1scale, int fl
   auto newton_system = [&](const double* d_x) {
     eval_lik(B, d_x);
     factor(B, true, skip_next && !no_skip);
-    k_mnewton_rhs<<<dim3(GN, B), 256, 0, stream_>>>((int)n, T, G, segc_.p, qcp_.p, qri_.p, comp_.p, nnz_, coef_.p,
-                                                    atp_.p, ati_.p, atv_.p, nobs, grad_.p, d_x, step_.p);
+    newton_rhs(B, d_x);
     F_->solve(step_.p, n, B);
     k_seg_max<256><<<dim3(G, B), 256, 0, stream_>>>(latoff_.p, G, n, step_.p, stats_.p);
-    launches_ += 2;
+    ++launches_;
   };
   auto fetch = [&]() {
     INLA_CUDA(cudaMemcpyAsync(st.data(), stats_.p, sizeof(double) * 2 * BG, cudaMemcpyDeviceToHost, stream_));
@@ -444,7 +475,7 @@ void MultiLaplace::eval(int B, const double* coef, const double* p1scale, int fl
     k_seg_sum<256><<<dim3(G, B), 256, 0, stream_>>>(obsoff_.p, G, nobs, logp_.p, scal_.p);
     ++launches_;
   }
-  k_seg_quad<256><<<dim3(G, B), 256, 0, stream_>>>(latoff_.p, G, (int)n, T, qcp_.p, qri_.p, comp_.p, nnz_, coef_.p,
+  k_seg_quad<1024><<<dim3(G, B), 1024, 0, stream_>>>(eoff_.p, G, (int)n, T, qri_.p, qci_.p, comp_.p, nnz_, coef_.p,
                                                    nullptr, x_.p, d_xMx);
   ++launches_;
   if (spec_.family == FAM_GAUSSIAN && grad && nobs > 0) {
@@ -458,7 +489,7 @@ void MultiLaplace::eval(int B, const double* coef, const double* p1scale, int fl
     if (grad) {
       k_pattern_full<<<dim3(grid1(nnz_), B), 256, 0, stream_>>>(nnz_, F_->d_spos_full(), F_->d_sigma(0),
                                                                 F_->front_total(), sig_.p);
-      k_seg_trace<256><<<dim3(G, B), 256, 0, stream_>>>(eoff_.p, G, nnz_, T, comp_.p, sig_.p, cptr_.p, cobs_.p,
+      k_seg_trace<1024><<<dim3(G, B), 1024, 0, stream_>>>(eoff_.p, G, nnz_, T, comp_.p, sig_.p, cptr_.p, cobs_.p,
                                                         cprod_.p, w_.p, nobs, d_trQ);
       launches_ += 2;
       if (spec_.family != FAM_GAUSSIAN && nobs > 0) {
@@ -466,11 +497,11 @@ void MultiLaplace::eval(int B, const double* coef, const double* p1scale, int fl
         k_predictor_var<<<dim3(grid1(nobs), B), 256, 0, stream_>>>(nobs, acp_.p, av_.p, oppos_.p, opptr_.p, sig_.p,
                                                                    nnz_, tmp_o_.p);
         k_mul<<<dim3(grid1(nobs), B), 256, 0, stream_>>>(nobs, tmp_o_.p, dw_.p, tmp_o_.p);
-        k_spmv_at<<<dim3(GN, B), 256, 0, stream_>>>((int)n, atp_.p, ati_.p, atv_.p, nobs, tmp_o_.p, tmp_n_.p);
+        spmv_at(B, tmp_o_.p, tmp_n_.p);
         F_->solve(tmp_n_.p, n, B);
-        k_seg_quad<256><<<dim3(G, B), 256, 0, stream_>>>(latoff_.p, G, (int)n, T, qcp_.p, qri_.p, comp_.p, nnz_,
+        k_seg_quad<1024><<<dim3(G, B), 1024, 0, stream_>>>(eoff_.p, G, (int)n, T, qri_.p, qci_.p, comp_.p, nnz_,
                                                          coef_.p, tmp_n_.p, x_.p, d_zMx);
-        launches_ += 4;
+        launches_ += 3;
       }
     }
   }

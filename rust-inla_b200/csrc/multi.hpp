@@ -66,6 +66,8 @@ class MultiLaplace {
 
  private:
   void eval_lik(int B, const double* d_xsrc);
+  void newton_rhs(int B, const double* d_x);             // step_ <- A^T grad_ - Q x
+  void spmv_at(int B, const double* d_v, double* d_u);   // u <- A^T v
   // posterior with `skip`: the pairs whose mask entry (active_, [B][G]) is 0 keep their factor
   void factor(int B, bool posterior, bool skip = false);
 
@@ -76,7 +78,8 @@ class MultiLaplace {
   std::unique_ptr<GpuFactor> F_;
   DBuf<double> comp_, y_, p1_, p2_, av_, atv_, cprod_;
   DBuf<int64_t> qcp_, acp_, atp_, opptr_, oppos_, latoff_, obsoff_, poff_, eoff_;
-  DBuf<int> qri_, aci_, ati_, cptr_, cobs_, segc_, sego_, pseg_;
+  DBuf<int> qri_, qci_, aci_, ati_, cptr_, cobs_, segc_, sego_, pseg_, longc_;
+  int nlong_ = 0;  // columns of more than long_col(lanes) entries (longc_)
   DBuf<unsigned char> pdiag_, active_;
   DBuf<double> coef_, p1s_, x_, xt_, step_, eta_, logp_, grad_, w_, dw_, var_, sig_, tmp_n_, tmp_o_, stats_, alpha_,
       mdiff_, scal_, ld_, red_;
