@@ -1,19 +1,21 @@
 // Blocked dense LDL^T of a symmetric block held in shared memory.
 //
-// The pivots are taken 16 at a time. One warp factors the 16 x 16 diagonal
-// block in registers (warp_ldlt16: one __syncwarp per pivot, no CTA barrier
-// on the pivot chain) and forms its inverse Lam = L_kk^-1 alongside. The rows
-// below and the trailing matrix are then updated by all warps with FP64
+// The pivots are taken 8 at a time. One warp factors the 8 x 8 diagonal block with every lane
+// holding the whole block in registers (warp_ldlt8: no exchange on the pivot chain) and forms its
+// inverse Lam = L_kk^-1. The rows below and the trailing matrix are updated by all warps with FP64
 // tensor-core tiles (mma.sync m8n8k4):
 //   U_bk = A_bk Lam^T            (= L_bk D_k),  L_bk = U_bk D_k^-1
 //   A_bb -= L_bk U_bk^T          (lower triangle)
 // which is the right-looking blocked LDL^T (Golub & Van Loan, Matrix
 // Computations, 4th ed., Sec. 4.2) with the diagonal-block solve done through
-// the explicit inverse of the unit triangle. Optionally the inverse of the
-// whole unit lower factor of the leading kp x kp block is accumulated as well
+// the explicit inverse of the unit triangle. The pivot warp looks ahead: it updates the next
+// diagonal block itself and factors it while the other warps update the rest. Optionally the
+// inverse of the whole unit lower factor of the leading kp x kp block is accumulated as well
 // (block forward elimination: Li_k <- Lam Li_k, Li_b <- Li_b - L_bk Li_k).
 #pragma once
 #include <cstdint>
+#include <type_traits>
+
 #include <cuda_runtime.h>
 
 namespace inla {
@@ -36,63 +38,110 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
 }
 
-// Shared scratch of the blocked routine (doubles).
-constexpr int kLamLd = 20;  // leading dimension of the 16 x 16 Lam block (== 4 mod 16: conflict-free tiles)
-constexpr int kDenseScratch = 64 + 16 * kLamLd + 32;
+constexpr int kLamLd = 20;  // leading dimension of a 16 x 16 Lam block (== 4 mod 16: conflict-free tiles)
+// Shared scratch of the blocked routine (doubles): two buffers of Lam (8 x 8) and 1 / d.
+constexpr int kLam8Ld = 12;
+constexpr int kLam8Buf = 8 * kLam8Ld + 8;
+constexpr int kDenseScratch = 2 * kLam8Buf;
 
 // Leading dimension for an m-row block in shared memory: >= m and == 4 (mod 16),
 // so the 16 lanes of a half-warp reading an 8 x 4 fragment hit 16 distinct banks.
 __host__ __device__ constexpr int dense_ld(int m) { return ((m + 11) / 16) * 16 + 4; }
-// Leading dimension of the 16-column U buffer of cta_ldlt (rows rounded up to 8).
+// Leading dimension of the 8-column U buffer of cta_ldlt (rows rounded up to 8).
 __host__ __device__ constexpr int dense_uld(int m) { return dense_ld(m + 8); }
 
-// One warp: LDL^T and inverse of the w x w (w <= 16) leading block of A
-// (shared memory, column-major, leading dimension lda; lower triangle read).
-// On exit A holds L strictly below the diagonal and D on it (inside w x w
-// only); Lam (ld kLamLd) holds L^-1 as a 16 x 16 unit lower triangle
-// (identity beyond w); dv[t] = d_t and di[t] = 1 / d_t (1 beyond w).
-// Lane layout: row r = lane / 2 and the columns j = (lane & 1) + 2q, q < 8.
-// xbuf: 64 doubles (double-buffered pivot column and pivot row of Lam).
-__device__ __forceinline__ void warp_ldlt16(double* A, int lda, int w, double* Lam, double* dv, double* di,
-                                            double* xbuf) {
-  const int lane = threadIdx.x & 31, r = lane >> 1, h = lane & 1;
-  double v[8], li[8];
+// Barrier id: `arrive` counts the caller's warp in without waiting.
+__device__ __forceinline__ void bar_sync_id(int id, int threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void bar_arrive_id(int id, int threads) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+// 1 / d for 1e-300 <= |d| < 1e300 without a branch: the hardware approximation y (relative error e <
+// 2^-20) and one step of the third-order Householder iteration y (1 + e + e^2), whose error e^3 is below
+// the rounding of the last product. d = 0 gives NaN. The operator's slow path for special operands is a
+// branch that keeps the compiler from moving anything across it (90 cycles per division and the block's
+// products in between exposed); this is 65 cycles and leaves one straight line.
+__device__ __forceinline__ double rcp_straight(double d) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+  const double e = fma(-d, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+
+// One warp: LDL^T and inverse of the w x w (w <= 8) leading block of A (shared memory, column-major,
+// even leading dimension lda, 16-byte aligned; lower triangle read). On exit A holds L strictly below
+// the diagonal and D on it (inside w x w only); Lam (ld kLam8Ld) holds L^-1 as an 8 x 8 unit lower
+// triangle (identity beyond w), di[t] = 1 / d_t (1 beyond w), and lam0 / lam1 the lane's entries
+// (g, tg) and (g, tg + 4) of Lam (g = lane / 4, tg = lane % 4: its tensor-core fragments).
+// The chain per pivot is a reciprocal (65 cycles) and two dependent FMAs (12 each). Exchanging the
+// pivot column between lanes put a store -> __syncwarp -> load (40 cycles) and the issue of the
+// exchanged row's loads on it as well: 360 cycles per pivot for 16 x 16 blocks. So every lane repeats
+// the block's 112 products instead, which fit in the shadow of the reciprocals.
+__device__ __forceinline__ void warp_ldlt8(double* A, int lda, int w, double* Lam, double* di, double& lam0,
+                                           double& lam1) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, tg = lane & 3;
+  double a[8][8];  // a[i][j], i >= j
 #pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const int j = h + 2 * q;
-    v[q] = (r < w && j < w) ? (r >= j ? A[r + j * lda] : A[j + r * lda]) : (r == j ? 1.0 : 0.0);
-    li[q] = (r == j) ? 1.0 : 0.0;
-  }
-#pragma unroll 16
-  for (int p = 0; p < 16; ++p) {
-    double* col = xbuf + (p & 1) * 32;  // col[0..15]: column p; col[16..31]: row p of Lam
-    if (h == (p & 1)) col[r] = v[p >> 1];
-    if (r == p) {
+  for (int j = 0; j < 8; ++j)
 #pragma unroll
-      for (int q = 0; q < 8; ++q) col[16 + h + 2 * q] = li[q];
+    for (int i = j & ~1; i < 8; i += 2) {
+      const double2 v = *reinterpret_cast<const double2*>(A + i + j * lda);
+      if (i >= j) a[i][j] = v.x;
+      a[i + 1][j] = v.y;
     }
-    __syncwarp();
-    const double dinv = 1.0 / col[p];
-    if (lane == p) {
-      dv[p] = col[p];
-      di[p] = dinv;
-    }
-    const double ci = (r > p) ? col[r] * dinv : 0.0;
+  if (w < 8) {
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int j = h + 2 * q;
-      if (j > p) v[q] -= ci * col[j];
-      li[q] -= ci * col[16 + j];
-    }
-  }
-  __syncwarp();
+    for (int j = 0; j < 8; ++j)
 #pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const int j = h + 2 * q;
-    if (r < w && j < w && r >= j) A[r + j * lda] = (r == j) ? v[q] : v[q] * di[j];
-    Lam[r + j * kLamLd] = li[q];
+      for (int i = j; i < 8; ++i)
+        if (i >= w) a[i][j] = (i == j) ? 1.0 : 0.0;
   }
-  __syncwarp();
+  // Right-looking elimination of the block and of the columns tg and tg + 4 of L^-1 (x0, x1: rows 4 to 7
+  // of the latter). A finished column leaves for shared memory at once (lane 0), which frees its registers.
+  double x0[8], x1[4];
+  const int lim = lane == 0 ? w : 0;
+  auto eliminate = [&](auto rcp) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) x0[i] = (i == tg) ? 1.0 : 0.0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) x1[i] = (i == tg) ? 1.0 : 0.0;
+#pragma unroll
+    for (int p = 0; p < 8; ++p) {
+      const double r = rcp(a[p][p]);
+      if (lane == 0) di[p] = r;
+      if (p < lim) A[p + p * lda] = a[p][p];
+      double l[8];
+#pragma unroll
+      for (int i = p + 1; i < 8; ++i) l[i] = a[i][p] * r;
+#pragma unroll
+      for (int j = p + 1; j < 8; ++j)
+#pragma unroll
+        for (int i = j; i < 8; ++i) a[i][j] -= l[i] * a[j][p];
+#pragma unroll
+      for (int i = p + 1; i < 8; ++i) {
+        if (i < lim) A[i + p * lda] = l[i];
+        x0[i] -= l[i] * x0[p];
+        if (p >= 4) x1[i - 4] -= l[i] * x1[p - 4];
+      }
+    }
+  };
+  // largest diagonal entry by its high word (sign off; NaN and infinity compare as large)
+  int big = 0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) big = max(big, __double2hiint(a[i][i]) & 0x7fffffff);
+  if (big < 0x7c300000) eliminate([](double d) { return rcp_straight(d); });  // |a_ii| < 2^964
+  else eliminate([](double d) { return 1.0 / d; });  // outside the range of rcp_straight
+  lam0 = x0[0];
+  lam1 = 0.0;
+#pragma unroll
+  for (int i = 1; i < 8; ++i) {
+    if (g == i) lam0 = x0[i];
+    if (i >= 4 && g == i) lam1 = x1[i - 4];
+  }
+  Lam[g + tg * kLam8Ld] = lam0;
+  Lam[g + (tg + 4) * kLam8Ld] = lam1;
 }
 
 // One warp: Lam = L^-1 of the unit lower w x w (w <= 16) block of L (shared
@@ -121,135 +170,149 @@ __device__ __forceinline__ void warp_trinv16(const double* L, int ldl, int w, do
   __syncwarp();
 }
 
-// Lower-triangle tile index: task = I (I + 1) / 2 + J, J <= I.
-__device__ __forceinline__ void tri_decode(int task, int& I, int& J) {
-  int t = (int)((sqrtf(8.0f * (float)task + 1.0f) - 1.0f) * 0.5f);
-  while ((t + 1) * (t + 2) / 2 <= task) ++t;
-  while (t * (t + 1) / 2 > task) --t;
-  I = t;
-  J = task - t * (t + 1) / 2;
-}
-
-// Partial LDL^T of the m x m symmetric matrix A (shared memory, column-major,
+// Partial LDL^T of the m x m symmetric matrix A (shared memory, column-major, 16-byte aligned, even
 // leading dimension lda, lower triangle), eliminating the first kp columns.
 // On exit A[:, :kp] holds L (unit, strictly lower) with D on the diagonal and
 // the lower triangle of A[kp:, kp:] holds the Schur complement. With kInv, Li
 // (shared, leading dimension ldi, kp x kp) receives the inverse of the unit
 // lower factor of the leading kp x kp block (Li must be zero on entry). Called
-// by all threads of the CTA; U: 16 x ldu doubles with ldu = dense_uld(m);
-// ws: kDenseScratch doubles. Ends with a barrier.
+// by all threads of the CTA (at least two warps); U: 8 x ldu doubles with ldu = dense_uld(m);
+// ws: kDenseScratch doubles (16-byte aligned). Ends with a barrier. Uses barrier 1.
+//
+// Per block of 8 pivots the pivot warp (warp 0) runs factor -> its own 8 rows below -> the next
+// diagonal tile without waiting for the others; they wait for Lam (barrier 0), form their rows, wait
+// for the pivot warp's rows (barrier 1, which the pivot warp only counts into), and update the
+// trailing tiles while the pivot warp is already in the next block. What bounds it is the pivot
+// warp's chain. Lam and 1 / d are double-buffered: they are overwritten two blocks later, after a
+// barrier that every reader has passed.
+// Measured for a 64 x 64 block with its inverse, one CTA of 256 threads: 14.3 k cycles (11.6 k without the inverse); the 16-wide form it
+// replaces (one warp factoring 16 x 16 with the others waiting, three barriers per block): 32.7 k (25.5 k).
 template <bool kInv>
 __device__ __forceinline__ void cta_ldlt(double* A, int lda, int m, int kp, double* Li, int ldi, double* U, int ldu, double* ws) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   const int g = lane >> 2, tg = lane & 3;
-  double* xbuf = ws;
-  double* lam = ws + 64;
-  double* dv = lam + 16 * kLamLd;
-  double* di = dv + 16;
-  for (int o = 0; o < kp; o += 16) {
-    const int w = min(16, kp - o);
-    if (warp == 0) {
-      warp_ldlt16(A + o + (int64_t)o * lda, lda, w, lam, dv, di, xbuf);
-      if (kInv) {
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const int e = lane + 32 * q, rr = e & 15, cc = e >> 4;
-          if (rr < w && cc < w) Li[(o + rr) + (int64_t)(o + cc) * ldi] = lam[rr + cc * kLamLd];
-        }
-      }
-    }
-    __syncthreads();
+  int buf = 0;
+  for (int o = 0; o < kp; o += 8, buf ^= 1) {
+    const int w = min(8, kp - o);
+    double* lam = ws + buf * kLam8Buf;
+    double* di = lam + 8 * kLam8Ld;
     const int base = o + w, nb = m - base, T = (nb + 7) >> 3;
-    // U_bk = A_bk Lam^T and L_bk = U_bk D^-1 (8-row tasks, 16 columns each)
-    for (int task = warp; task < T; task += nw) {
-      const int i = base + 8 * task + g;
-      double c[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
-#pragma unroll
-      for (int kk = 0; kk < 16; kk += 4) {
-        const int u = kk + tg;
-        const double a = (u < w && i < m) ? A[i + (int64_t)(o + u) * lda] : 0.0;
-#pragma unroll
-        for (int ct = 0; ct < 2; ++ct) dmma884(c[ct][0], c[ct][1], a, lam[(ct * 8 + g) + u * kLamLd]);
+    const bool w0 = tg < w, w1 = tg + 4 < w;
+    double lam0, lam1;
+    if (warp == 0) {
+      warp_ldlt8(A + o + o * lda, lda, w, lam, di, lam0, lam1);
+      if (kInv) {
+        if (g < w && w0) Li[(o + g) + (o + tg) * ldi] = lam0;
+        if (g < w && w1) Li[(o + g) + (o + tg + 4) * ldi] = lam1;
       }
+    }
+    __syncthreads();
+    const double* Ar = A + base + g + (o + tg) * lda;  // the lane's operand entry of row task 0
+    // rows of 8-row task t: U = A Lam^T and L = U D^-1
+    auto form_rows = [&](int t) {
+      const int i = base + 8 * t + g;
+      const double a0 = (w0 && i < m) ? Ar[8 * t] : 0.0;
+      const double a1 = (w1 && i < m) ? Ar[8 * t + 4 * lda] : 0.0;
+      const double d0 = di[2 * tg], d1 = di[2 * tg + 1];
+      double c0 = 0.0, c1 = 0.0, e0 = 0.0, e1 = 0.0;
+      dmma884(c0, c1, a0, lam0);
+      dmma884(e0, e1, a1, lam1);
+      c0 += e0;
+      c1 += e1;
       __syncwarp();
-      const int ri = base + 8 * task + g;
+      const bool k0 = i < m && 2 * tg < w, k1 = i < m && 2 * tg + 1 < w;
+      double* Ut = U + 2 * tg * ldu + 8 * t + g;
+      double* At = A + i + (o + 2 * tg) * lda;
+      Ut[0] = k0 ? c0 : 0.0;
+      Ut[ldu] = k1 ? c1 : 0.0;
+      if (k0) At[0] = c0 * d0;
+      if (k1) At[lda] = c1 * d1;
+    };
+    // C[8 I + g, 2 tg + h] -= L_I B for N row tiles I = I0, I0 + 1, ... of one column of tiles (the
+    // lane's operand entries b0, b1), all loads before the first store. Rows r with max(lo, diag + h)
+    // <= r < rows (r counted from `base`) are updated.
+    auto column = [&](auto ntiles, int I0, double b0, double b1, double* C, int ldc, int diag, int lo, int rows) {
+      constexpr int N = decltype(ntiles)::value;
+      double a0[N], a1[N], v[N][2], c[N][2];
+      bool ok[N][2];
 #pragma unroll
-      for (int ct = 0; ct < 2; ++ct)
+      for (int q = 0; q < N; ++q) {
+        const int r = 8 * (I0 + q) + g;
+        a0[q] = (w0 && r < rows) ? Ar[8 * (I0 + q)] : 0.0;
+        a1[q] = (w1 && r < rows) ? Ar[8 * (I0 + q) + 4 * lda] : 0.0;
 #pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-          const int t = ct * 8 + 2 * tg + hh;
-          const bool ok = ri < m && t < w;
-          U[t * ldu + (ri - base)] = ok ? c[ct][hh] : 0.0;
-          if (ok) A[ri + (int64_t)(o + t) * lda] = c[ct][hh] * di[t];
+        for (int h = 0; h < 2; ++h) {
+          ok[q][h] = r < rows && r >= diag + h && r >= lo;
+          v[q][h] = ok[q][h] ? C[8 * (I0 + q) + h * ldc] : 0.0;
+          c[q][h] = 0.0;
         }
-    }
-    if (kInv) {
-      // Li_k[:, :o] <- Lam Li_k[:, :o]  (16 rows x 8 columns per task)
-      for (int task = warp; task < (o >> 3); task += nw) {
-        const int c0 = 8 * task;
-        double c[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+      }
 #pragma unroll
-        for (int kk = 0; kk < 16; kk += 4) {
-          const int u = kk + tg;
-          const double b = (u < w) ? Li[(o + u) + (int64_t)(c0 + g) * ldi] : 0.0;
+      for (int q = 0; q < N; ++q) dmma884(c[q][0], c[q][1], a0[q], b0);
 #pragma unroll
-          for (int rt = 0; rt < 2; ++rt) dmma884(c[rt][0], c[rt][1], lam[(rt * 8 + g) + u * kLamLd], b);
-        }
+      for (int q = 0; q < N; ++q) dmma884(c[q][0], c[q][1], a1[q], b1);
+#pragma unroll
+      for (int q = 0; q < N; ++q)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          if (ok[q][h]) C[8 * (I0 + q) + h * ldc] = v[q][h] - c[q][h];
+    };
+    const std::integral_constant<int, 1> one{};
+    const std::integral_constant<int, 4> four{};
+    if (warp == 0) {
+      if (T > 0) {
+        form_rows(0);
         __syncwarp();
-#pragma unroll
-        for (int rt = 0; rt < 2; ++rt)
-#pragma unroll
-          for (int hh = 0; hh < 2; ++hh) {
-            const int rr = rt * 8 + g;
-            if (rr < w) Li[(o + rr) + (int64_t)(c0 + 2 * tg + hh) * ldi] = c[rt][hh];
-          }
+        bar_arrive_id(1, blockDim.x);
+        const double* Ub = U + tg * ldu + g;
+        column(one, 0, Ub[0], Ub[4 * ldu], A + base + g + (base + 2 * tg) * lda, lda, 2 * tg, 0, nb);
+        __syncwarp();
       }
+      continue;
     }
-    __syncthreads();
-    if (nb <= 0) break;
-    // trailing update A_bb -= L_bk U_bk^T (lower 8 x 8 tiles)
-    const int ntask = T * (T + 1) / 2;
-    for (int task = warp; task < ntask; task += nw) {
-      int I, J;
-      tri_decode(task, I, J);
-      const int i = base + 8 * I + g, jb = 8 * J + g;
-      double c0 = 0.0, c1 = 0.0;
-#pragma unroll
-      for (int kk = 0; kk < 16; kk += 4) {
-        const int u = kk + tg;
-        const double a = (u < w && i < m) ? A[i + (int64_t)(o + u) * lda] : 0.0;
-        const double b = U[u * ldu + jb];
-        dmma884(c0, c1, a, b);
-      }
-      const int jc = base + 8 * J + 2 * tg;
-      if (i < m) {
-        if (jc < m && i >= jc) A[i + (int64_t)jc * lda] -= c0;
-        if (jc + 1 < m && i >= jc + 1) A[i + (int64_t)(jc + 1) * lda] -= c1;
-      }
-    }
+    lam0 = lam[g + tg * kLam8Ld];
+    lam1 = lam[g + (tg + 4) * kLam8Ld];
+    for (int t = warp; t < T; t += nw - 1) form_rows(t);
     if (kInv) {
-      // Li_b[:, :base] -= L_bk Li_k[:, :base]  (rows of later blocks inside kp)
-      const int nbi = kp - base, Ti = (nbi + 7) >> 3, Tc = (base + 7) >> 3;
-      for (int task = warp; task < Ti * Tc; task += nw) {
-        const int I = task / Tc, Jc = task - I * Tc;
-        const int i = base + 8 * I + g;
-        double c0 = 0.0, c1 = 0.0;
-#pragma unroll
-        for (int kk = 0; kk < 16; kk += 4) {
-          const int u = kk + tg;
-          const double a = (u < w && i < kp) ? A[i + (int64_t)(o + u) * lda] : 0.0;
-          const double b = (u < w) ? Li[(o + u) + (int64_t)(8 * Jc + g) * ldi] : 0.0;
-          dmma884(c0, c1, a, b);
-        }
-        const int jc = 8 * Jc + 2 * tg;
-        if (i < kp) {
-          if (jc < base) Li[i + (int64_t)jc * ldi] -= c0;
-          if (jc + 1 < base) Li[i + (int64_t)(jc + 1) * ldi] -= c1;
+      // Li_k[:, :o] <- Lam Li_k[:, :o]  (8 columns per task)
+      for (int t = warp - 1; t < (o >> 3); t += nw - 1) {
+        const double* Lb = Li + (o + tg) + (8 * t + g) * ldi;
+        const double b0 = w0 ? Lb[0] : 0.0, b1 = w1 ? Lb[4] : 0.0;
+        double c0 = 0.0, c1 = 0.0, e0 = 0.0, e1 = 0.0;
+        dmma884(c0, c1, lam0, b0);
+        dmma884(e0, e1, lam1, b1);
+        __syncwarp();
+        if (g < w) {
+          Li[(o + g) + (8 * t + 2 * tg) * ldi] = c0 + e0;
+          Li[(o + g) + (8 * t + 2 * tg + 1) * ldi] = c1 + e1;
         }
       }
     }
-    __syncthreads();
+    if (T == 0) continue;
+    bar_sync_id(1, blockDim.x);
+    // Trailing tiles A_IJ -= L_I U_J^T (I >= J) and, with kInv, Li_IJ -= L_I Li_kJ for the rows of
+    // later blocks inside kp: one task is up to four row tiles of a tile column.
+    const int Tc = kInv ? base >> 3 : 0;
+    const int nbi = kp - base;
+    int left = warp - 1;  // tasks to skip before this warp's next one
+    for (int I0 = 0; I0 < T; I0 += 4) {
+      const int nj = min(T, I0 + 4), ni = 8 * I0 < nbi ? Tc : 0;
+      for (; left < nj + ni; left += nw - 1) {
+        if (left < nj) {
+          const int J = left, c = 8 * J + 2 * tg;
+          const double* Ub = U + tg * ldu + 8 * J + g;
+          // the first eight rows of column 0 are the pivot warp's
+          column(four, I0, Ub[0], Ub[4 * ldu], A + base + g + (base + c) * lda, lda, c, J == 0 ? 8 : 0, nb);
+        } else if (kInv) {
+          const int J = left - nj, c = 8 * J + 2 * tg;
+          const double* Lb = Li + (o + tg) + (8 * J + g) * ldi;
+          column(four, I0, Lb[0], Lb[4], Li + base + g + c * ldi, ldi, -8, 0, nbi);  // w = 8: rows follow
+        }
+      }
+      left -= nj + ni;
+    }
   }
+  __syncthreads();
 }
 
 }  // namespace

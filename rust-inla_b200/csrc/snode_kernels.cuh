@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(256) k_fill_panels_model(DevSym S, const int* 
 
 // Shared memory of k_factor_small for fronts of up to m rows (bytes).
 __host__ __device__ constexpr int small_factor_smem(int m) {
-  return (m * dense_ld(m) + 16 * dense_uld(m) + kDenseScratch) * 8;
+  return (m * dense_ld(m) + 8 * dense_uld(m) + kDenseScratch) * 8;
 }
 
 // One CTA per (front, problem): the front in shared memory (leading dimension
@@ -206,7 +206,7 @@ __device__ __forceinline__ void factor_small_body(const DevSym& S, int s, int b,
   const int lda = dense_ld(m), uld = dense_uld(m);
   double* A = sm;
   double* U = A + m * lda;
-  double* ws = U + 16 * uld;
+  double* ws = U + 8 * uld;
   int* rs = reinterpret_cast<int*>(U);  // child relative indices (U is free until the factorization)
   double* Fs = Fb + S.fptr[s];
   const int mm = m * m;
@@ -255,8 +255,10 @@ __device__ __forceinline__ void factor_small_body(const DevSym& S, int s, int b,
   }
 }
 
+// At most 128 registers: four CTAs of 128 threads or two of 256 per SM, which is what the shared memory
+// of 64- and 96-row fronts allows (the pivot warp's block alone would take the kernel to 160).
 template <int NT>
-__global__ void __launch_bounds__(NT) k_factor_small(DevSym S, const int* __restrict__ list,
+__global__ void __launch_bounds__(NT, 512 / NT) k_factor_small(DevSym S, const int* __restrict__ list,
                                                      double* __restrict__ F, int64_t fstride) {
   extern __shared__ double sm[];
   factor_small_body<NT>(S, list[blockIdx.x], blockIdx.y, F, fstride, sm);

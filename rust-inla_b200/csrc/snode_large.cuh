@@ -33,7 +33,7 @@ constexpr int kB64 = 64;         // block-column width
 constexpr int kPanelRows = 64;   // rows per panel GEMM sub-block
 constexpr int kLd64 = dense_ld(kB64);
 constexpr int kULd64 = dense_uld(kB64);
-constexpr int kPanelSmem = (2 * kB64 * kLd64 + 16 * kULd64 + kDenseScratch) * 8;
+constexpr int kPanelSmem = (2 * kB64 * kLd64 + 8 * kULd64 + kDenseScratch) * 8;
 constexpr int kSiGemmSmem = 3 * 64 * kLd64 * 8;  // three stage buffers
 constexpr int kSiDiagSmem = 3 * kB64 * (kB64 + 1) * 8;
 
@@ -184,8 +184,8 @@ __device__ __forceinline__ void panel64_body(const DevSym& S, int s, int b, int 
 
   double* Ds = smem64;         // [64 cols][ld]: diagonal block, factored in place; then row sub-blocks
   double* Li = Ds + kB64 * ld; // L_JJ^-1, then Bm[u + t*ld] = Li[t][u] / d_t
-  double* U = Li + kB64 * ld;  // [16][kULd64] scratch of cta_ldlt, then 1 / d_t
-  double* ws = U + 16 * kULd64;
+  double* U = Li + kB64 * ld;  // [8][kULd64] scratch of cta_ldlt, then 1 / d_t
+  double* ws = U + 8 * kULd64;
   const int k = lg_k(S, s), m = lg_m(S, s);
   if (j0 >= k) return;
   const int w = min(kB64, k - j0);
@@ -274,7 +274,7 @@ __device__ __forceinline__ void panel64_body(const DevSym& S, int s, int b, int 
   }
 }
 
-__global__ void __launch_bounds__(256) k_panel64(DevSym S, const int* __restrict__ list, int j0, int rpc,
+__global__ void __launch_bounds__(256, 2) k_panel64(DevSym S, const int* __restrict__ list, int j0, int rpc,
                                                  double* __restrict__ F, int64_t fstride,
                                                  double* __restrict__ dcache, double* __restrict__ linv) {
   extern __shared__ double smem64[];

@@ -218,7 +218,7 @@ __device__ __forceinline__ void update64w8_body(const DevSym& S, int s, int b, i
     double* Ds = smu;             // [64 cols][ld]: the next diagonal block, factored in place
     double* Li = Ds + kB64 * ld;  // its L^-1
     double* U = Li + kB64 * ld;
-    double* ws = U + 16 * kULd64;
+    double* ws = U + 8 * kULd64;
     __syncthreads();  // the operand tiles are consumed
     for (int e = threadIdx.x; e < kB64 * kB64; e += blockDim.x) {
       Ds[(e & 63) + (e >> 6) * ld] = 0.0;
