@@ -218,10 +218,8 @@ class GpuFactor {
   DBuf<int64_t> d_fptr_, d_lptr_, d_dpos_, spos_, spos_full_, d_gptr_;
   DBuf<int2> d_grng_;  // extend-add source-column ranges per (front, chunk, child)
   DBuf<int> d_pmap_, d_lists_, d_csn_, d_csnm_, d_lbo_;
-  DBuf<double> F_, Sg_, xp_, ub_, logdet_, dcache_, ppart_, linv_, ldpart_;
+  DBuf<double> F_, Sg_, xp_, ub_, logdet_, dcache_, linv_, ldpart_;
   DBuf<int> status_, ldflag_;
-  DBuf<double> gpart_;  // split-K pieces of the selected inverse's G (narrow levels)
-  DBuf<int> sicnt_;     // arrival counters of the selected inverse's step kernel (kept zeroed)
   DBuf<unsigned> ldticket_;
   int nfill_ = 0, nfillm_ = 0, nldchunk_ = 0;  // fill chunks (values, model); log-det chunks per problem
   int num_sms_ = 148;

@@ -10,15 +10,7 @@
 //   update      F[i,j] -= sum_{t in J} L_it d_t L_jt on 64x64 tiles of the lower
 //               trailing matrix (tensor-core tiles, operands staged with cp.async;
 //               update64w8_body in snode_persist.cuh, launched as k_update64w8).
-// Selected inverse, per block J from right to left (A = rows after J):
-//   k_si_step64 G = Sigma[A,A] L[A,J] per 64-row tile of A (the K range split over
-//               several CTAs where the launch would leave SMs idle), X = -G L_JJ^-1
-//               (cached inverse block), Sigma[A,J] = X, and the tile's partial
-//               P = L[I,J]^T X[I,J];
-//   k_si_diag64 Sigma_JJ = L_JJ^-T (D^-1 L_JJ^-1 - P), P the fixed-order sum of
-//               the partials: the closed form of the in-block Takahashi
-//   recurrence S_ij = -P_ji - sum_{l in J, l>j} L_lj S_li,
-//   S_jj = 1/d_j - P_jj - sum_{l in J, l>j} L_lj S_lj.
+// Selected inverse: matrix products over the whole front (k_si_gemm).
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -35,7 +27,6 @@ constexpr int kLd64 = dense_ld(kB64);
 constexpr int kULd64 = dense_uld(kB64);
 constexpr int kPanelSmem = (2 * kB64 * kLd64 + 8 * kULd64 + kDenseScratch) * 8;
 constexpr int kSiGemmSmem = 3 * 64 * kLd64 * 8;  // three stage buffers
-constexpr int kSiDiagSmem = 3 * kB64 * (kB64 + 1) * 8;
 
 __device__ __forceinline__ int lg_k(const DevSym& S, int s) { return S.first[s + 1] - S.first[s]; }
 __device__ __forceinline__ int lg_m(const DevSym& S, int s) { return S.rowptr[s + 1] - S.rowptr[s]; }
@@ -760,371 +751,213 @@ __global__ void __launch_bounds__(32 * kTinySweepWarps) k_bwd_tiny(DevSym S, con
 // selected inverse
 // ---------------------------------------------------------------------------
 
-// Sigma[row, col] of a front stored as its lower triangle (column-major, ld m)
-__device__ __forceinline__ double sig_lower(const double* Ss, int m, int row, int col) {
-  return row >= col ? Ss[row + (int64_t)col * m] : Ss[col + (int64_t)row * m];
-}
+constexpr int kSiT = 64;  // rows of B per tile
 
-constexpr int kSiT = 64;  // rows of A per CTA
+// ---------------------------------------------------------------------------
+// Selected inverse of the large fronts as matrix products over the whole front. With K the k pivot
+// rows, B the r rows below, X = L_KK^-1 and W = L_BK X:
+//   Sigma_BK = -Sigma_BB W,   Sigma_KK = X^T D^-1 X - W^T Sigma_BK,
+// the closed form of the Takahashi recurrence S_ij = -sum_{l>j} L_lj S_li, S_jj = 1/d_j - sum_{l>j}
+// L_lj S_lj over the block K (Sigma_BB comes from the parent). X is built from the cached 64 x 64
+// inverses by doubling: for neighbouring block ranges 1 and 2, X_21 = -X_22 (L_21 X_11).
+//
+// The blockwise recurrence takes two dependent launches per 64 pivot columns (22 for the 644-column
+// root front of the SPDE 200^2 model); this takes 2 log2(k / 64) + 3 with the same number of products,
+// every launch over all tiles of the level. Measured, SPDE 200^2 posterior, all products of the large
+// fronts: 1.71 -> 1.02 ms at B = 1 (1.27 with 64-row tiles only), 3.69 -> 2.95 ms at B = 10, 4.66 ->
+// 3.98 ms at B = 15. Chains of launches bound the small batches, padding of 100- to 200-row fronts to
+// 64 x 64 tiles the large ones.
+//
+// X and W live transposed in the strictly upper triangle of the front's Sigma buffer (block (I, J) of X
+// at (J, I), W at (K, B)), which nothing else uses; the products L_21 X_11 in the lower block that
+// Sigma_KK takes at the end. One CTA per 64 x 64 tile, K in chunks of 32 through three cp.async stages.
+// ---------------------------------------------------------------------------
+enum SiMode : int {
+  SI_T = 0,      // T = L_21 X_11                      (lower block (I, J))
+  SI_X = 1,      // X_21 = -X_22 T                     (transposed, upper block)
+  SI_W = 2,      // W = L_BK X                         (transposed, upper block)
+  SI_BK = 3,     // Sigma_BK = -Sigma_BB W
+  SI_KK = 4,     // Sigma_KK = X^T D^-1 X - W^T Sigma_BK
+};
 
-// Split of the K loop of G = Sigma[I,A] L[A,J]: a front whose A spans at least
-// kSiSplitMinChunks chunks of 32 rows has its K range cut into pieces of kSiChunksPerSplit
-// chunks, one CTA each, when the launch allows it (the host allows it where one CTA per row
-// tile would leave SMs idle). The pieces are summed in a fixed order, so a given launch shape
-// always gives the same result; split and unsplit steps differ by rounding only.
-constexpr int kSiChunksPerSplit = 4;
-constexpr int kSiSplitMinChunks = 8;
-__host__ __device__ inline int si_nsplit(int nch, bool allow) {
-  return (allow && nch >= kSiSplitMinChunks) ? (nch + kSiChunksPerSplit - 1) / kSiChunksPerSplit : 1;
-}
-
-// Sigma_JJ = L^-T (D^-1 L^-1 - P), L = L_JJ unit lower, P = L[A,J]^T Sigma[A,J]
-// (the closed form of the in-block Takahashi recurrence), with L^-1 from the
-// inverse-block cache and the product as a tensor-core GEMM. Block jb of front s, problem b
-// (256 threads); pp_front: the tiles' partial P blocks (tile z at pp_front + z * 4096), read
-// through L2 because other CTAs of the same launch wrote them.
-__device__ __forceinline__ void si_diag64_body(const DevSym& S, int s, int b, int jb, const double* __restrict__ F,
-                                               double* __restrict__ Sg, int64_t fstride,
-                                               const double* __restrict__ pp_front,
-                                               const double* __restrict__ linv, double* smem64) {
-  constexpr int ld = kB64 + 1;
-  double* Pm = smem64;            // P, then M = D^-1 L^-1 - P  (Pm[r + c*ld] = entry (r, c))
-  double* Ld = Pm + kB64 * ld;    // L_JJ with D on the diagonal
-  double* Li = Ld + kB64 * ld;    // L_JJ^-1
+// Tile z of front s, problem b. hb: block count of the ranges joined (SI_T, SI_X). TM = 32 cuts every
+// tile into two CTAs of 32 rows, for launches whose 64-row tiles would leave SMs idle (the K loop of
+// one 64 x 64 tile is 1.1 us per chunk at the tensor-core rate of one SM); an entry's sum is the same.
+template <int MODE, int TM>
+__device__ __forceinline__ void si_gemm_body(const DevSym& S, int s, int b, int z, int hb,
+                                             const double* __restrict__ F, double* __restrict__ Sg, int64_t fstride,
+                                             const double* __restrict__ linv, double* smem64) {
+  constexpr int ld = kLd64, kBuf = 64 * kLd64;  // one stage: As[32][ld], Bs[32][ld]
+  __shared__ double scale[3][32];
   const int k = lg_k(S, s), m = lg_m(S, s);
-  const int nblk = (k + kB64 - 1) / kB64;
-  if (jb >= nblk) return;
-  const int bi = nblk - 1 - jb;
-  const int j0 = bi * kB64, j1 = min(k, j0 + kB64), w = j1 - j0;
-  const int ntiles = (m - j1 + kSiT - 1) / kSiT;
+  const int nblk = (k + kB64 - 1) / kB64, rt = (m - k + kSiT - 1) / kSiT;
+  const int half = TM == 32 ? (z & 1) : 0;
+  if (TM == 32) z >>= 1;
+  // tile (rows i0 .. i1, columns j0 .. j1) and the K range t0 .. t1, all in rows of the front
+  int i0, i1, j0, t0, t1;
+  if (MODE == SI_T || MODE == SI_X) {
+    const int pr = z / (hb * hb), q = z - pr * hb * hb, first = 2 * pr * hb;
+    const int I = first + hb + q / hb, J = first + q % hb;
+    if (I >= nblk) return;
+    i0 = I * kB64;
+    i1 = min(k, i0 + kB64);
+    j0 = J * kB64;
+    t0 = MODE == SI_T ? j0 : (first + hb) * kB64;
+    t1 = MODE == SI_T ? (first + hb) * kB64 : i1;
+  } else if (MODE == SI_W || MODE == SI_BK) {
+    const int I = z / nblk, J = z - I * nblk;
+    if (I >= rt) return;
+    i0 = k + I * kSiT;
+    i1 = min(m, i0 + kSiT);
+    j0 = J * kB64;
+    t0 = MODE == SI_W ? j0 : k;
+    t1 = MODE == SI_W ? k : m;
+  } else {
+    if (z >= nblk * (nblk + 1) / 2) return;
+    int I = 0, rem = z;
+    while (rem > I) rem -= ++I;
+    i0 = I * kB64;
+    i1 = min(k, i0 + kB64);
+    j0 = rem * kB64;
+    t0 = i0 + 32 * half;  // X is lower triangular
+    t1 = m;
+  }
+  if (TM == 32) {
+    i0 += 32 * half;
+    i1 = min(i1, i0 + 32);
+    if (i0 >= i1) return;
+  }
+  const int j1 = min(k, j0 + kB64);
   const double* Fs = F + (int64_t)b * fstride + S.fptr[s];
   double* Ss = Sg + (int64_t)b * fstride + S.fptr[s];
-  const double* pp = pp_front;
-  const double* lc = linv_block(S, linv, b, s, bi);
-  for (int e = threadIdx.x; e < kB64 * kB64; e += blockDim.x) {
-    const int c = e >> 6, r = e & 63;
-    if (r < w && c < w && r >= c) cp_async8(&Ld[r + c * ld], Fs + (j0 + r) + (int64_t)(j0 + c) * m);
-    else Ld[r + c * ld] = 0.0;
-    cp_async8(&Li[r + c * ld], lc + e);
-  }
-  cp_async_commit();
-  {
-    // partials are stored row-major: pp[j*64 + i] = P[j][i]; fixed summation order over tiles
-    double acc[16];
+  const double* lb = linv + (int64_t)b * S.lstride + (int64_t)S.lbo[s] * (kB64 * kB64);
+  // address of X (t < k) or W (t >= k) at (t, c), c < k, in a block on or below the diagonal
+  auto xw = [&](int t, int c) -> const double* {
+    const int cb = c >> 6;
+    if ((t >> 6) == cb && t < k) return lb + (int64_t)cb * (kB64 * kB64) + (t & 63) + (c & 63) * kB64;
+    return Ss + c + (int64_t)t * m;
+  };
+  auto load_chunk = [&](int c0, int buf) {
+    double* As = smem64 + buf * kBuf;
+    double* Bs = As + 32 * ld;
+    constexpr bool a_along_t = MODE == SI_X;
 #pragma unroll
-    for (int q = 0; q < 16; ++q) acc[q] = 0.0;
-    for (int z = 0; z < ntiles; ++z) {
-      const double* pz = pp + (int64_t)z * kB64 * kB64;
-#pragma unroll
-      for (int q = 0; q < 16; ++q) acc[q] += __ldcg(pz + threadIdx.x + 256 * q);
-    }
-#pragma unroll
-    for (int q = 0; q < 16; ++q) {
-      const int e = threadIdx.x + 256 * q, j = e >> 6, i = e & 63;
-      Pm[j + i * ld] = acc[q];
-    }
-  }
-  cp_async_wait<0>();
-  __syncthreads();
-  for (int e = threadIdx.x; e < kB64 * kB64; e += blockDim.x) {
-    const int c = e >> 6, r = e & 63;
-    Pm[r + c * ld] = (r < w && c < w) ? Li[r + c * ld] / Ld[r + r * ld] - Pm[r + c * ld] : 0.0;
-  }
-  __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (warp < 4) {
-    const int wr = (warp & 1) * 32, wc = (warp >> 1) * 32;
-    const int g = lane >> 2, tg = lane & 3;
-    double acc[4][4][2];
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int q = 0; q < 4; ++q) acc[a][q][0] = acc[a][q][1] = 0.0;
-#pragma unroll 4
-    for (int kk = 0; kk < kB64; kk += 4) {
-      double af[4], bf[4];
-#pragma unroll
-      for (int a = 0; a < 4; ++a) af[a] = Li[(kk + tg) + (wr + a * 8 + g) * ld];  // (L^-1)^T
-#pragma unroll
-      for (int q = 0; q < 4; ++q) bf[q] = Pm[(kk + tg) + (wc + q * 8 + g) * ld];
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) mma884(acc[a][q][0], acc[a][q][1], af[a], bf[q]);
-    }
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int r = wr + a * 8 + g, c = wc + q * 8 + tg * 2 + h;
-          if (r < w && c < w && r >= c) Ss[(j0 + r) + (int64_t)(j0 + c) * m] = acc[a][q][h];
-        }
-  }
-}
-
-// Last-arrival count: every thread's global writes are fenced, then one thread counts the
-// CTA in; true in the CTA whose arrival completes the count (it then resets the counter for
-// the next launch and reads what the others wrote). Nothing waits on another CTA.
-__device__ __forceinline__ bool si_arrive_last(int* counter, int expected, int* sh_flag) {
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const int t = atomicAdd(counter, 1);
-    *sh_flag = (t == expected - 1);
-    if (t == expected - 1) *counter = 0;
-  }
-  __syncthreads();
-  const bool last = *sh_flag != 0;
-  if (last) __threadfence();
-  return last;
-}
-
-// Off-diagonal part of one 64-column step of the selected inverse of the large fronts (block
-// jb counted from the right). CTA z = I * smax + sp handles row tile I of A (64 rows) and
-// K piece sp:
-//   G_I = Sigma[I,A] L[A,J] over its K piece (chunks of 32 rows, three cp.async stages);
-//   with a split K the pieces go to gp_front and the last piece to arrive sums them in piece
-//   order; X = -G_I L_JJ^-1 (cached inverse block) is Sigma[I,J]; the tile's partial
-//   P_I = L[I,J]^T X goes to pp_front (k_si_diag64 then forms Sigma_JJ).
-// Every sum has a fixed order, so the result does not depend on which CTA arrives last; with
-// one piece (smax == 1) the arithmetic is the single-CTA K loop.
-// cnt_front: ptiles zeroed counters (one per tile), left zeroed again.
-// Shared memory: three chunk buffers (Sa[32][68] + Lb[32][68] each) for the G loop;
-// afterwards buffer 0 holds G (then X), buffer 1 L_JJ^-1 and buffer 2 L[I,J].
-__device__ __forceinline__ void si_step64_body(const DevSym& S, int s, int b, int z, int jb,
-                                               const double* __restrict__ F, double* __restrict__ Sg,
-                                               int64_t fstride, double* __restrict__ pp_front,
-                                               const double* __restrict__ linv, double* smem64,
-                                               double* __restrict__ gp_front, int* cnt_front, int ptiles,
-                                               int smax, bool allow_split) {
-  __shared__ int sh_last;
-  constexpr int kBuf = 64 * kLd64;  // doubles per chunk buffer (Sa[32][68] + Lb[32][68])
-  typedef double Row68[kLd64];  // leading dimension 68 == 4 (mod 16): conflict-free fragments
-  Row68* Gs = reinterpret_cast<Row68*>(smem64);             // [64][68]: G, then X
-  Row68* Lt = reinterpret_cast<Row68*>(smem64 + 2 * kBuf);  // [64][68]: L[I0+l, j0+j]
-  const int k = lg_k(S, s), m = lg_m(S, s);
-  const int nblk = (k + kB64 - 1) / kB64;
-  if (jb >= nblk) return;
-  const int bi = nblk - 1 - jb;
-  const int j0 = bi * kB64, j1 = min(k, j0 + kB64), w = j1 - j0;
-  const int ntiles = (m - j1 + kSiT - 1) / kSiT;
-  if (ntiles == 0) return;
-  const int nch = (m - j1 + 31) / 32;
-  const int ns = si_nsplit(nch, allow_split);
-  const int I = z / smax, sp = z - I * smax;
-  if (I >= ntiles || sp >= ns) return;
-  const int I0 = j1 + I * kSiT;
-  const int cb = sp * kSiChunksPerSplit, ce = ns == 1 ? nch : min(nch, cb + kSiChunksPerSplit);
-  const double* Fs = F + (int64_t)b * fstride + S.fptr[s];
-  double* Ss = Sg + (int64_t)b * fstride + S.fptr[s];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // 8 warps, warp tile 32 x 16; warps whose columns lie beyond the block's w skip the products
-  const int wi = (warp & 1) * 32, wj = (warp >> 1) * 16;
-  const int g = lane >> 2, tg = lane & 3;
-  const bool wact = wj < w && I0 + wi < m;
-
-  // chunk loader: Sigma[I0.., l0..l0+32) (lower-triangle storage) and L[l0.., j0..j0+w)
-  auto load_chunk = [&](int l0, int buf) {
-    Row68* Sa = reinterpret_cast<Row68*>(smem64 + buf * kBuf);
-    Row68* Lb = reinterpret_cast<Row68*>(smem64 + buf * kBuf + 32 * kLd64);
-    if (I0 >= l0 + 31) {  // on/below the diagonal: stored at (i, l), coalesced over i
-      for (int e = threadIdx.x; e < 32 * kSiT; e += blockDim.x) {
-        const int l = e / kSiT, ii = e - l * kSiT, row = I0 + ii, col = l0 + l;
-        if (row < m && col < m) cp_async8(&Sa[l][ii], Ss + row + (int64_t)col * m);
-        else Sa[l][ii] = 0.0;
-      }
-    } else if (I0 + kSiT - 1 < l0) {  // above: read the transposed entry (l, i), coalesced over l
-      for (int e = threadIdx.x; e < 32 * kSiT; e += blockDim.x) {
-        const int ii = e / 32, l = e - ii * 32, row = I0 + ii, col = l0 + l;
-        if (row < m && col < m) cp_async8(&Sa[l][ii], Ss + col + (int64_t)row * m);
-        else Sa[l][ii] = 0.0;
-      }
-    } else {
-      for (int e = threadIdx.x; e < 32 * kSiT; e += blockDim.x) {
-        const int l = e / kSiT, ii = e - l * kSiT, row = I0 + ii, col = l0 + l;
-        if (row < m && col < m)
-          cp_async8(&Sa[l][ii], row >= col ? Ss + row + (int64_t)col * m : Ss + col + (int64_t)row * m);
-        else Sa[l][ii] = 0.0;
+    for (int u = 0; u < TM / 8; ++u) {
+      const int e = threadIdx.x + 256 * u;
+      bool along_t = a_along_t;
+      if (MODE == SI_BK) along_t = i0 + TM - 1 < c0;  // above the diagonal: stored at (t, i)
+      const int l = along_t ? (e & 31) : (e / TM), ii = along_t ? (e >> 5) : (e % TM);
+      const int t = c0 + l, i = i0 + ii;
+      double* dst = As + l * ld + ii;
+      if (t < t1 && i < i1) {
+        const double* src;
+        if (MODE == SI_T || MODE == SI_W) src = Fs + i + (int64_t)t * m;
+        else if (MODE == SI_X) src = xw(i, t);
+        else if (MODE == SI_BK) src = i >= t ? Ss + i + (int64_t)t * m : Ss + t + (int64_t)i * m;
+        else src = xw(t, i);
+        cp_async8(dst, src);
+      } else {
+        *dst = 0.0;
       }
     }
-    for (int e = threadIdx.x; e < 32 * kB64; e += blockDim.x) {
-      const int t = e / 32, l = e - t * 32;
-      if (t < w && l0 + l < m) cp_async8(&Lb[l][t], Fs + (l0 + l) + (int64_t)(j0 + t) * m);
-      else Lb[l][t] = 0.0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int e = threadIdx.x + 256 * u;
+      const bool along_t = MODE == SI_X || (MODE == SI_KK && c0 >= k);
+      const int l = along_t ? (e & 31) : (e >> 6), jj = along_t ? (e >> 5) : (e & 63);
+      const int t = c0 + l, j = j0 + jj;
+      double* dst = Bs + l * ld + jj;
+      if (t < t1 && j < j1) {
+        const double* src;
+        if (MODE == SI_X) src = Ss + t + (int64_t)j * m;
+        else if (MODE == SI_BK) src = Ss + j + (int64_t)t * m;
+        else if (MODE == SI_KK && t >= k) src = Ss + t + (int64_t)j * m;
+        else src = xw(t, j);
+        cp_async8(dst, src);
+      } else {
+        *dst = 0.0;
+      }
+    }
+    if (MODE == SI_KK && threadIdx.x < 32) {
+      const int t = c0 + threadIdx.x;
+      scale[buf][threadIdx.x] = t < k ? 1.0 / Fs[t + (int64_t)t * m] : -1.0;
     }
     cp_async_commit();
   };
-
-  double acc[4][2][2];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int NA = TM / 16;  // 8-row sub-tiles of a warp
+  const int wi = (warp & 1) * (TM / 2), wj = (warp >> 1) * 16;
+  const int g = lane >> 2, tg = lane & 3;
+  const bool wact = i0 + wi < i1 && j0 + wj < j1;
+  double acc[NA][2][2];
 #pragma unroll
-  for (int a = 0; a < 4; ++a)
+  for (int a = 0; a < NA; ++a)
 #pragma unroll
     for (int q = 0; q < 2; ++q) acc[a][q][0] = acc[a][q][1] = 0.0;
-  const int nc = ce - cb;
-  load_chunk(j1 + 32 * cb, 0);
-  if (nc > 1) load_chunk(j1 + 32 * (cb + 1), 1);
+  const int nc = (t1 - t0 + 31) / 32;
+  load_chunk(t0, 0);
+  if (nc > 1) load_chunk(t0 + 32, 1);
   for (int c = 0; c < nc; ++c) {
-    if (c + 2 < nc) {
-      load_chunk(j1 + 32 * (cb + c + 2), (c + 2) % 3);
-      cp_async_wait<2>();
-    } else if (c + 1 < nc) {
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
-    __syncthreads();
-    const Row68* Sa = reinterpret_cast<const Row68*>(smem64 + (c % 3) * kBuf);
-    const Row68* Lb = reinterpret_cast<const Row68*>(smem64 + (c % 3) * kBuf + 32 * kLd64);
+    if (c + 1 < nc) cp_async_wait<1>();
+    else cp_async_wait<0>();
+    __syncthreads();  // chunk c has landed, and every warp is done with chunk c - 1
+    if (c + 2 < nc) load_chunk(t0 + 32 * (c + 2), (c + 2) % 3);
+    const double* As = smem64 + (c % 3) * kBuf;
+    const double* Bs = As + 32 * ld;
     if (wact) {
 #pragma unroll
       for (int kk = 0; kk < 32; kk += 4) {
-        double af[4], bf[2];
+        double af[NA], bf[2];
 #pragma unroll
-        for (int a = 0; a < 4; ++a) af[a] = Sa[kk + tg][wi + a * 8 + g];
+        for (int a = 0; a < NA; ++a) af[a] = As[(kk + tg) * ld + wi + a * 8 + g];
 #pragma unroll
-        for (int q = 0; q < 2; ++q) bf[q] = Lb[kk + tg][wj + q * 8 + g];
+        for (int q = 0; q < 2; ++q) bf[q] = Bs[(kk + tg) * ld + wj + q * 8 + g];
+        if (MODE == SI_KK) {
+          const double sc = scale[c % 3][kk + tg];
+          bf[0] *= sc;
+          bf[1] *= sc;
+        }
 #pragma unroll
-        for (int a = 0; a < 4; ++a)
+        for (int a = 0; a < NA; ++a)
 #pragma unroll
           for (int q = 0; q < 2; ++q) mma884(acc[a][q][0], acc[a][q][1], af[a], bf[q]);
       }
     }
+  }
+  constexpr double sign = (MODE == SI_X || MODE == SI_BK) ? -1.0 : 1.0;
+  if (MODE == SI_X || MODE == SI_W) {  // transposed output: through shared memory, contiguous over j
     __syncthreads();
-  }
-  if (ns > 1) {  // this piece to gp_front; the last piece of the tile sums them in order
-    double* gp = gp_front + (int64_t)(I * smax + sp) * (kB64 * kB64);
+    double* Gs = smem64;  // [64][ld]
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+    for (int a = 0; a < NA; ++a)
 #pragma unroll
       for (int q = 0; q < 2; ++q)
 #pragma unroll
-        for (int h = 0; h < 2; ++h) gp[(wi + a * 8 + g) * kB64 + wj + q * 8 + tg * 2 + h] = acc[a][q][h];
-    if (!si_arrive_last(cnt_front + I, ns, &sh_last)) return;
-  }
-  // L_JJ^-1 (cached) and L[I,J] are fetched together, G goes to buffer 0
-  double* Li = smem64 + kBuf;
-  const int rows = min(kSiT, m - I0);
-  Row68* Lij = Lt;  // Lij[l][j] = L[I0+l, j0+j]
-  {
-    const double* lc = linv_block(S, linv, b, s, bi);
-    for (int e = threadIdx.x; e < kB64 * kB64; e += blockDim.x) cp_async8(&Li[(e & 63) + (e >> 6) * kLd64], lc + e);
-    for (int e = threadIdx.x; e < kSiT * kB64; e += blockDim.x) {
-      const int j = e / kSiT, l = e - j * kSiT;
-      if (l < rows && j < w) cp_async8(&Lij[l][j], Fs + (I0 + l) + (int64_t)(j0 + j) * m);
-      else Lij[l][j] = 0.0;
+        for (int h = 0; h < 2; ++h) Gs[(wi + a * 8 + g) * ld + wj + q * 8 + tg * 2 + h] = sign * acc[a][q][h];
+    __syncthreads();
+    for (int e = threadIdx.x; e < TM * kB64; e += 256) {
+      const int ii = e >> 6, jj = e & 63;
+      if (i0 + ii < i1 && j0 + jj < j1) Ss[(j0 + jj) + (int64_t)(i0 + ii) * m] = Gs[ii * ld + jj];
     }
-    cp_async_commit();
+    return;
   }
-  if (ns > 1) {
-    const double* gq = gp_front + (int64_t)(I * smax) * (kB64 * kB64);
-    for (int e = threadIdx.x; e < kB64 * kB64; e += blockDim.x) {
-      double v = __ldcg(gq + e);
-      for (int q = 1; q < ns; ++q) v += __ldcg(gq + (int64_t)q * (kB64 * kB64) + e);
-      Gs[e >> 6][e & 63] = v;
-    }
-  } else {
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int q = 0; q < 2; ++q)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) Gs[wi + a * 8 + g][wj + q * 8 + tg * 2 + h] = acc[a][q][h];
-  }
-  // X = -G L_JJ^-1 as a tensor-core GEMM with the cached inverse of the unit
-  // lower diagonal block
-  cp_async_wait<0>();
-  __syncthreads();
-  {
-    double xa[4][2][2];
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int q = 0; q < 2; ++q) xa[a][q][0] = xa[a][q][1] = 0.0;
-    const int wk = (w + 3) & ~3;
-    if (wact) {
-#pragma unroll 4
-      for (int kk = 0; kk < wk; kk += 4) {
-        double af[4], bf[2];
-#pragma unroll
-        for (int a = 0; a < 4; ++a) af[a] = Gs[wi + a * 8 + g][kk + tg];
-#pragma unroll
-        for (int q = 0; q < 2; ++q) bf[q] = Li[(kk + tg) + (wj + q * 8 + g) * kLd64];
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-          for (int q = 0; q < 2; ++q) mma884(xa[a][q][0], xa[a][q][1], af[a], bf[q]);
-      }
-    }
-    __syncthreads();  // all reads of G done before X overwrites it
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int q = 0; q < 2; ++q)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int ii = wi + a * 8 + g, t = wj + q * 8 + tg * 2 + h;
-          const double xv = -xa[a][q][h];
-          Gs[ii][t] = xv;
-          if (I0 + ii < m && t < w) Ss[(I0 + ii) + (int64_t)(j0 + t) * m] = xv;
-        }
-  }
-  __syncthreads();
-  // partial P[j][i] = sum_{rows l of this tile} L[I0+l, j0+j] X[l, i]  (tensor-core tiles)
-  double pa[4][2][2];
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int q = 0; q < 2; ++q) pa[a][q][0] = pa[a][q][1] = 0.0;
-  const int wr = (warp & 1) * 32, wc = (warp >> 1) * 16;  // output rows j, cols i
-  if (wr < w && wc < w) {
-    const int kr = (rows + 3) & ~3;
-#pragma unroll 4
-    for (int kk = 0; kk < kr; kk += 4) {
-      double af[4], bf[2];
-#pragma unroll
-      for (int a = 0; a < 4; ++a) af[a] = Lij[kk + tg][wr + a * 8 + g];
-#pragma unroll
-      for (int q = 0; q < 2; ++q) bf[q] = Gs[kk + tg][wc + q * 8 + g];
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int q = 0; q < 2; ++q) mma884(pa[a][q][0], pa[a][q][1], af[a], bf[q]);
-    }
-  }
-  double* pp = pp_front + (int64_t)I * (kB64 * kB64);
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
+  for (int a = 0; a < NA; ++a)
 #pragma unroll
     for (int q = 0; q < 2; ++q)
 #pragma unroll
-      for (int h = 0; h < 2; ++h) pp[(wr + a * 8 + g) * kB64 + wc + q * 8 + tg * 2 + h] = pa[a][q][h];
+      for (int h = 0; h < 2; ++h) {
+        const int i = i0 + wi + a * 8 + g, j = j0 + wj + q * 8 + tg * 2 + h;
+        if (i < i1 && j < j1 && (MODE != SI_KK || i >= j)) Ss[i + (int64_t)j * m] = sign * acc[a][q][h];
+      }
 }
 
-// ppart: [list index][b][tile][64*64] partial P blocks; gpart: [list index][b][tile][piece]
-// [64*64] pieces of G (used when smax > 1); cnt: [list index][b][ptiles] counters.
-__global__ void __launch_bounds__(256) k_si_step64(DevSym S, const int* __restrict__ list, int jb,
-                                                  const double* __restrict__ F, double* __restrict__ Sg,
-                                                  int64_t fstride, double* __restrict__ ppart, int ptiles,
-                                                  const double* __restrict__ linv, double* __restrict__ gpart,
-                                                  int* __restrict__ cnt, int smax, int allow_split) {
+template <int MODE, int TM>
+__global__ void __launch_bounds__(256, 2) k_si_gemm(DevSym S, const int* __restrict__ list, int hb,
+                                                    const double* __restrict__ F, double* __restrict__ Sg,
+                                                    int64_t fstride, const double* __restrict__ linv) {
   extern __shared__ double smem64[];
-  const int64_t slot = (int64_t)blockIdx.x * gridDim.y + blockIdx.y;
-  // gpart is sized for split launches only (smax > 1)
-  si_step64_body(S, list[blockIdx.x], blockIdx.y, blockIdx.z, jb, F, Sg, fstride,
-                 ppart + slot * ptiles * (kB64 * kB64), linv, smem64,
-                 smax > 1 ? gpart + slot * ptiles * smax * (kB64 * kB64) : gpart, cnt + slot * ptiles, ptiles, smax,
-                 allow_split != 0);
-}
-
-__global__ void __launch_bounds__(256) k_si_diag64(DevSym S, const int* __restrict__ list, int jb,
-                                                  const double* __restrict__ F, double* __restrict__ Sg,
-                                                  int64_t fstride, const double* __restrict__ ppart, int ptiles,
-                                                  const double* __restrict__ linv) {
-  extern __shared__ double smem64[];
-  const double* pp = ppart + ((int64_t)blockIdx.x * gridDim.y + blockIdx.y) * ptiles * (kB64 * kB64);
-  si_diag64_body(S, list[blockIdx.x], blockIdx.y, jb, F, Sg, fstride, pp, linv, smem64);
+  si_gemm_body<MODE, TM>(S, list[blockIdx.x], blockIdx.y, blockIdx.z, hb, F, Sg, fstride, linv, smem64);
 }
 
 }  // namespace
