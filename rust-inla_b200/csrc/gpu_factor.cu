@@ -33,22 +33,16 @@ __global__ void __launch_bounds__(256, 2) k_update64w8(DevSym S, const int* __re
                                                          double* __restrict__ F, int64_t fstride,
                                                          const double* __restrict__ dcache) {
   extern __shared__ double smu[];
-  const double* dc = dcache + ((int64_t)blockIdx.x * gridDim.y + blockIdx.y) * (kB64 * kB64);
+  const double* dc = dcache ? dcache + ((int64_t)blockIdx.x * gridDim.y + blockIdx.y) * (kB64 * kB64) : nullptr;
   update64w8_body(S, list[blockIdx.x], blockIdx.y, blockIdx.z, j0, F, fstride, dc, smu);
 }
 
-// The same update with look-ahead: tile 0 of every (front, problem) also factors the next
-// diagonal block (D and L into the other cache slot, L^-1 into the inverse-block cache), so the
-// pivot chain of block J + 1 runs while the other tiles of step J are updated and the step
-// after needs no diagonal-block launch. Results are bit-identical to the split form.
-__global__ void __launch_bounds__(256, 2) k_update64la(DevSym S, const int* __restrict__ list, int j0,
-                                                         double* __restrict__ F, int64_t fstride,
-                                                         const double* __restrict__ dcache,
-                                                         double* __restrict__ dcache_next, double* __restrict__ linv) {
+// Diagonal blocks of step j0 >= 64 in the look-ahead form, one CTA per (front, problem).
+__global__ void __launch_bounds__(256, 2) k_diag_next(DevSym S, const int* __restrict__ list, int j0,
+                                                      double* __restrict__ F, int64_t fstride,
+                                                      double* __restrict__ linv) {
   extern __shared__ double smu[];
-  const int64_t slot = ((int64_t)blockIdx.x * gridDim.y + blockIdx.y) * (kB64 * kB64);
-  update64w8_body<true>(S, list[blockIdx.x], blockIdx.y, blockIdx.z, j0, F, fstride, dcache + slot, smu,
-                        dcache_next + slot, linv);
+  diag_next_body(S, list[blockIdx.x], blockIdx.y, j0, F, fstride, linv, smu);
 }
 
 // Parent columns per extend-add CTA: the m-row slice must fit in shared memory.
@@ -319,6 +313,8 @@ GpuFactor::GpuFactor(const Symbolic& sym, int max_batch, cudaStream_t stream)
     d_grng_.upload(grng, stream_);
   }
 
+  INLA_CUDA(cudaStreamCreateWithFlags(&chain_stream_, cudaStreamNonBlocking));
+  for (auto& e : chain_ev_) INLA_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   panel_form_ = g_panel_form.load();
   plan_persist();
   const auto ta = std::chrono::steady_clock::now();
@@ -331,9 +327,7 @@ GpuFactor::GpuFactor(const Symbolic& sym, int max_batch, cudaStream_t stream)
   {
     int64_t nlmax = 1;
     for (const LevelPlan& P : levels_) nlmax = std::max<int64_t>(nlmax, (int64_t)P.large.size());
-    // two slots: the look-ahead form factors block J + 1 while step J still reads block J
-    dslot_ = nlmax * max_batch_ * kB64 * kB64;
-    dcache_.alloc((size_t)(2 * dslot_));
+    dcache_.alloc((size_t)nlmax * max_batch_ * kB64 * kB64);
   }
   set_smem(k_factor_small<128>, small_factor_smem(kSmallA));
   set_smem(k_factor_small<256>, small_factor_smem(kSmallB));
@@ -356,7 +350,7 @@ GpuFactor::GpuFactor(const Symbolic& sym, int max_batch, cudaStream_t stream)
     struct_hash_ = h;
   }
   set_smem(k_update64w8, kPersistUpdSmem);
-  set_smem(k_update64la, kPanelSmem);
+  set_smem(k_diag_next, kPanelSmem);
   set_smem(k_rows64, kRowsSmem);
   set_smem(k_fwd32<128>, (int)((S.max_m + 2 + 32 * 33) * 8));
   set_smem(k_bwd32<128>, (int)((S.max_m + 2 + 32 * 33) * 8));
@@ -395,6 +389,9 @@ GpuFactor::GpuFactor(const Symbolic& sym, int max_batch, cudaStream_t stream)
 }
 
 GpuFactor::~GpuFactor() {
+  for (auto& e : chain_ev_)
+    if (e) cudaEventDestroy(e);
+  if (chain_stream_) cudaStreamDestroy(chain_stream_);
   for (auto& kv : graphs_) cudaGraphExecDestroy(kv.second.exec);
 }
 
@@ -498,17 +495,16 @@ bool make_persist_plan(const Symbolic& S, const std::vector<LevelPlan>& levels, 
   pl = PersistPlan();
   pl.gstart = {0};
   pl.total.assign(ns, 0);
-  pl.lid.assign(ns, -1);
   pl.gptr.assign(ns, 0);
-  auto push = [&](int type, int sn, int sub, int need, int j0, int gcols) {
-    pl.task.insert(pl.task.end(), {type, sn, sub, need, j0, gcols});
+  auto push = [&](int type, int sn, int sub, int need, int j0, int arg) {
+    pl.task.insert(pl.task.end(), {type, sn, sub, need, j0, arg});
   };
   auto close_group = [&] {
     const int cnt = (int)(pl.task.size() / 6);
     if (cnt > pl.gstart.back()) pl.gstart.push_back(cnt);
   };
   struct Phase {
-    int type, count, j0;
+    int type, count, j0, sub0, need, arg;  // tasks sub0 .. sub0 + count - 1
   };
   for (const LevelPlan& P : levels) {
     for (size_t i = 0; i < P.tiny.size(); i += kPersistTinyWarps) {
@@ -527,17 +523,16 @@ bool make_persist_plan(const Symbolic& S, const std::vector<LevelPlan>& levels, 
       }
     close_group();
     if (P.large.empty()) continue;
-    // phases of every large front: 0 extend-add, then (diagonal, rows, update) per block
+    // phases of every large front: extend-add, first diagonal block, then per block J the next diagonal
+    // block, the rows and the update
     std::vector<std::vector<Phase>> ph(P.large.size());
-    std::vector<int> gc(P.large.size());
     size_t maxp = 0;
     for (size_t f = 0; f < P.large.size(); ++f) {
       const int sn = P.large[f];
       const int k = (int)(S.sn_first[sn + 1] - S.sn_first[sn]), m = (int)(S.sn_rowptr[sn + 1] - S.sn_rowptr[sn]);
       const int gcols = std::max(1, std::min(kGatherCols, kGatherBudget / (8 * m)));
-      gc[f] = gcols;
       smem = std::max(smem, gcols * m * 8);
-      pl.lid[sn] = pl.nlarge++;
+      ++pl.nlarge;
       const int nz = cdiv(m, gcols);
       pl.gptr[sn] = (int64_t)pl.grng.size();
       for (int z = 0; z < nz; ++z) {
@@ -552,26 +547,29 @@ bool make_persist_plan(const Symbolic& S, const std::vector<LevelPlan>& levels, 
           pl.grng.push_back(make_int2(lo, hi));
         }
       }
-      ph[f].push_back({PT_GATHER, nz, 0});
+      ph[f].push_back({PT_GATHER, nz, 0, 0, 0, gcols});
+      ph[f].push_back({PT_DIAG, 1, 0, 0, nz, 0});
+      int done = nz;  // extend-add, row and update tasks so far
       for (int j0 = 0; j0 < k; j0 += kB64) {
         const int w = std::min(kB64, k - j0), below = std::max(m - j0 - w, 0);
-        const int nt = cdiv(below, kUT64);
-        ph[f].push_back({PT_DIAG, 1, j0});
-        ph[f].push_back({PT_ROWS, cdiv(below, kPanelRows), j0});
-        ph[f].push_back({PT_UPDATE, std::max(1, nt * (nt + 1) / 2), j0});
+        const int nt = cdiv(below, kUT64), nrow = cdiv(below, kPanelRows);
+        const bool next = j0 + kB64 < k;  // then tile 0 of the update is the next diagonal block's
+        const int diags = j0 / kB64 + 1;
+        ph[f].push_back({PT_NEXT, next ? 1 : 0, j0 + kB64, 0, done, diags});
+        ph[f].push_back({PT_ROWS, nrow, j0, 0, done, diags});
+        done += nrow;
+        const int ntile = nt * (nt + 1) / 2 - (next ? 1 : 0);
+        ph[f].push_back({PT_UPDATE, ntile, j0, next ? 1 : 0, done, 0});
+        done += ntile;
       }
       maxp = std::max(maxp, ph[f].size());
-      int tot = 0;
-      for (const Phase& x : ph[f]) tot += x.count;
-      pl.total[sn] = tot;
+      pl.total[sn] = done;
     }
-    std::vector<int> done(P.large.size(), 0);
     for (size_t p = 0; p < maxp; ++p) {
       for (size_t f = 0; f < P.large.size(); ++f) {
         if (p >= ph[f].size()) continue;
         const Phase& x = ph[f][p];
-        for (int u = 0; u < x.count; ++u) push(x.type, P.large[f], u, done[f], x.j0, gc[f]);
-        done[f] += x.count;
+        for (int u = 0; u < x.count; ++u) push(x.type, P.large[f], x.sub0 + u, x.need, x.j0, x.arg);
       }
       close_group();
     }
@@ -592,7 +590,7 @@ std::string check_persist_plan(const Symbolic& S, const PersistPlan& pl) {
   if (pl.gstart.back() != ntask) return "group table does not cover the tasks";
   for (size_t g = 0; g + 1 < pl.gstart.size(); ++g)
     if (pl.gstart[g + 1] <= pl.gstart[g]) return "empty or decreasing group " + std::to_string(g);
-  std::vector<int> prog(ns, 0);
+  std::vector<int> prog(ns, 0), diag(ns, 0), step(ns, -1);
   auto children_done = [&](int sn) {
     for (int64_t q = S.child_ptr[sn]; q < S.child_ptr[sn + 1]; ++q) {
       const int c = (int)S.child_list[q];
@@ -600,6 +598,7 @@ std::string check_persist_plan(const Symbolic& S, const PersistPlan& pl) {
     }
     return true;
   };
+  auto blocks = [&](int sn) { return cdiv(S.sn_first[sn + 1] - S.sn_first[sn], kB64); };
   for (int t = 0; t < ntask; ++t) {
     const int* T = pl.task.data() + 6 * t;
     const int type = T[0], sn = T[1], sub = T[2], need = T[3];
@@ -621,23 +620,35 @@ std::string check_persist_plan(const Symbolic& S, const PersistPlan& pl) {
       if (m > GpuFactor::kSmallB) return at + "front too large for the small body";
       if (!children_done(sn)) return at + "small front before its children";
     } else if (type == PT_GATHER) {
-      if (pl.lid[sn] < 0 || !children_done(sn)) return at + "extend-add before the children";
+      if (m <= GpuFactor::kSmallB || !children_done(sn)) return at + "extend-add before the children";
       const int gcols = T[5], nch = (int)(S.child_ptr[sn + 1] - S.child_ptr[sn]);
       if (gcols < 1 || (int64_t)gcols * m * 8 > pl.smem) return at + "extend-add slice exceeds shared memory";
       if (sub >= cdiv(m, gcols) || pl.gptr[sn] + (int64_t)(sub + 1) * nch > (int64_t)pl.grng.size())
         return at + "extend-add chunk out of range";
       if (need != 0 || prog[sn] != sub) return at + "extend-add count";
-    } else if (type == PT_DIAG || type == PT_ROWS || type == PT_UPDATE) {
-      if (pl.lid[sn] < 0) return at + "step of a front that is not large";
+    } else if (type == PT_DIAG || type == PT_NEXT || type == PT_ROWS || type == PT_UPDATE) {
+      if (m <= GpuFactor::kSmallB) return at + "step of a front that is not large";
       if (T[4] < 0 || T[4] >= k || T[4] % kB64) return at + "block column out of range";
-      if (prog[sn] < need) return at + "phase before its predecessors";
+      if (prog[sn] < need || diag[sn] < T[5]) return at + "phase before its predecessors";
+      const int J = T[4] / kB64;
+      if (type == PT_DIAG || type == PT_NEXT) {
+        // block J after block J - 1; its mirror rows and its tile after the updates of step J - 2
+        if (J != diag[sn] || (type == PT_DIAG) != (J == 0) || (J > 0 && T[5] < J)) return at + "diagonal block order";
+        if (J >= 2 && step[sn] < J - 2) return at + "diagonal block before its updates";
+        ++diag[sn];
+        continue;
+      }
+      if (type == PT_ROWS && T[5] < J + 1) return at + "rows before their diagonal block";
+      if (type == PT_UPDATE) step[sn] = J;
     } else {
       return at + "unknown task type";
     }
     ++prog[sn];
   }
   for (int sn = 0; sn < ns; ++sn)
-    if (pl.total[sn] < 1 || prog[sn] != pl.total[sn]) return "front " + std::to_string(sn) + " incomplete";
+    if (pl.total[sn] < 1 || prog[sn] != pl.total[sn] ||
+        (S.sn_rowptr[sn + 1] - S.sn_rowptr[sn] > GpuFactor::kSmallB && diag[sn] != blocks(sn)))
+      return "front " + std::to_string(sn) + " incomplete";
   return std::string();
 }
 
@@ -735,19 +746,17 @@ void GpuFactor::plan_persist() {
   PersistPlan pl;
   if (!make_persist_plan(sym_, levels_, pl)) return;  // a front too wide for the schedule's shared memory
   const int ns = (int)sym_.nsuper;
-  const size_t dc_doubles = (size_t)std::max(pl.nlarge, 1) * max_batch_ * kB64 * kB64;
-  if (dc_doubles * 8 > ((size_t)4 << 30)) return;
+  // (the limit of the former block cache, kept so that the same engines stay with level launches)
+  if ((size_t)std::max(pl.nlarge, 1) * max_batch_ * kB64 * kB64 * 8 > ((size_t)4 << 30)) return;
   persist_groups_ = (int)pl.gstart.size() - 1;
   d_pgstart_.upload(pl.gstart, stream_);
   d_ptask_.upload(pl.task, stream_);
   d_ptiny_.upload(pl.tiny, stream_);
   d_ptotal_.upload(pl.total, stream_);
-  d_plid_.upload(pl.lid, stream_);
   d_pgptr_.upload(pl.gptr, stream_);
   d_pgrng_.upload(pl.grng, stream_);
-  d_pstate_.alloc(2 + (size_t)max_batch_ * ns);
-  INLA_CUDA(cudaMemsetAsync(d_pstate_.p, 0, sizeof(int) * (2 + (size_t)max_batch_ * ns), stream_));
-  dcache_p_.alloc(dc_doubles);
+  d_pstate_.alloc(2 + 2 * (size_t)max_batch_ * ns);
+  INLA_CUDA(cudaMemsetAsync(d_pstate_.p, 0, sizeof(int) * (2 + 2 * (size_t)max_batch_ * ns), stream_));
   persist_smem_ = pl.smem;
   persist_ = true;
   plan_solve_persist();
@@ -762,7 +771,7 @@ void GpuFactor::run_factor_persist(int B, const int* total_override, long long l
                                    const unsigned char* active, int nseg) {
   const int ns = (int)sym_.nsuper;
   // head and the completion counts start at zero; the error record (word 0) stays until read
-  INLA_CUDA(cudaMemsetAsync(d_pstate_.p + 1, 0, sizeof(int) * (1 + (size_t)B * ns), stream_));
+  INLA_CUDA(cudaMemsetAsync(d_pstate_.p + 1, 0, sizeof(int) * (1 + 2 * (size_t)B * ns), stream_));
   PersistArgs a;
   a.S = ds_;
   a.F = F_.p;
@@ -774,10 +783,9 @@ void GpuFactor::run_factor_persist(int B, const int* total_override, long long l
   a.tiny_list = d_ptiny_.p;
   a.total = total_override ? total_override : d_ptotal_.p;
   a.prog = d_pstate_.p + 2;
+  a.dprog = d_pstate_.p + 2 + (size_t)B * ns;
   a.head = reinterpret_cast<unsigned*>(d_pstate_.p + 1);
   a.err = d_pstate_.p;
-  a.dcache = dcache_p_.p;
-  a.lid = d_plid_.p;
   a.linv = linv_.p;
   a.gptr = d_pgptr_.p;
   a.grng = d_pgrng_.p;
@@ -909,16 +917,24 @@ void GpuFactor::run_factor_levels(int B, const std::vector<char>* fuse, cudaEven
         int nt = cdiv(rows, kUT64);
         const dim3 ug(nl, B, std::max(1, nt * (nt + 1) / 2));
         if (form == kFormLookahead) {
-          // block 0 by one CTA per (front, problem); every later diagonal block by tile 0 of
-          // the previous step's update
-          double* cur = dcache_.p + ((j0 / kB64) & 1) * dslot_;
-          double* nxt = dcache_.p + (((j0 / kB64) + 1) & 1) * dslot_;
+          // The pivot chain runs on a stream of its own: the diagonal block of step J + 1 depends on
+          // the one of step J and on the updates of step J - 1, and runs beside the rows and updates
+          // of step J.
           if (j0 == 0) {
-            k_panel64<<<dim3(nl, B, 1), 256, kPanelSmem, stream_>>>(ds_, lst, j0, 0, F_.p, fs, cur, linv_.p);
+            k_panel64<<<dim3(nl, B, 1), 256, kPanelSmem, stream_>>>(ds_, lst, j0, 0, F_.p, fs, nullptr, linv_.p);
             ++launches_;
           }
-          k_rows64<<<dim3(nl, B, nrb), 256, kRowsSmem, stream_>>>(ds_, lst, j0, F_.p, fs, cur, linv_.p);
-          k_update64la<<<ug, 256, kPanelSmem, stream_>>>(ds_, lst, j0, F_.p, fs, cur, nxt, linv_.p);
+          const bool next = j0 + kB64 < P.kmax_large;
+          if (next) {
+            INLA_CUDA(cudaEventRecord(chain_ev_[0], stream_));
+            INLA_CUDA(cudaStreamWaitEvent(chain_stream_, chain_ev_[0], 0));
+            k_diag_next<<<dim3(nl, B), 256, kPanelSmem, chain_stream_>>>(ds_, lst, j0 + kB64, F_.p, fs, linv_.p);
+            INLA_CUDA(cudaEventRecord(chain_ev_[1], chain_stream_));
+            ++launches_;
+          }
+          k_rows64<<<dim3(nl, B, nrb), 256, kRowsSmem, stream_>>>(ds_, lst, j0, F_.p, fs, nullptr, linv_.p);
+          k_update64w8<<<ug, 256, kPersistUpdSmem, stream_>>>(ds_, lst, j0, F_.p, fs, nullptr);
+          if (next) INLA_CUDA(cudaStreamWaitEvent(stream_, chain_ev_[1], 0));
           launches_ += 2;
           continue;
         }

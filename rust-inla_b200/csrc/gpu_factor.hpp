@@ -80,10 +80,10 @@ struct LevelPlan {
 };
 
 // Task queue of the persistent schedule for one problem (snode_persist.cuh): 6 ints per task
-// {type, front, sub, need, j0, gcols}, group starts, tiny-front list, completion counts per
-// front, large-front index, extend-add chunk table, shared memory in bytes.
+// {type, front, sub, need, j0, arg}, group starts, tiny-front list, completion counts per
+// front, extend-add chunk table, shared memory in bytes.
 struct PersistPlan {
-  std::vector<int> gstart, task, tiny, total, lid;
+  std::vector<int> gstart, task, tiny, total;
   std::vector<int64_t> gptr;
   std::vector<int2> grng;
   int nlarge = 0, smem = 0;
@@ -231,11 +231,11 @@ class GpuFactor {
   std::map<int, bool> persist_at_;  // measured choice per batch size
   int persist_smem_ = 0, persist_grid_ = 0, persist_groups_ = 0;
   long long persist_limit_ns_ = 2000000000LL;
-  DBuf<int> d_pgstart_, d_ptask_, d_ptiny_, d_ptotal_, d_plid_, d_pstate_;  // pstate: err, head, prog[B][ns]
+  DBuf<int> d_pgstart_, d_ptask_, d_ptiny_, d_ptotal_, d_pstate_;  // pstate: err, head, prog[B][ns], dprog[B][ns]
   DBuf<int64_t> d_pgptr_;
   DBuf<int2> d_pgrng_;
-  DBuf<double> dcache_p_;
-  int64_t dslot_ = 0;  // doubles per slot of dcache_ (two slots)
+  cudaStream_t chain_stream_ = nullptr;  // pivot chain of the look-ahead form, joined with stream_
+  cudaEvent_t chain_ev_[2] = {nullptr, nullptr};
   int panel_form_ = -1;  // forced panel form (set_panel_form at construction), -1 autotuned
   DBuf<int> d_fseg_;
   // persistent solve

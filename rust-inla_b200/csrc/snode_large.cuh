@@ -167,7 +167,8 @@ __global__ void __launch_bounds__(256) k_si_gather8(DevSym S, const int* __restr
 // staged in the diagonal block's buffer once it is no longer needed, which
 // keeps the CTA at 84 KB of shared memory (two CTAs per SM).
 // Block J = [j0, j0 + 64) of front s, problem b, row CTA z (256 threads). dc: this front's and
-// problem's slot of the factored-diagonal-block cache (written when z == 0).
+// problem's slot of the factored-diagonal-block cache (written when z == 0), or nullptr in the chain
+// form (one CTA per front and problem, rpc = 0), which writes the factored block into the front.
 __device__ __forceinline__ void panel64_body(const DevSym& S, int s, int b, int z, int j0, int rpc,
                                              double* __restrict__ F, int64_t fstride, double* __restrict__ dc,
                                              double* __restrict__ linv, double* smem64) {
@@ -199,9 +200,17 @@ __device__ __forceinline__ void panel64_body(const DevSym& S, int s, int b, int 
     double* lc = const_cast<double*>(linv_block(S, linv, b, s, j0 / kB64));
     for (int e = threadIdx.x; e < kB64 * kB64; e += blockDim.x) {
       const int c = e >> 6, r = e & 63;
-      dc[e] = (r < w && c < w) ? Ds[r + c * ld] : 0.0;
       lc[e] = Li[r + c * ld];  // zero outside the w x w lower triangle
+      if (dc) dc[e] = (r < w && c < w) ? Ds[r + c * ld] : 0.0;
+      else if (r < w && c < w && r >= c) Fs[(j0 + r) + (int64_t)(j0 + c) * m] = Ds[r + c * ld];
     }
+    // chain form: the next diagonal block's task reads the unscaled rows from their mirror position
+    // while the row tasks scale them in place
+    if (!dc && j0 + kB64 < k)
+      for (int e = threadIdx.x; e < kB64 * kB64; e += blockDim.x) {
+        const int c = e & 63, r = e >> 6, i = j0 + kB64 + r;
+        if (i < m) Fs[(j0 + c) + (int64_t)i * m] = Fs[i + (int64_t)(j0 + c) * m];
+      }
   }
   if (r0 >= r1) return;
   double* dinv = U;
@@ -269,7 +278,7 @@ __global__ void __launch_bounds__(256, 2) k_panel64(DevSym S, const int* __restr
                                                  double* __restrict__ F, int64_t fstride,
                                                  double* __restrict__ dcache, double* __restrict__ linv) {
   extern __shared__ double smem64[];
-  double* dc = dcache + ((int64_t)blockIdx.x * gridDim.y + blockIdx.y) * (kB64 * kB64);
+  double* dc = dcache ? dcache + ((int64_t)blockIdx.x * gridDim.y + blockIdx.y) * (kB64 * kB64) : nullptr;
   panel64_body(S, list[blockIdx.x], blockIdx.y, blockIdx.z, j0, rpc, F, fstride, dc, linv, smem64);
 }
 
@@ -279,7 +288,8 @@ __global__ void __launch_bounds__(256, 2) k_panel64(DevSym S, const int* __restr
 // tensor-core GEMM. Used when many fronts x problems share a step, where a
 // factorization per row CTA would be redundant work.
 constexpr int kRowsSmem = (2 * kB64 * kLd64 + kB64) * 8;
-// Row block z of block J of front s, problem b (256 threads); dc as in panel64_body.
+// Row block z of block J of front s, problem b (256 threads); dc as in panel64_body (nullptr: D is
+// read from the front).
 __device__ __forceinline__ void rows64_body(const DevSym& S, int s, int b, int z, int j0, double* __restrict__ F,
                                             int64_t fstride, const double* __restrict__ dc,
                                             const double* __restrict__ linv, double* smr) {
@@ -302,7 +312,9 @@ __device__ __forceinline__ void rows64_body(const DevSym& S, int s, int b, int z
   }
   cp_async_commit();
   const double* lc = linv_block(S, linv, b, s, j0 / kB64);
-  if (threadIdx.x < kB64) dinv[threadIdx.x] = threadIdx.x < w ? 1.0 / dc[threadIdx.x * (kB64 + 1)] : 0.0;
+  const double* dg = dc ? dc : Fs + j0 + (int64_t)j0 * m;  // d_t at dg[t * ds]
+  const int64_t ds = dc ? kB64 + 1 : m + 1;
+  if (threadIdx.x < kB64) dinv[threadIdx.x] = threadIdx.x < w ? 1.0 / dg[threadIdx.x * ds] : 0.0;
   __syncthreads();
   double lv[16];
 #pragma unroll
@@ -350,7 +362,7 @@ __global__ void __launch_bounds__(256) k_rows64(DevSym S, const int* __restrict_
                                                 double* __restrict__ F, int64_t fstride,
                                                 const double* __restrict__ dcache, const double* __restrict__ linv) {
   extern __shared__ double smr[];
-  const double* dc = dcache + ((int64_t)blockIdx.x * gridDim.y + blockIdx.y) * (kB64 * kB64);
+  const double* dc = dcache ? dcache + ((int64_t)blockIdx.x * gridDim.y + blockIdx.y) * (kB64 * kB64) : nullptr;
   rows64_body(S, list[blockIdx.x], blockIdx.y, blockIdx.z, j0, F, fstride, dc, linv, smr);
 }
 

@@ -6,15 +6,18 @@
 // resident CTAs with one atomic counter:
 //   tiny fronts (m <= 32): up to 8 fronts per task, one warp each;
 //   small fronts (m <= 96): one task per front;
-//   large fronts: extend-add chunks, then per 64-column block J one diagonal-block task,
-//   the row-block tasks and the trailing-update tiles.
+//   large fronts: extend-add chunks, then per 64-column block J the row-block tasks, the
+//   trailing-update tiles and, beside them, the task of the next diagonal block (diag_next_body:
+//   it depends on block J's diagonal task and step J - 1 only, so the pivot chain of a front does
+//   not wait for the rest of step J).
 // Tasks are ordered level by level and, inside a level, phase by phase (every problem of the
 // batch in turn). A task waits only for tasks earlier in the queue: the fronts of its
 // children (all of their tasks done) and the earlier phases of its own front. Every task
 // earlier in the queue was claimed by a CTA that is already running, so the smallest
 // unfinished task can always proceed and the schedule cannot deadlock whatever the grid.
 //
-// Completion is counted per (problem, front): the last thread of a task's CTA publishes
+// Completion is counted per (problem, front), the diagonal blocks apart from the rest (rows and
+// updates of step J do not wait for the diagonal block J + 1): the last thread of a task's CTA publishes
 // its writes (barrier, then a gpu-scope fence and an atomic increment); a waiting CTA reads
 // the counter with a gpu-scope acquire load and releases its threads with a barrier.
 // Every wait is bounded: past the time limit the CTA records an error code and leaves, and
@@ -34,16 +37,24 @@
 namespace inla {
 namespace {
 
-enum PersistTaskType : int { PT_TINY = 0, PT_SMALL = 1, PT_GATHER = 2, PT_DIAG = 3, PT_ROWS = 4, PT_UPDATE = 5 };
+enum PersistTaskType : int {
+  PT_TINY = 0,
+  PT_SMALL = 1,
+  PT_GATHER = 2,
+  PT_DIAG = 3,    // the first diagonal block of a large front
+  PT_NEXT = 4,    // a later one (diag_next_body)
+  PT_ROWS = 5,
+  PT_UPDATE = 6
+};
 
 // One task of one problem (the batch repeats the per-problem list).
 struct PersistTask {
   int type;
   int s;      // front; PT_TINY: offset of the first front in the tiny list
   int sub;    // PT_TINY: number of fronts; PT_GATHER: chunk; PT_ROWS: row block; PT_UPDATE: tile
-  int need;   // tasks of the same front that must be done first (completion count)
+  int need;   // extend-add, row and update tasks of the same front that must be done first
   int j0;     // first column of the 64-column block (steps)
-  int gcols;  // PT_GATHER: columns per chunk
+  int arg;    // PT_GATHER: columns per chunk; steps: diagonal blocks of the front that must be done first
 };
 
 struct PersistArgs {
@@ -56,11 +67,10 @@ struct PersistArgs {
   const PersistTask* task;  // [gstart[ngroups]] per-problem tasks, group after group
   const int* tiny_list;     // fronts of the tiny tasks
   const int* total;         // [ns] tasks of each front (its completion count)
-  int* prog;                // [B][ns] completed tasks per (problem, front)
+  int* prog;                // [B][ns] completed tasks per (problem, front) other than diagonal blocks
+  int* dprog;               // [B][ns] factored diagonal blocks per (problem, front)
   unsigned* head;           // next task to claim
   int* err;                 // 0, or the reason the launch stopped early
-  double* dcache;           // [nlarge][B] factored diagonal blocks
-  const int* lid;           // [ns] index of a large front (-1 otherwise)
   double* linv;
   const int64_t* gptr;      // extend-add chunk table of this schedule
   const int2* grng;
@@ -96,7 +106,7 @@ __device__ bool wait_at_least(const int* p, int target, int* err, long long limi
     if (*(volatile int*)err != 0) return false;
     if (globaltimer_ns() - t0 > limit_ns) break;
     __nanosleep(sleep);
-    if (sleep < 1024) sleep <<= 1;
+    if (sleep < 128) sleep <<= 1;  // a step of the pivot chain is 15 us: long naps were a tenth of it
   }
   atomicCAS(err, 0, kErrTimeout);
   return false;
@@ -115,19 +125,13 @@ __device__ bool wait_children(const PersistArgs& a, int s, int b) {
 // warp tiles): every entry accumulates its products over K in the same order as any other warp
 // tiling of the same step, so the result does not depend on the tiling.
 //
-// kNext (look-ahead): tile 0 holds the next diagonal block [c, c + w') (w' = min(64, k - c))
-// once its update is done, so that CTA factors it right away, exactly as k_panel64 with no
-// rows would after this launch: the updated values go to shared memory as well as to the
-// front, cta_ldlt<true> factors them, and the CTA writes the factored block into the front,
-// D and L to dc_next (the cache slot of the next step; dc is this step's) and L^-1 to the
-// inverse-block cache. The other tiles of this launch read only block column J and their own
-// targets, so nothing else reads the block while it is factored. smu: kPanelSmem bytes.
-template <bool kNext = false>
+// dc == nullptr (chain form): D is read from the front, which already holds the factored diagonal
+// block; tile 0, the next diagonal block, is left to diag_next_body while the front has pivots left;
+// and tile 1, the rows below that block, also goes to its mirror position in the upper triangle, from
+// where the diag_next_body after next reads it.
 __device__ __forceinline__ void update64w8_body(const DevSym& S, int s, int b, int tile, int j0,
                                                 double* __restrict__ F, int64_t fstride,
-                                                const double* __restrict__ dc, double* smu,
-                                                double* __restrict__ dc_next = nullptr,
-                                                double* __restrict__ linv = nullptr) {
+                                                const double* __restrict__ dc, double* smu) {
   if (front_skipped(S, s, b)) return;
   constexpr int ld = kLd64;
   double* As = smu;              // As[t*ld + i] = L[I0+i, j0+t]
@@ -139,7 +143,8 @@ __device__ __forceinline__ void update64w8_body(const DevSym& S, int s, int b, i
   const int c = j0 + w;
   const int T = m - c;
   double* Fs = F + (int64_t)b * fstride + S.fptr[s];
-  if (tile == 0) {  // factored diagonal block -> front
+  if (!dc && tile == 0 && c < k) return;
+  if (dc && tile == 0) {  // factored diagonal block -> front
     double* D0 = Fs + j0 + (int64_t)j0 * m;
     for (int e = threadIdx.x; e < w * w; e += blockDim.x) {
       const int cc = e / w, r = e - cc * w;
@@ -166,7 +171,9 @@ __device__ __forceinline__ void update64w8_body(const DevSym& S, int s, int b, i
     else Bs[t * ld + ii] = 0.0;
   }
   cp_async_commit();
-  for (int t = threadIdx.x; t < kB64; t += blockDim.x) dsh[t] = t < w ? dc[t + t * kB64] : 0.0;
+  const double* dg = dc ? dc : Lb + j0;  // d_t at dg[t * ds]
+  const int64_t ds = dc ? kB64 + 1 : m + 1;
+  for (int t = threadIdx.x; t < kB64; t += blockDim.x) dsh[t] = t < w ? dg[t * ds] : 0.0;
   cp_async_wait<0>();
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -192,6 +199,7 @@ __device__ __forceinline__ void update64w8_body(const DevSym& S, int s, int b, i
 #pragma unroll
       for (int q = 0; q < 2; ++q) mma884(acc[a][q][0], acc[a][q][1], af[a], bf[q]);
   }
+  const bool mirror = !dc && tile == 1 && c + kB64 < k;
   double cv[4][2][2];  // read all targets before writing any (the loads stay in flight together)
 #pragma unroll
   for (int a = 0; a < 4; ++a)
@@ -212,39 +220,130 @@ __device__ __forceinline__ void update64w8_body(const DevSym& S, int s, int b, i
         const int i = I0 + wi + a * 8 + g;
         const int j = J0 + wj + q * 8 + tg * 2 + h;
         if (i < m && j < m && i >= j) Fs[i + (int64_t)j * m] = cv[a][q][h] - acc[a][q][h];
+        if (mirror && i < m) Fs[j + (int64_t)i * m] = cv[a][q][h] - acc[a][q][h];
       }
-  if (kNext && tile == 0 && c < k) {
-    const int wn = min(kB64, k - c);
-    double* Ds = smu;             // [64 cols][ld]: the next diagonal block, factored in place
-    double* Li = Ds + kB64 * ld;  // its L^-1
-    double* U = Li + kB64 * ld;
-    double* ws = U + 8 * kULd64;
-    __syncthreads();  // the operand tiles are consumed
-    for (int e = threadIdx.x; e < kB64 * kB64; e += blockDim.x) {
-      Ds[(e & 63) + (e >> 6) * ld] = 0.0;
-      Li[(e & 63) + (e >> 6) * ld] = 0.0;
-    }
-    __syncthreads();
+}
+
+// The pivot chain of a front in the chain form: the task of the diagonal block at j0 >= 64 (block J + 1)
+// needs only the block before it, so it runs while the other tasks of step J form its rows and update
+// the rest. It takes the 64 rows from j0 of block column J unscaled from their mirror position, forms
+// X = F L_JJ^-T D_J^-1 (as rows64_body does, which writes them), applies them to the 64 x 64 tile at
+// j0 (as tile 0 of the update would), factors the tile's pivot columns and writes the block into the
+// front and L^-1 to the inverse-block cache. Same arithmetic in the same order as the separate tasks:
+// bit-identical. 256 threads; smu: kPanelSmem bytes. What bounds it is the factorization of the 64
+// pivots (7.3 us of about 13).
+__device__ __forceinline__ void diag_next_body(const DevSym& S, int s, int b, int j0, double* __restrict__ F,
+                                               int64_t fstride, double* __restrict__ linv, double* smu) {
+  if (front_skipped(S, s, b)) return;
+  constexpr int ld = kLd64;
+  const int k = lg_k(S, s), m = lg_m(S, s);
+  if (j0 >= k) return;
+  double* Xs = smu;              // rows of block J, then X (Xs[t * ld + i]), then the block to factor
+  double* Bm = Xs + kB64 * ld;   // L_JJ^-T D^-1, then L^-1 of the new block
+  double* U = Bm + kB64 * ld;    // 1 / d, d, then scratch of cta_ldlt
+  double* ws = U + 8 * kULd64;
+  const int jp = j0 - kB64, w = min(kB64, k - j0), rows = min(kB64, m - j0);
+  double* Fs = F + (int64_t)b * fstride + S.fptr[s];
+  for (int e = threadIdx.x; e < kB64 * kB64; e += 256) {
+    const int t = e & 63, r = e >> 6;
+    if (r < rows) cp_async8(&Xs[t * ld + r], Fs + (jp + t) + (int64_t)(j0 + r) * m);
+    else Xs[t * ld + r] = 0.0;
+  }
+  cp_async_commit();
+  const double* lc = linv_block(S, linv, b, s, jp / kB64);
+  if (threadIdx.x < kB64) {
+    const double d = Fs[(jp + threadIdx.x) * (int64_t)(m + 1)];
+    U[threadIdx.x] = 1.0 / d;
+    U[kB64 + threadIdx.x] = d;
+  }
+  double lv[16];
+#pragma unroll
+  for (int q = 0; q < 16; ++q) lv[q] = lc[threadIdx.x + 256 * q];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int wi = (warp & 1) * 32, wj = (warp >> 1) * 16;
+  const int g = lane >> 2, tg = lane & 3;
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < 16; ++q) {
+    const int e = threadIdx.x + 256 * q, t = e & 63, u = e >> 6;
+    Bm[u + t * ld] = lv[q] * U[t];
+  }
+  cp_async_wait<0>();
+  __syncthreads();
+  double acc[4][2][2];
+  auto clear = [&] {
 #pragma unroll
     for (int a = 0; a < 4; ++a)
 #pragma unroll
-      for (int q = 0; q < 2; ++q)
+      for (int q = 0; q < 2; ++q) acc[a][q][0] = acc[a][q][1] = 0.0;
+  };
+  clear();
+#pragma unroll 4
+  for (int kk = 0; kk < kB64; kk += 4) {
+    double af[4], bf[2];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int r = wi + a * 8 + g, cc = wj + q * 8 + tg * 2 + h;  // I0 == J0 == c for tile 0
-          if (r < wn && cc < wn && r >= cc) Ds[r + cc * ld] = cv[a][q][h] - acc[a][q][h];
-        }
-    __syncthreads();
-    cta_ldlt<true>(Ds, ld, wn, wn, Li, ld, U, kULd64, ws);
-    double* D0 = Fs + c + (int64_t)c * m;
-    double* lc = const_cast<double*>(linv_block(S, linv, b, s, c / kB64));
-    for (int e = threadIdx.x; e < kB64 * kB64; e += blockDim.x) {
-      const int cc = e >> 6, r = e & 63;
-      const double v = (r < wn && cc < wn) ? Ds[r + cc * ld] : 0.0;
-      dc_next[e] = v;
-      lc[e] = Li[r + cc * ld];
-      if (r < wn && cc < wn && r >= cc) D0[r + (int64_t)cc * m] = v;
-    }
+    for (int a = 0; a < 4; ++a) af[a] = Xs[(kk + tg) * ld + wi + a * 8 + g];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) bf[q] = Bm[(kk + tg) + (wj + q * 8 + g) * ld];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int q = 0; q < 2; ++q) mma884(acc[a][q][0], acc[a][q][1], af[a], bf[q]);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) Xs[(wj + q * 8 + tg * 2 + h) * ld + wi + a * 8 + g] = acc[a][q][h];
+  for (int e = threadIdx.x; e < kB64 * kB64; e += 256) Bm[(e & 63) + (e >> 6) * ld] = 0.0;
+  __syncthreads();
+  double cv[4][2][2];  // the tile, in flight during the products
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int r = wi + a * 8 + g, cc = wj + q * 8 + tg * 2 + h;
+        cv[a][q][h] = (r < rows && r >= cc) ? Fs[(j0 + r) + (int64_t)(j0 + cc) * m] : 0.0;
+      }
+  clear();
+  const int wk = wj > wi + 31 ? 0 : kB64;
+#pragma unroll 2
+  for (int kk = 0; kk < wk; kk += 4) {
+    double af[4], bf[2];
+    const double dk = U[kB64 + kk + tg];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) af[a] = Xs[(kk + tg) * ld + wi + a * 8 + g];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) bf[q] = Xs[(kk + tg) * ld + wj + q * 8 + g] * dk;
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int q = 0; q < 2; ++q) mma884(acc[a][q][0], acc[a][q][1], af[a], bf[q]);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int r = wi + a * 8 + g, cc = wj + q * 8 + tg * 2 + h;
+        const double v = cv[a][q][h] - acc[a][q][h];
+        const bool low = r < rows && r >= cc, piv = r < w && cc < w;
+        Xs[r + cc * ld] = low && piv ? v : 0.0;
+        if (low && !piv) Fs[(j0 + r) + (int64_t)(j0 + cc) * m] = v;
+      }
+  __syncthreads();
+  cta_ldlt<true>(Xs, ld, w, w, Bm, ld, U, kULd64, ws);
+  double* ln = const_cast<double*>(linv_block(S, linv, b, s, j0 / kB64));
+  for (int e = threadIdx.x; e < kB64 * kB64; e += 256) {
+    const int cc = e >> 6, r = e & 63;
+    ln[e] = Bm[r + cc * ld];
+    if (r < w && r >= cc) Fs[(j0 + r) + (int64_t)(j0 + cc) * m] = Xs[r + cc * ld];
   }
 }
 
@@ -279,7 +378,8 @@ __global__ void __launch_bounds__(kPersistThreads, 2) k_factor_persist(PersistAr
       } else if (T.type == PT_SMALL || T.type == PT_GATHER) {
         ok = wait_children(a, T.s, b);
       } else {
-        ok = wait_at_least(pg + T.s, T.need, a.err, a.limit_ns);
+        ok = wait_at_least(pg + T.s, T.need, a.err, a.limit_ns) &&
+             (T.arg == 0 || wait_at_least(a.dprog + (int64_t)b * S.ns + T.s, T.arg, a.err, a.limit_ns));
       }
       sh_go = ok;
     }
@@ -300,19 +400,19 @@ __global__ void __launch_bounds__(kPersistThreads, 2) k_factor_persist(PersistAr
         factor_small_body<kPersistThreads>(S, T.s, b, a.F, a.fstride, psm);
         break;
       case PT_GATHER:
-        gather8_body(S, T.s, b, T.sub, a.F, a.fstride, T.gcols, a.gptr, a.grng, psm);
+        gather8_body(S, T.s, b, T.sub, a.F, a.fstride, T.arg, a.gptr, a.grng, psm);
         break;
       case PT_DIAG:
-        panel64_body(S, T.s, b, 0, T.j0, 0, a.F, a.fstride,
-                     a.dcache + ((int64_t)a.lid[T.s] * a.B + b) * (kB64 * kB64), a.linv, psm);
+        panel64_body(S, T.s, b, 0, T.j0, 0, a.F, a.fstride, nullptr, a.linv, psm);
+        break;
+      case PT_NEXT:
+        diag_next_body(S, T.s, b, T.j0, a.F, a.fstride, a.linv, psm);
         break;
       case PT_ROWS:
-        rows64_body(S, T.s, b, T.sub, T.j0, a.F, a.fstride,
-                    a.dcache + ((int64_t)a.lid[T.s] * a.B + b) * (kB64 * kB64), a.linv, psm);
+        rows64_body(S, T.s, b, T.sub, T.j0, a.F, a.fstride, nullptr, a.linv, psm);
         break;
       default:
-        update64w8_body(S, T.s, b, T.sub, T.j0, a.F, a.fstride,
-                        a.dcache + ((int64_t)a.lid[T.s] * a.B + b) * (kB64 * kB64), psm);
+        update64w8_body(S, T.s, b, T.sub, T.j0, a.F, a.fstride, nullptr, psm);
         break;
     }
     __syncthreads();  // every thread's writes of this task are issued
@@ -321,7 +421,8 @@ __global__ void __launch_bounds__(kPersistThreads, 2) k_factor_persist(PersistAr
       if (T.type == PT_TINY) {
         for (int u = 0; u < T.sub; ++u) atomicAdd(pg + a.tiny_list[T.s + u], 1);
       } else {
-        atomicAdd(pg + T.s, 1);
+        const bool diag = T.type == PT_DIAG || T.type == PT_NEXT;
+        atomicAdd((diag ? a.dprog + (int64_t)b * S.ns : pg) + T.s, 1);
       }
     }
   }
