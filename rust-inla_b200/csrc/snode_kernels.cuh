@@ -207,47 +207,73 @@ __device__ __forceinline__ void factor_small_body(const DevSym& S, int s, int b,
   double* A = sm;
   double* U = A + m * lda;
   double* ws = U + 8 * uld;
-  int* rs = reinterpret_cast<int*>(U);  // child relative indices (U is free until the factorization)
   double* Fs = Fb + S.fptr[s];
   const int mm = m * m;
-  for (int e = threadIdx.x; e < mm; e += NT) {
-    const int col = e / m, row = e - col * m;
-    if (col < k) cp_async8(&A[row + col * lda], Fs + e);
-    else A[row + col * lda] = 0.0;
-  }
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int nw = NT / 32;
+  // Column c belongs to warp c % nw: it stages the column, adds the children's columns in child order
+  // and never waits for another warp before the factorization. Children's descriptors are read 32 at a
+  // time, one per lane; of one child the warp's columns go four at a time, their loads together (one
+  // child after the other for the whole CTA, two barriers each: SPDE 200^2 at B = 15, fronts of 65 to
+  // 96 rows 1.30 -> 1.18 ms).
+  for (int col = warp; col < m; col += nw)
+    for (int row = lane; row < m; row += 32) {
+      if (col < k) cp_async8(&A[row + col * lda], Fs + row + col * m);
+      else A[row + col * lda] = 0.0;
+    }
   cp_async_commit();
+  const int q0 = S.child_ptr[s], nch = S.child_ptr[s + 1] - q0;
+  bool ready = false;
+  for (int qb = 0; qb < nch; qb += 32) {
+    int64_t src_l = 0;
+    int mc_l = 0, rc_l = 0, rp_l = 0;
+    if (qb + lane < nch) {
+      const int c = S.child_list[q0 + qb + lane];
+      const int kc = sn_k(S, c);
+      mc_l = sn_m(S, c);
+      rc_l = mc_l - kc;
+      rp_l = S.rowptr[c] + kc;
+      src_l = S.fptr[c] + (int64_t)kc * (mc_l + 1);
+    }
+    for (int q = 0; q < min(32, nch - qb); ++q) {
+      const int mc = __shfl_sync(0xffffffffu, mc_l, q), rc = __shfl_sync(0xffffffffu, rc_l, q);
+      const int rp = __shfl_sync(0xffffffffu, rp_l, q);
+      const double* Uc = Fb + __shfl_sync(0xffffffffu, src_l, q);
+      int rel[3];  // parent rows of the child's rows lane, lane + 32, lane + 64
+#pragma unroll
+      for (int h = 0; h < 3; ++h) rel[h] = lane + 32 * h < rc ? S.relx[rp + lane + 32 * h] : -1;
+#pragma unroll
+      for (int h0 = 0; h0 < 3; ++h0) {
+        unsigned own = __ballot_sync(0xffffffffu, rel[h0] >= 0 && rel[h0] % nw == warp);
+        while (own) {
+          double v[4][3];
+          int jj[4], pc[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int at = __ffs(own) - 1;
+            jj[u] = at < 0 ? 1 << 30 : at + 32 * h0;
+            pc[u] = __shfl_sync(0xffffffffu, rel[h0], at < 0 ? 0 : at);
+            own &= own - 1;
+#pragma unroll
+            for (int h = 0; h < 3; ++h) {
+              const int ii = lane + 32 * h;
+              v[u][h] = (ii < rc && ii >= jj[u]) ? Uc[ii + jj[u] * mc] : 0.0;
+            }
+          }
+          if (!ready) cp_async_wait<0>();
+          ready = true;
+          __syncwarp();
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int h = 0; h < 3; ++h)
+              if (rel[h] >= 0 && lane + 32 * h >= jj[u]) A[rel[h] + pc[u] * lda] += v[u][h];
+        }
+      }
+    }
+  }
   cp_async_wait<0>();
   __syncthreads();
-  for (int q = S.child_ptr[s]; q < S.child_ptr[s + 1]; ++q) {
-    const int c = S.child_list[q];
-    const int kc = sn_k(S, c), mc = sn_m(S, c), rc = mc - kc;
-    const double* Uc = Fb + S.fptr[c] + (int64_t)kc * mc + kc;
-    const int* relc = S.relx + S.rowptr[c] + kc;
-    for (int t = threadIdx.x; t < rc; t += NT) rs[t] = relc[t];
-    __syncthreads();
-    const int rr = rc * rc;
-    int e = threadIdx.x;
-    for (; e + 3 * NT < rr; e += 4 * NT) {
-      double v[4];
-      int dst[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int ee = e + u * NT;
-        const int jj = ee / rc, ii = ee - jj * rc;
-        const bool ok = ii >= jj;
-        v[u] = ok ? Uc[ii + (int64_t)jj * mc] : 0.0;
-        dst[u] = ok ? rs[ii] + rs[jj] * lda : -1;
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (dst[u] >= 0) A[dst[u]] += v[u];
-    }
-    for (; e < rr; e += NT) {
-      const int jj = e / rc, ii = e - jj * rc;
-      if (ii >= jj) A[rs[ii] + rs[jj] * lda] += Uc[ii + (int64_t)jj * mc];
-    }
-    __syncthreads();
-  }
   cta_ldlt<false>(A, lda, m, k, nullptr, 0, U, uld, ws);
   for (int e = threadIdx.x; e < mm; e += NT) {
     const int col = e / m, row = e - col * m;
