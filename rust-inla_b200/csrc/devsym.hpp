@@ -16,6 +16,10 @@ struct DevSym {
   const int* child_list = nullptr;
   const int* parent = nullptr;     // ns
   const int* uoff = nullptr;       // ns+1 : offsets of the per-supernode update vectors (sum r)
+  // children's update entries that add into each front row, in child order: entries
+  // rss[rsp[i] .. rsp[i + 1]) of the update vectors for row i of the concatenated structures
+  const int* rsp = nullptr;        // sum m + 1
+  const int* rss = nullptr;        // sum r
   const int64_t* dpos = nullptr;   // n : front offset of D_j
   const int* perm = nullptr;       // n : perm[new] = old
   // 64 x 64 inverse-block cache of the large fronts: block (s, j0 / 64) of

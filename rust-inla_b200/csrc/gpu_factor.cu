@@ -19,6 +19,8 @@ namespace inla {
 namespace {
 inline int cdiv(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }
 
+constexpr size_t kSolvePersistLevels = 8;  // see GpuFactor::solve
+
 // Panel forms of a level's large fronts (entries of the per-level schedule).
 constexpr char kFormSplit = 0, kFormFused = 1, kFormLookahead = 2, kNumForms = 3;
 // Process-wide panel form for engines built from now on: -1 the autotuner's choice per level
@@ -80,7 +82,7 @@ size_t g_maps_bytes = 0;
 
 size_t host_maps_bytes(const HostMaps& M) {
   return sizeof(int) * (M.first.size() + M.rowptr.size() + M.rows.size() + M.relx.size() + M.child_ptr.size() +
-                        M.child_list.size() + M.parent.size() + M.uoff.size() + M.perm.size() + M.pmap.size()) +
+                        M.child_list.size() + M.parent.size() + M.uoff.size() + M.perm.size() + M.pmap.size() + M.rsp.size() + M.rss.size()) +
          sizeof(int64_t) * (M.fptr.size() + M.lptr.size() + M.dpos.size() + M.spos.size() + M.spos_full.size());
 }
 
@@ -124,6 +126,25 @@ std::shared_ptr<const HostMaps> build_host_maps(const Symbolic& S) {
     }
   }
   for (int64_t j = 0; j < n; ++j) perm[j] = (int)S.perm[j];
+
+  // children's update entries per front row, in child order
+  {
+    const size_t nrows = S.sn_rows.size();
+    std::vector<int>&rsp = M.rsp, &rss = M.rss;
+    rsp.assign(nrows + 1, 0);
+    rss.resize(std::max(uoff[ns], 1));
+    auto each = [&](auto&& use) {  // (row of the parent, update entry), children in their list's order
+      for (int64_t s = 0; s < ns; ++s)
+        for (int q = child_ptr[s]; q < child_ptr[s + 1]; ++q) {
+          const int c = child_list[q], kc = first[c + 1] - first[c], rc = uoff[c + 1] - uoff[c];
+          for (int t = 0; t < rc; ++t) use(rowptr[s] + relx[rowptr[c] + kc + t], uoff[c] + t);
+        }
+    };
+    each([&](int row, int) { ++rsp[row + 1]; });
+    for (size_t i = 0; i < nrows; ++i) rsp[i + 1] += rsp[i];
+    std::vector<int> fill(rsp.begin(), rsp.end() - 1);
+    each([&](int row, int src) { rss[fill[row]++] = src; });
+  }
 
   // panel map (compact panel index -> input entry) and front positions of input entries
   std::vector<int>& pmap = M.pmap;
@@ -217,6 +238,8 @@ GpuFactor::GpuFactor(const Symbolic& sym, int max_batch, cudaStream_t stream)
   d_parent_.upload(parent, stream_);
   d_uoff_.upload(uoff, stream_);
   d_perm_.upload(perm, stream_);
+  d_rsp_.upload(M.rsp, stream_);
+  d_rss_.upload(M.rss, stream_);
   d_fptr_.upload(fptr, stream_);
   d_lptr_.upload(lptr, stream_);
   d_dpos_.upload(dpos, stream_);
@@ -238,6 +261,8 @@ GpuFactor::GpuFactor(const Symbolic& sym, int max_batch, cudaStream_t stream)
   ds_.uoff = d_uoff_.p;
   ds_.dpos = d_dpos_.p;
   ds_.perm = d_perm_.p;
+  ds_.rsp = d_rsp_.p;
+  ds_.rss = d_rss_.p;
 
   const auto tm2 = std::chrono::steady_clock::now();
   // inverse-block cache: one 64 x 64 block per 64 pivot columns of every large front
@@ -1157,7 +1182,13 @@ void GpuFactor::solve(double* d_x, int64_t xstride, int B, int slot0) {
   const double* Fp = F_.p + (int64_t)slot0 * fs;
   dim3 gp(cdiv(n, 256) > 1024 ? 1024 : cdiv(n, 256), B);
   auto pa = persist_at_.find(B);
-  const bool per = solve_persist_ && (persist_mode_ == 2 || (pa != persist_at_.end() && pa->second));
+  // Follows the factorization's choice on trees of at least kSolvePersistLevels levels, where the level
+  // launches (up to three per level and direction) cost more than the waits of the persistent sweep:
+  // 169 against 187 us on 13 levels (n = 900), 450 / 519 on 28 (n = 10 000), 514 / 585 on 18 (group
+  // 24x24x14). One level of one 902-row front: 208 against 122, the launch's one CTA per SM having
+  // twice the loads in flight.
+  const bool per = solve_persist_ && (persist_mode_ == 2 || (pa != persist_at_.end() && pa->second &&
+                                                             levels_.size() >= kSolvePersistLevels));
   if (per) {
     launch_cached({3, B, (int64_t)(uintptr_t)d_x, xstride, slot0, 1}, [&] {
       const int ns = (int)sym_.nsuper;

@@ -90,11 +90,12 @@ struct PersistPlan {
 };
 // Host tables of an analysis that an engine uploads: 32-bit copies of the supernode arrays,
 // front offsets fptr (sum m^2) and panel offsets lptr, D positions dpos, the panel map pmap
-// (compact panel index -> input entry) and the front positions of the input entries (spos:
+// (compact panel index -> input entry), the children's update entries of every front row (rsp, rss:
+// DevSym) and the front positions of the input entries (spos:
 // entries stored in a panel; spos_full: every entry). Shared by the engines built on one
 // analysis (cached by Symbolic::id).
 struct HostMaps {
-  std::vector<int> first, rowptr, rows, relx, child_ptr, child_list, parent, uoff, perm, pmap;
+  std::vector<int> first, rowptr, rows, relx, child_ptr, child_list, parent, uoff, perm, pmap, rsp, rss;
   std::vector<int64_t> fptr, lptr, dpos, spos, spos_full;
 };
 std::shared_ptr<const HostMaps> host_maps(const Symbolic& S);
@@ -214,7 +215,7 @@ class GpuFactor {
   int64_t ftotal_ = 0, nnz_ = 0, usum_ = 0;
   DevSym ds_;
   std::vector<LevelPlan> levels_;
-  DBuf<int> d_first_, d_rowptr_, d_rows_, d_relx_, d_child_ptr_, d_child_list_, d_parent_, d_uoff_, d_perm_;
+  DBuf<int> d_first_, d_rowptr_, d_rows_, d_relx_, d_child_ptr_, d_child_list_, d_parent_, d_uoff_, d_perm_, d_rsp_, d_rss_;
   DBuf<int64_t> d_fptr_, d_lptr_, d_dpos_, spos_, spos_full_, d_gptr_;
   DBuf<int2> d_grng_;  // extend-add source-column ranges per (front, chunk, child)
   DBuf<int> d_pmap_, d_lists_, d_csn_, d_csnm_, d_lbo_;

@@ -439,6 +439,24 @@ constexpr int kUT64 = 64;
 // (two barriers per block instead of one per column)
 // ---------------------------------------------------------------------------
 
+// v plus the children's update entries of front row `row` (of the concatenated structures), in child
+// order, eight loads in flight. One child after the other for the whole CTA, a barrier each, cost a
+// memory latency per child: fronts of grouped models have 20 to 324 of them (persistent solve of the
+// group model 24x24x14, B = 2: 1.30 -> 0.51 ms).
+__device__ __forceinline__ double fwd_row_start(const DevSym& S, int row, const double* __restrict__ ub, double v) {
+  int q = S.rsp[row];
+  const int e = S.rsp[row + 1];
+  for (; q + 8 <= e; q += 8) {
+    double u[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) u[i] = ub[S.rss[q + i]];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v += u[i];
+  }
+  for (; q < e; ++q) v += ub[S.rss[q]];
+  return v;
+}
+
 // Forward sweep of front s, problem b (NT threads; y: m + 2 + 32 * 33 doubles of shared memory).
 template <int NT>
 __device__ __forceinline__ void fwd32_body(const DevSym& S, int s, int b, const double* __restrict__ F,
@@ -448,16 +466,9 @@ __device__ __forceinline__ void fwd32_body(const DevSym& S, int s, int b, const 
   const double* Fs = F + (int64_t)b * fstride + S.fptr[s];
   double* xb = xp + (int64_t)b * S.n;
   double* ubb = ub + (int64_t)b * ustride;
-  for (int t = threadIdx.x; t < m; t += NT) y[t] = t < k ? xb[f + t] : 0.0;
+  for (int t = threadIdx.x; t < m; t += NT)
+    y[t] = fwd_row_start(S, S.rowptr[s] + t, ubb, t < k ? xb[f + t] : 0.0);
   __syncthreads();
-  for (int q = S.child_ptr[s]; q < S.child_ptr[s + 1]; ++q) {
-    const int c = S.child_list[q];
-    const int kc = lg_k(S, c), rc = lg_m(S, c) - kc;
-    const int* relc = S.relx + S.rowptr[c] + kc;
-    const double* uc = ubb + S.uoff[c];
-    for (int t = threadIdx.x; t < rc; t += NT) y[relc[t]] += uc[t];
-    __syncthreads();
-  }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double* Ls = y + ((m + 1) & ~1);  // [32][33] strictly lower part of the block's diagonal tile
   for (int jb = 0; jb < k; jb += 32) {
@@ -597,16 +608,9 @@ __device__ __forceinline__ void fwd64_body(const DevSym& S, int s, int b, const 
   const double* Fs = F + (int64_t)b * fstride + S.fptr[s];
   double* xb = xp + (int64_t)b * S.n;
   double* ubb = ub + (int64_t)b * ustride;
-  for (int t = threadIdx.x; t < m; t += NT) y[t] = t < k ? xb[f + t] : 0.0;
+  for (int t = threadIdx.x; t < m; t += NT)
+    y[t] = fwd_row_start(S, S.rowptr[s] + t, ubb, t < k ? xb[f + t] : 0.0);
   __syncthreads();
-  for (int q = S.child_ptr[s]; q < S.child_ptr[s + 1]; ++q) {
-    const int c = S.child_list[q];
-    const int kc = lg_k(S, c), rc = lg_m(S, c) - kc;
-    const int* relc = S.relx + S.rowptr[c] + kc;
-    const double* uc = ubb + S.uoff[c];
-    for (int t = threadIdx.x; t < rc; t += NT) y[relc[t]] += uc[t];
-    __syncthreads();
-  }
   const int nblk = (k + kB64 - 1) / kB64;
   for (int bi = 0; bi < nblk; ++bi) {
     const int jb = bi * kB64, wb = min(kB64, k - jb);
@@ -748,15 +752,7 @@ __device__ __forceinline__ void fwd_tiny_warp(const DevSym& S, int s, int b, con
   const double* Fs = F + (int64_t)b * fstride + S.fptr[s];
   double* xb = xp + (int64_t)b * S.n;
   double* ubb = ub + (int64_t)b * ustride;
-  y[lane] = lane < k ? xb[f + lane] : 0.0;
-  __syncwarp();
-  for (int q = S.child_ptr[s]; q < S.child_ptr[s + 1]; ++q) {
-    const int c = S.child_list[q];
-    const int kc = lg_k(S, c), rc = lg_m(S, c) - kc;
-    if (lane < rc) y[S.relx[S.rowptr[c] + kc + lane]] += ubb[S.uoff[c] + lane];
-    __syncwarp();
-  }
-  double yi = y[lane];
+  double yi = lane < m ? fwd_row_start(S, S.rowptr[s] + lane, ubb, lane < k ? xb[f + lane] : 0.0) : 0.0;
   {  // diagonal block: unit lower L_JJ
     double yd = lane < k ? yi : 0.0;
     for (int j = 0; j < k; ++j) {
