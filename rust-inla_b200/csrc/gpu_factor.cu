@@ -12,6 +12,7 @@
 #include "host_par.hpp"
 #include "snode_kernels.cuh"
 #include "snode_large.cuh"
+#include "snode_mini.cuh"
 #include "snode_persist.cuh"
 
 namespace inla {
@@ -487,6 +488,54 @@ void GpuFactor::plan_levels() {
   std::vector<int> flat;
   levels_ = make_level_plans(sym_, flat);
   d_lists_.upload(flat, stream_);
+  plan_minis();
+}
+
+// Bands of up to kMiniLevels consecutive levels whose fronts all have at most kMiniM rows, cut into the
+// tasks of snode_mini.cuh: the fronts of a band that are connected through parent links, children
+// first. (INLA_NO_TINY_FRONTS switches these off with the other small-front kernels.)
+void GpuFactor::plan_minis() {
+  const Symbolic& S = sym_;
+  const int L = (int)levels_.size();
+  band_at_.assign(L, -1);
+  static const bool on = std::getenv("INLA_NO_TINY_FRONTS") == nullptr;
+  if (!on) return;
+  std::vector<int> task(S.nsuper, -1);  // task of a front within the band being built
+  std::vector<int> ptr{0}, list;
+  for (int l = 0; l < L;) {
+    int e = l;
+    while (e < L && e - l < kMiniLevels && levels_[e].mmax_all <= kMiniM) ++e;
+    if (e - l < 2) {  // a single level gains nothing over the level kernels
+      l = std::max(e, l + 1);
+      continue;
+    }
+    // from the top level down: a front joins its parent's task if the parent lies in the band
+    const int off = (int)ptr.size() - 1;
+    std::vector<std::vector<int>> tasks;
+    for (int q = e - 1; q >= l; --q)
+      for (int s : levels_[q].all) {
+        const int64_t p = S.sn_parent[s];
+        task[s] = p >= 0 && task[p] >= 0 ? task[p] : (int)tasks.size();
+        if (task[s] == (int)tasks.size()) tasks.emplace_back();
+        tasks[task[s]].push_back(s);
+      }
+    // similar lengths side by side: the four tasks of a warp run for the longest of them
+    std::stable_sort(tasks.begin(), tasks.end(),
+                     [](const std::vector<int>& a, const std::vector<int>& b) { return a.size() > b.size(); });
+    for (const std::vector<int>& t : tasks) {
+      list.insert(list.end(), t.rbegin(), t.rend());
+      ptr.push_back((int)list.size());
+    }
+    for (int q = l; q < e; ++q) {
+      band_at_[q] = (int)bands_.size();
+      for (int s : levels_[q].all) task[s] = -1;
+    }
+    bands_.push_back({l, e, off, (int)tasks.size()});
+    l = e;
+  }
+  if (bands_.empty()) return;
+  d_mptr_.upload(ptr, stream_);
+  d_mlist_.upload(list, stream_);
 }
 
 // ---------------------------------------------------------------------------
@@ -909,6 +958,19 @@ void GpuFactor::run_factor_levels(int B, const std::vector<char>* fuse, cudaEven
   const int64_t fs = ftotal_;
   for (size_t li = 0; li < levels_.size(); ++li) {
     const LevelPlan& P = levels_[li];
+    if (band_at_[li] >= 0) {
+      const MiniBand& M = bands_[band_at_[li]];
+      if ((int)li == M.l0) {
+        k_factor_mini<<<dim3(cdiv(M.ntask, kMiniGroups), B), kMiniThreads, 0, stream_>>>(
+            ds_, d_mptr_.p + M.off, d_mlist_.p, M.ntask, F_.p, fs);
+        ++launches_;
+      }
+      if (ev) {
+        INLA_CUDA(cudaEventRecord(ev[2 * li], stream_));
+        INLA_CUDA(cudaEventRecord(ev[2 * li + 1], stream_));
+      }
+      continue;
+    }
     if (!P.tiny.empty()) {
       const int nt = (int)P.tiny.size();
       k_factor_tiny<<<dim3(cdiv(nt, kTinyWarps), B), 32 * kTinyWarps, 0, stream_>>>(ds_, d_lists_.p + P.off_tiny, nt,
@@ -1225,7 +1287,16 @@ void GpuFactor::solve(double* d_x, int64_t xstride, int B, int slot0) {
     const double* Lp = linv_.p + (int64_t)slot0 * ds_.lstride;
     // fronts of up to kSmallB rows (contiguous lists small_a, small_b) in 32-column blocks by one
     // CTA each; larger fronts in 64-column blocks with their cached inverse blocks
-    for (const LevelPlan& P : levels_) {
+    for (size_t li = 0; li < levels_.size(); ++li) {
+      const LevelPlan& P = levels_[li];
+      if (band_at_[li] >= 0) {
+        const MiniBand& M = bands_[band_at_[li]];
+        if ((int)li != M.l0) continue;
+        k_fwd_mini<<<dim3(cdiv(M.ntask, kMiniGroups), B), kMiniThreads, 0, stream_>>>(
+            ds_, d_mptr_.p + M.off, d_mlist_.p, M.ntask, Fp, fs, xp_.p, ub_.p, us);
+        ++launches_;
+        continue;
+      }
       if (!P.tiny.empty()) {
         const int nt = (int)P.tiny.size();
         k_fwd_tiny<<<dim3(cdiv(nt, kTinySweepWarps), B), 32 * kTinySweepWarps, 0, stream_>>>(
@@ -1250,6 +1321,14 @@ void GpuFactor::solve(double* d_x, int64_t xstride, int B, int slot0) {
     }
     for (int l = (int)levels_.size() - 1; l >= 0; --l) {
       const LevelPlan& P = levels_[l];
+      if (band_at_[l] >= 0) {
+        const MiniBand& M = bands_[band_at_[l]];
+        if (l != M.l0) continue;
+        k_bwd_mini<<<dim3(cdiv(M.ntask, kMiniGroups), B), kMiniThreads, 0, stream_>>>(
+            ds_, d_mptr_.p + M.off, d_mlist_.p, M.ntask, Fp, fs, xp_.p);
+        ++launches_;
+        continue;
+      }
       if (!P.tiny.empty()) {
         const int nt = (int)P.tiny.size();
         k_bwd_tiny<<<dim3(cdiv(nt, kTinySweepWarps), B), 32 * kTinySweepWarps, 0, stream_>>>(
@@ -1290,6 +1369,14 @@ void GpuFactor::selinv_levels(int B, int slot0) {
   const double* Lp = linv_.p + (int64_t)slot0 * ds_.lstride;
   for (int l = (int)levels_.size() - 1; l >= 0; --l) {
     const LevelPlan& P = levels_[l];
+    if (band_at_[l] >= 0) {
+      const MiniBand& M = bands_[band_at_[l]];
+      if (l != M.l0) continue;
+      k_selinv_mini<<<dim3(cdiv(M.ntask, kMiniGroups), B), kMiniThreads, 0, stream_>>>(
+          ds_, d_mptr_.p + M.off, d_mlist_.p, M.ntask, Fp, Sp, fs);
+      ++launches_;
+      continue;
+    }
     if (!P.si_tiny.empty()) {
       const int nt = (int)P.si_tiny.size();
       k_selinv_tiny<<<dim3(cdiv(nt, kTinySiWarps), B), 32 * kTinySiWarps, 0, stream_>>>(

@@ -79,6 +79,12 @@ struct LevelPlan {
   int off_si_tiny = 0, off_si_small = 0, off_si_large = 0, mmax_si_small = 0, kmax_si_small = 0, kmax_si_large = 0, mmax_si_large = 0, rmax_si_large = 0;
 };
 
+// Consecutive levels [l0, l1) whose fronts all have at most kMiniM rows: tasks off .. off + ntask of the
+// mini task table (snode_mini.cuh).
+struct MiniBand {
+  int l0, l1, off, ntask;
+};
+
 // Task queue of the persistent schedule for one problem (snode_persist.cuh): 6 ints per task
 // {type, front, sub, need, j0, arg}, group starts, tiny-front list, completion counts per
 // front, extend-add chunk table, shared memory in bytes.
@@ -215,6 +221,10 @@ class GpuFactor {
   int64_t ftotal_ = 0, nnz_ = 0, usum_ = 0;
   DevSym ds_;
   std::vector<LevelPlan> levels_;
+  std::vector<MiniBand> bands_;
+  std::vector<int> band_at_;         // band of a level, -1 none
+  DBuf<int> d_mptr_, d_mlist_;       // mini tasks: front ranges, fronts (children before parents)
+  void plan_minis();
   DBuf<int> d_first_, d_rowptr_, d_rows_, d_relx_, d_child_ptr_, d_child_list_, d_parent_, d_uoff_, d_perm_, d_rsp_, d_rss_;
   DBuf<int64_t> d_fptr_, d_lptr_, d_dpos_, spos_, spos_full_, d_gptr_;
   DBuf<int2> d_grng_;  // extend-add source-column ranges per (front, chunk, child)
