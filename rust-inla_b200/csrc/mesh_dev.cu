@@ -161,7 +161,8 @@ __device__ __forceinline__ int cell_of(double v, double lo, double inv_w, int g)
 // One point per thread: walk from the seed of the point's cell; flag 1 when certified.
 __global__ void __launch_bounds__(kNT) k_locate(MeshView m, Locator L, int64_t npts, const double* __restrict__ xy,
                                                int* __restrict__ tri_out, double* __restrict__ w_out,
-                                               unsigned char* __restrict__ flag, unsigned char* __restrict__ cnt) {
+                                               unsigned char* __restrict__ flag, unsigned char* __restrict__ cnt,
+                                               unsigned long long* __restrict__ open) {
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < npts; r += (int64_t)gridDim.x * blockDim.x) {
     const double px = xy[2 * r], py = xy[2 * r + 1];
     int start = 0;
@@ -174,6 +175,7 @@ __global__ void __launch_bounds__(kNT) k_locate(MeshView m, Locator L, int64_t n
     const int t = m.ntri > 0 ? walk_locate(m, start, px, py, L.maxsteps, L.delta, w, cert) : -1;
     tri_out[r] = t;
     flag[r] = (t >= 0 && cert) ? 1 : 0;
+    if (!flag[r]) atomicAdd(open, 1ull);
     for (int k = 0; k < 3; ++k) w_out[3 * r + k] = w[k];
     cnt[r] = (unsigned char)((fabs(w[0]) > kEps) + (fabs(w[1]) > kEps) + (fabs(w[2]) > kEps));
   }
@@ -181,12 +183,94 @@ __global__ void __launch_bounds__(kNT) k_locate(MeshView m, Locator L, int64_t n
 
 __global__ void __launch_bounds__(kNT) k_apply_fix(int64_t nfix, const int64_t* __restrict__ idx,
                                                   const int* __restrict__ tri, const double* __restrict__ w,
-                                                  int* __restrict__ tri_out, double* __restrict__ w_out) {
+                                                  int* __restrict__ tri_out, double* __restrict__ w_out,
+                                                  unsigned char* __restrict__ cnt) {
   for (int64_t f = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; f < nfix; f += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = idx[f];
     tri_out[r] = tri[f];
-    for (int k = 0; k < 3; ++k) w_out[3 * r + k] = w[3 * f + k];
+    int c = 0;
+    for (int k = 0; k < 3; ++k) {
+      w_out[3 * r + k] = w[3 * f + k];
+      c += fabs(w[3 * f + k]) > kEps;
+    }
+    cnt[r] = (unsigned char)c;
   }
+}
+
+// Row pointers of the projector from the entry counts: sums of kScan points per CTA, their prefix by one
+// CTA (total in *total), then the prefix within each CTA. The counts stay on the device: through the
+// host (counts, flags and triangles down, row pointers up, pageable copies and two loops) a projector
+// of 50 000 points waited 0.4 ms for 15 us of kernels; the scan takes 7 us.
+constexpr int kScan = 8 * kNT;
+__global__ void __launch_bounds__(kNT) k_scan_sums(int64_t npts, const unsigned char* __restrict__ cnt,
+                                                  int64_t* __restrict__ sums) {
+  __shared__ int red[kNT / 32];
+  int v = 0;
+  for (int u = 0; u < 8; ++u) {
+    const int64_t r = blockIdx.x * (int64_t)kScan + u * kNT + threadIdx.x;
+    if (r < npts) v += cnt[r];
+  }
+  v = __reduce_add_sync(0xffffffffu, v);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int64_t t = 0;
+    for (int w = 0; w < kNT / 32; ++w) t += red[w];
+    sums[blockIdx.x] = t;
+  }
+}
+
+__device__ __forceinline__ int64_t warp_scan(int64_t v) {  // inclusive
+  for (int o = 1; o < 32; o <<= 1) {
+    const int64_t u = __shfl_up_sync(0xffffffffu, v, o);
+    if ((int)(threadIdx.x & 31) >= o) v += u;
+  }
+  return v;
+}
+
+__global__ void __launch_bounds__(1024) k_scan_top(int64_t nblk, int64_t* __restrict__ sums,
+                                                  unsigned long long* __restrict__ total) {
+  __shared__ int64_t part[32];
+  __shared__ int64_t carry;
+  if (threadIdx.x == 0) carry = 0;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int64_t i0 = 0; i0 < nblk; i0 += 1024) {
+    __syncthreads();
+    const int64_t i = i0 + threadIdx.x, v = i < nblk ? sums[i] : 0, incl = warp_scan(v);
+    if (lane == 31) part[warp] = incl;
+    __syncthreads();
+    if (warp == 0) part[lane] = warp_scan(part[lane]);
+    __syncthreads();
+    const int64_t base = carry + (warp > 0 ? part[warp - 1] : 0);
+    if (i < nblk) sums[i] = base + incl - v;
+    __syncthreads();
+    if (threadIdx.x == 0) carry += part[31];
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) *total = (unsigned long long)carry;
+}
+
+__global__ void __launch_bounds__(kNT) k_scan_write(int64_t npts, const unsigned char* __restrict__ cnt,
+                                                   const int64_t* __restrict__ sums, int64_t* __restrict__ rowptr) {
+  __shared__ int64_t part[kNT / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t r0 = blockIdx.x * (int64_t)kScan + 8 * threadIdx.x;  // eight consecutive points per thread
+  int c[8], mine = 0;
+  for (int u = 0; u < 8; ++u) {
+    c[u] = r0 + u < npts ? cnt[r0 + u] : 0;
+    mine += c[u];
+  }
+  const int64_t incl = warp_scan(mine);
+  if (lane == 31) part[warp] = incl;
+  __syncthreads();
+  int64_t at = sums[blockIdx.x] + incl - mine;
+  for (int w = 0; w < warp; ++w) at += part[w];
+  for (int u = 0; u < 8; ++u)
+    if (r0 + u < npts) {
+      rowptr[r0 + u] = at;
+      at += c[u];
+      if (r0 + u == npts - 1) rowptr[npts] = at;
+    }
 }
 
 // Row r of the projector: weights with |w| > 1e-15, columns ascending.
@@ -195,6 +279,7 @@ __global__ void __launch_bounds__(kNT) k_proj_write(MeshView m, int64_t npts, co
                                                    int64_t* __restrict__ colidx, double* __restrict__ vals) {
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < npts; r += (int64_t)gridDim.x * blockDim.x) {
     const int t = tri[r];
+    if (t < 0) continue;  // not located yet: the host's walk settles the point and the rows are written again
     int col[3];
     double val[3];
     int ne = 0;
@@ -365,9 +450,8 @@ std::string projector_device(const Mesh2D& m, MeshDevPlan& p, int64_t npts, cons
                              int64_t* d_colidx, double* d_vals, int64_t* nnz_out, cudaStream_t st) {
   std::string err = ensure_mesh_device(m, p, st);
   if (!err.empty()) return err;
-  std::vector<int64_t> rp(npts + 1, 0);
   if (npts == 0) {
-    INLA_CUDA(cudaMemcpyAsync(d_rowptr, rp.data(), sizeof(int64_t), cudaMemcpyHostToDevice, st));
+    INLA_CUDA(cudaMemsetAsync(d_rowptr, 0, sizeof(int64_t), st));
     INLA_CUDA(cudaStreamSynchronize(st));
     if (nnz_out) *nnz_out = 0;
     return std::string();
@@ -387,58 +471,63 @@ std::string projector_device(const Mesh2D& m, MeshDevPlan& p, int64_t npts, cons
   L.inv_wx = p.inv_wx;
   L.inv_wy = p.inv_wy;
   L.delta = p.delta;
-  k_locate<<<grid_for(npts), kNT, 0, st>>>(mv, L, npts, d_xy, p.ptri.p, p.pw.p, p.pflag.p, p.pcnt.p);
+  const int64_t nblk = (npts + kScan - 1) / kScan;
+  p.psums.alloc(nblk);
+  p.pmeta.alloc(2);  // points left to the host, entries
+  INLA_CUDA(cudaMemsetAsync(p.pmeta.p, 0, sizeof(unsigned long long), st));
+  k_locate<<<grid_for(npts), kNT, 0, st>>>(mv, L, npts, d_xy, p.ptri.p, p.pw.p, p.pflag.p, p.pcnt.p, p.pmeta.p);
   INLA_CUDA(cudaGetLastError());
   ++g_launches;
-  std::vector<unsigned char> flag(npts), cnt(npts);
-  std::vector<int> tri(npts);
-  INLA_CUDA(cudaMemcpyAsync(flag.data(), p.pflag.p, npts, cudaMemcpyDeviceToHost, st));
-  INLA_CUDA(cudaMemcpyAsync(cnt.data(), p.pcnt.p, npts, cudaMemcpyDeviceToHost, st));
-  INLA_CUDA(cudaMemcpyAsync(tri.data(), p.ptri.p, npts * sizeof(int), cudaMemcpyDeviceToHost, st));
-  INLA_CUDA(cudaStreamSynchronize(st));
-  // points without a certified location: the reference's walk in point order, each from the
-  // previous point's triangle, as the host projector runs it
-  std::vector<int64_t> fidx;
-  std::vector<int> ftri;
-  std::vector<double> fw;
-  std::vector<double> xy;
-  for (int64_t r = 0; r < npts; ++r) {
-    if (flag[r]) continue;
-    if (xy.empty()) {
-      xy.resize(2 * npts);
-      INLA_CUDA(cudaMemcpyAsync(xy.data(), d_xy, 2 * npts * sizeof(double), cudaMemcpyDeviceToHost, st));
-      INLA_CUDA(cudaStreamSynchronize(st));
+  unsigned long long meta[2] = {0, 0};
+  auto rows = [&] {  // row pointers and entries from the counts, triangles and weights
+    k_scan_sums<<<(unsigned)nblk, kNT, 0, st>>>(npts, p.pcnt.p, p.psums.p);
+    k_scan_top<<<1, 1024, 0, st>>>(nblk, p.psums.p, p.pmeta.p + 1);
+    k_scan_write<<<(unsigned)nblk, kNT, 0, st>>>(npts, p.pcnt.p, p.psums.p, d_rowptr);
+    k_proj_write<<<grid_for(npts), kNT, 0, st>>>(mv, npts, p.ptri.p, p.pw.p, d_rowptr, d_colidx, d_vals);
+    INLA_CUDA(cudaGetLastError());
+    g_launches += 4;
+    INLA_CUDA(cudaMemcpyAsync(meta, p.pmeta.p, sizeof(meta), cudaMemcpyDeviceToHost, st));
+    INLA_CUDA(cudaStreamSynchronize(st));
+  };
+  rows();
+  if (meta[0] > 0) {
+    // points without a certified location: the reference's walk in point order, each from the
+    // previous point's triangle, as the host projector runs it
+    std::vector<unsigned char> flag(npts);
+    std::vector<int> tri(npts);
+    std::vector<double> xy(2 * npts);
+    INLA_CUDA(cudaMemcpyAsync(flag.data(), p.pflag.p, npts, cudaMemcpyDeviceToHost, st));
+    INLA_CUDA(cudaMemcpyAsync(tri.data(), p.ptri.p, npts * sizeof(int), cudaMemcpyDeviceToHost, st));
+    INLA_CUDA(cudaMemcpyAsync(xy.data(), d_xy, 2 * npts * sizeof(double), cudaMemcpyDeviceToHost, st));
+    INLA_CUDA(cudaStreamSynchronize(st));
+    std::vector<int64_t> fidx;
+    std::vector<int> ftri;
+    std::vector<double> fw;
+    for (int64_t r = 0; r < npts; ++r) {
+      if (flag[r]) continue;
+      double w[3];
+      const int64_t t = locate_point(m, r == 0 ? 0 : tri[r - 1], xy[2 * r], xy[2 * r + 1], w);
+      if (t < 0) {
+        char buf[128];
+        std::snprintf(buf, sizeof(buf), "observation point (%.17g, %.17g) is outside the mesh", xy[2 * r],
+                      xy[2 * r + 1]);
+        return buf;
+      }
+      tri[r] = (int)t;
+      fidx.push_back(r);
+      ftri.push_back((int)t);
+      fw.insert(fw.end(), w, w + 3);
     }
-    double w[3];
-    const int64_t t = locate_point(m, r == 0 ? 0 : tri[r - 1], xy[2 * r], xy[2 * r + 1], w);
-    if (t < 0) {
-      char buf[128];
-      std::snprintf(buf, sizeof(buf), "observation point (%.17g, %.17g) is outside the mesh", xy[2 * r],
-                    xy[2 * r + 1]);
-      return buf;
-    }
-    tri[r] = (int)t;
-    fidx.push_back(r);
-    ftri.push_back((int)t);
-    fw.insert(fw.end(), w, w + 3);
-    cnt[r] = (unsigned char)((std::fabs(w[0]) > kEps) + (std::fabs(w[1]) > kEps) + (std::fabs(w[2]) > kEps));
-  }
-  if (!fidx.empty()) {
     const int64_t nfix = (int64_t)fidx.size();
     p.fix_idx.upload(fidx, st);
     p.fix_tri.upload(ftri, st);
     p.fix_w.upload(fw, st);
-    k_apply_fix<<<grid_for(nfix), kNT, 0, st>>>(nfix, p.fix_idx.p, p.fix_tri.p, p.fix_w.p, p.ptri.p, p.pw.p);
+    k_apply_fix<<<grid_for(nfix), kNT, 0, st>>>(nfix, p.fix_idx.p, p.fix_tri.p, p.fix_w.p, p.ptri.p, p.pw.p, p.pcnt.p);
     INLA_CUDA(cudaGetLastError());
     ++g_launches;
+    rows();
   }
-  for (int64_t r = 0; r < npts; ++r) rp[r + 1] = rp[r] + cnt[r];
-  INLA_CUDA(cudaMemcpyAsync(d_rowptr, rp.data(), (npts + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, st));
-  k_proj_write<<<grid_for(npts), kNT, 0, st>>>(mv, npts, p.ptri.p, p.pw.p, d_rowptr, d_colidx, d_vals);
-  INLA_CUDA(cudaGetLastError());
-  ++g_launches;
-  INLA_CUDA(cudaStreamSynchronize(st));
-  if (nnz_out) *nnz_out = rp[npts];
+  if (nnz_out) *nnz_out = (int64_t)meta[1];
   return std::string();
 }
 

@@ -55,7 +55,8 @@ struct MeshDevPlan {
   DBuf<int> ptri;
   DBuf<double> pw;
   DBuf<unsigned char> pflag, pcnt;
-  DBuf<int64_t> fix_idx;
+  DBuf<int64_t> fix_idx, psums;
+  DBuf<unsigned long long> pmeta;
   DBuf<int> fix_tri;
   DBuf<double> fix_w;
 };

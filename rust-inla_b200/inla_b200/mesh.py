@@ -67,6 +67,12 @@ class Mesh:
         check(lib().inla_mesh_fem_pattern(self._h, w, None, lptr(cp), lptr(ri)))
         return cp, ri
 
+    def _fem_nnz(self, which):
+        """Entries of FEM block ``which`` (index into ``FEM_BLOCKS``) without copying its pattern."""
+        nnz = C.c_int64()
+        check(lib().inla_mesh_fem_pattern(self._h, which, C.byref(nnz), None, None))
+        return nnz.value
+
     def fem_device(self, triangle_scale=None, diffusion=None):
         """The blocks of ``fem`` computed on the current CUDA device: dict of float64 tensors of
         the values on ``fem_pattern``'s patterns, plus ``areas``; ``triangle_scale`` a device
@@ -76,8 +82,8 @@ class Mesh:
 
         dev = torch.device("cuda", torch.cuda.current_device())
         out = {"areas": torch.empty(self.ntri, dtype=torch.float64, device=dev)}
-        for name in FEM_BLOCKS:
-            out[name] = torch.empty(len(self.fem_pattern(name)[1]), dtype=torch.float64, device=dev)
+        for which, name in enumerate(FEM_BLOCKS):
+            out[name] = torch.empty(self._fem_nnz(which), dtype=torch.float64, device=dev)
         sc = None
         if triangle_scale is not None:
             sc = torch.as_tensor(triangle_scale, dtype=torch.float64, device=dev).expand(self.ntri).contiguous()
