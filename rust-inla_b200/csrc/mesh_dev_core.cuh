@@ -112,6 +112,17 @@ __host__ __device__ inline double fem_contrib(int which, int64_t code, const Mes
   return rmul(rmul(g.scale, g.e[k][j]), vij);
 }
 
+// The c1 and g1 values of one contribution of their common list, as fem_contrib gives them.
+__host__ __device__ inline void fem_contrib_c1g1(int64_t code, const MeshView& m, const double* tscale, double hxx,
+                                                 double hxy, double hyy, double& c1, double& g1) {
+  const int64_t t = code / 9;
+  const int s = (int)(code - 9 * t), a = slot_a(s), b = slot_b(s);
+  TriGeom g;
+  tri_geom(m, t, tscale, hxx, hxy, hyy, g);
+  c1 = a == b ? rdiv(g.area, 6.0) : rdiv(g.area, 12.0);
+  g1 = rdiv(rmul(g.scale, g.e[a][b]), rmul(4.0, g.fa));
+}
+
 // The reference's walk (fmesher.rs:221-263) from `start`, at most `maxsteps` triangles. Returns
 // the accepting triangle with its barycentric weights, or -1 when the walk left the mesh or ran
 // out of steps. certified: every edge test in that triangle exceeds delta and the weights are
