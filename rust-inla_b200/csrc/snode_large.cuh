@@ -26,7 +26,8 @@ constexpr int kPanelRows = 64;   // rows per panel GEMM sub-block
 constexpr int kLd64 = dense_ld(kB64);
 constexpr int kULd64 = dense_uld(kB64);
 constexpr int kPanelSmem = (2 * kB64 * kLd64 + 8 * kULd64 + kDenseScratch) * 8;
-constexpr int kSiGemmSmem = 3 * 64 * kLd64 * 8;  // three stage buffers
+constexpr int kSiStages = 2, kSiCtas = 3;
+constexpr int kSiGemmSmem = kSiStages * 64 * kLd64 * 8;  // stage buffers
 
 __device__ __forceinline__ int lg_k(const DevSym& S, int s) { return S.first[s + 1] - S.first[s]; }
 __device__ __forceinline__ int lg_m(const DevSym& S, int s) { return S.rowptr[s + 1] - S.rowptr[s]; }
@@ -170,7 +171,9 @@ __device__ __forceinline__ void gather8_body(const DevSym& S, int s, int b, int 
     gather_column(S, s, Fb, Fb + S.fptr[s], k, m, c0 + cc, rng, gsl + (int64_t)cc * m);
 }
 
-__global__ void __launch_bounds__(256) k_gather8(DevSym S, const int* __restrict__ list, double* __restrict__ F,
+// 48 registers: five CTAs per SM even with a few spills (79 registers, three CTAs: 3.20 ms instead of
+// 2.58 in the SPDE 200^2 factorization at B = 30; 64 and four: 2.73).
+__global__ void __launch_bounds__(256, 5) k_gather8(DevSym S, const int* __restrict__ list, double* __restrict__ F,
                                                  int64_t fstride, int gcols, const int64_t* __restrict__ gptr,
                                                  const int2* __restrict__ grng) {
   extern __shared__ double gsl[];  // [gcols][m] column slice
@@ -861,7 +864,7 @@ __device__ __forceinline__ void si_gemm_body(const DevSym& S, int s, int b, int 
                                              const double* __restrict__ F, double* __restrict__ Sg, int64_t fstride,
                                              const double* __restrict__ linv, double* smem64) {
   constexpr int ld = kLd64, kBuf = 64 * kLd64;  // one stage: As[32][ld], Bs[32][ld]
-  __shared__ double scale[3][32];
+  __shared__ double scale[kSiStages][32];
   const int k = lg_k(S, s), m = lg_m(S, s);
   const int nblk = (k + kB64 - 1) / kB64, rt = (m - k + kSiT - 1) / kSiT;
   const int half = TM == 32 ? (z & 1) : 0;
@@ -969,13 +972,14 @@ __device__ __forceinline__ void si_gemm_body(const DevSym& S, int s, int b, int 
     for (int q = 0; q < 2; ++q) acc[a][q][0] = acc[a][q][1] = 0.0;
   const int nc = (t1 - t0 + 31) / 32;
   load_chunk(t0, 0);
-  if (nc > 1) load_chunk(t0 + 32, 1);
+  if (kSiStages > 2 && nc > 1) load_chunk(t0 + 32, 1);
   for (int c = 0; c < nc; ++c) {
-    if (c + 1 < nc) cp_async_wait<1>();
+    if (kSiStages > 2 && c + 1 < nc) cp_async_wait<1>();
     else cp_async_wait<0>();
     __syncthreads();  // chunk c has landed, and every warp is done with chunk c - 1
-    if (c + 2 < nc) load_chunk(t0 + 32 * (c + 2), (c + 2) % 3);
-    const double* As = smem64 + (c % 3) * kBuf;
+    constexpr int kAhead = kSiStages - 1;
+    if (c + kAhead < nc) load_chunk(t0 + 32 * (c + kAhead), (c + kAhead) % kSiStages);
+    const double* As = smem64 + (c % kSiStages) * kBuf;
     const double* Bs = As + 32 * ld;
     if (wact) {
 #pragma unroll
@@ -986,7 +990,7 @@ __device__ __forceinline__ void si_gemm_body(const DevSym& S, int s, int b, int 
 #pragma unroll
         for (int q = 0; q < 2; ++q) bf[q] = Bs[(kk + tg) * ld + wj + q * 8 + g];
         if (MODE == SI_KK) {
-          const double sc = scale[c % 3][kk + tg];
+          const double sc = scale[c % kSiStages][kk + tg];
           bf[0] *= sc;
           bf[1] *= sc;
         }
@@ -1026,7 +1030,7 @@ __device__ __forceinline__ void si_gemm_body(const DevSym& S, int s, int b, int 
 }
 
 template <int MODE, int TM>
-__global__ void __launch_bounds__(256, 2) k_si_gemm(DevSym S, const int* __restrict__ list, int hb,
+__global__ void __launch_bounds__(256, kSiCtas) k_si_gemm(DevSym S, const int* __restrict__ list, int hb,
                                                     const double* __restrict__ F, double* __restrict__ Sg,
                                                     int64_t fstride, const double* __restrict__ linv) {
   extern __shared__ double smem64[];

@@ -174,11 +174,22 @@ __device__ __forceinline__ void update64w8_body(const DevSym& S, int s, int b, i
   const double* dg = dc ? dc : Lb + j0;  // d_t at dg[t * ds]
   const int64_t ds = dc ? kB64 + 1 : m + 1;
   for (int t = threadIdx.x; t < kB64; t += blockDim.x) dsh[t] = t < w ? dg[t * ds] : 0.0;
-  cp_async_wait<0>();
-  __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int wi = (warp & 1) * 32, wj = (warp >> 1) * 16;
   const int g = lane >> 2, tg = lane & 3;
+  double cv[4][2][2];  // all targets, in flight beside the operands
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int i = I0 + wi + a * 8 + g;
+        const int j = J0 + wj + q * 8 + tg * 2 + h;
+        cv[a][q][h] = (i < m && j < m && i >= j) ? Fs[i + (int64_t)j * m] : 0.0;
+      }
+  cp_async_wait<0>();
+  __syncthreads();
   double acc[4][2][2];
 #pragma unroll
   for (int a = 0; a < 4; ++a)
@@ -200,17 +211,6 @@ __device__ __forceinline__ void update64w8_body(const DevSym& S, int s, int b, i
       for (int q = 0; q < 2; ++q) mma884(acc[a][q][0], acc[a][q][1], af[a], bf[q]);
   }
   const bool mirror = !dc && tile == 1 && c + kB64 < k;
-  double cv[4][2][2];  // read all targets before writing any (the loads stay in flight together)
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int q = 0; q < 2; ++q)
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int i = I0 + wi + a * 8 + g;
-        const int j = J0 + wj + q * 8 + tg * 2 + h;
-        cv[a][q][h] = (i < m && j < m && i >= j) ? Fs[i + (int64_t)j * m] : 0.0;
-      }
 #pragma unroll
   for (int a = 0; a < 4; ++a)
 #pragma unroll
