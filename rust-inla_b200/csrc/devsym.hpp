@@ -35,6 +35,29 @@ struct DevSym {
   int nseg = 1;
 };
 
+// Tables of the bands of small fronts (snode_mini.cuh). A front: its F offset, rows, pivots, first entry in
+// the child table, and the F offset and rows of its parent.
+struct alignas(16) MiniFront {
+  int64_t fptr;
+  int rowptr, first;
+  int k, m, child0, nch;
+  int64_t pptr;
+  int pm, uoff;
+};
+// A child's update block: F offset of its first entry, its place in relx, rows of the child * 16 + rows of
+// the block.
+struct alignas(16) MiniChild {
+  int64_t src;
+  int rel, dim;
+};
+// Task ranges, fronts in task order (children before parents; `list`: their numbers) and their children.
+struct MiniTables {
+  const int* ptr;
+  const int* list;
+  const MiniFront* front;
+  const MiniChild* child;
+};
+
 __host__ __device__ inline bool front_skipped(const DevSym& S, int s, int b) {
   return S.active && !S.active[(int64_t)b * S.nseg + S.fseg[s]];
 }

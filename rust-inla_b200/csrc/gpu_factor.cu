@@ -308,7 +308,7 @@ GpuFactor::GpuFactor(const Symbolic& sym, int max_batch, cudaStream_t stream)
   INLA_CUDA(cudaMemsetAsync(ldticket_.p, 0, sizeof(unsigned) * max_batch_, stream_));
 
   const auto tm3 = std::chrono::steady_clock::now();
-  plan_levels();
+  plan_levels(M);
   // extend-add range table: for every large front, column chunk z (of the
   // level's gcols columns) and child, the child's source columns whose parent
   // column lies in the chunk
@@ -484,17 +484,17 @@ std::vector<LevelPlan> make_level_plans(const Symbolic& S, std::vector<int>& fla
   return levels;
 }
 
-void GpuFactor::plan_levels() {
+void GpuFactor::plan_levels(const HostMaps& maps) {
   std::vector<int> flat;
   levels_ = make_level_plans(sym_, flat);
   d_lists_.upload(flat, stream_);
-  plan_minis();
+  plan_minis(maps);
 }
 
 // Bands of up to kMiniLevels consecutive levels whose fronts all have at most kMiniM rows, cut into the
 // tasks of snode_mini.cuh: the fronts of a band that are connected through parent links, children
 // first. (INLA_NO_TINY_FRONTS switches these off with the other small-front kernels.)
-void GpuFactor::plan_minis() {
+void GpuFactor::plan_minis(const HostMaps& maps) {
   const Symbolic& S = sym_;
   const int L = (int)levels_.size();
   band_at_.assign(L, -1);
@@ -534,8 +534,24 @@ void GpuFactor::plan_minis() {
     l = e;
   }
   if (bands_.empty()) return;
+  std::vector<MiniFront> front;
+  std::vector<MiniChild> child;
+  front.reserve(list.size());
+  auto rows = [&](int s) { return maps.rowptr[s + 1] - maps.rowptr[s]; };
+  auto pivots = [&](int s) { return maps.first[s + 1] - maps.first[s]; };
+  for (int s : list) {
+    const int p = maps.parent[s], c0 = maps.child_ptr[s], c1 = maps.child_ptr[s + 1];
+    front.push_back({maps.fptr[s], maps.rowptr[s], maps.first[s], pivots(s), rows(s), (int)child.size(), c1 - c0,
+                     p < 0 ? 0 : maps.fptr[p], p < 0 ? 0 : rows(p), maps.uoff[s]});
+    for (int q = c0; q < c1; ++q) {
+      const int c = maps.child_list[q], kc = pivots(c), mc = rows(c);
+      child.push_back({maps.fptr[c] + (int64_t)kc * mc + kc, maps.rowptr[c] + kc, mc * 16 + (mc - kc)});
+    }
+  }
   d_mptr_.upload(ptr, stream_);
   d_mlist_.upload(list, stream_);
+  d_mfront_.upload(front, stream_);
+  d_mchild_.upload(child, stream_);
 }
 
 // ---------------------------------------------------------------------------
@@ -962,7 +978,7 @@ void GpuFactor::run_factor_levels(int B, const std::vector<char>* fuse, cudaEven
       const MiniBand& M = bands_[band_at_[li]];
       if ((int)li == M.l0) {
         k_factor_mini<<<dim3(cdiv(M.ntask, kMiniGroups), B), kMiniThreads, 0, stream_>>>(
-            ds_, d_mptr_.p + M.off, d_mlist_.p, M.ntask, F_.p, fs);
+            ds_, mini_tables(M.off), M.ntask, F_.p, fs);
         ++launches_;
       }
       if (ev) {
@@ -1293,7 +1309,7 @@ void GpuFactor::solve(double* d_x, int64_t xstride, int B, int slot0) {
         const MiniBand& M = bands_[band_at_[li]];
         if ((int)li != M.l0) continue;
         k_fwd_mini<<<dim3(cdiv(M.ntask, kMiniGroups), B), kMiniThreads, 0, stream_>>>(
-            ds_, d_mptr_.p + M.off, d_mlist_.p, M.ntask, Fp, fs, xp_.p, ub_.p, us);
+            ds_, mini_tables(M.off), M.ntask, Fp, fs, xp_.p, ub_.p, us);
         ++launches_;
         continue;
       }
@@ -1325,7 +1341,7 @@ void GpuFactor::solve(double* d_x, int64_t xstride, int B, int slot0) {
         const MiniBand& M = bands_[band_at_[l]];
         if (l != M.l0) continue;
         k_bwd_mini<<<dim3(cdiv(M.ntask, kMiniGroups), B), kMiniThreads, 0, stream_>>>(
-            ds_, d_mptr_.p + M.off, d_mlist_.p, M.ntask, Fp, fs, xp_.p);
+            ds_, mini_tables(M.off), M.ntask, Fp, fs, xp_.p);
         ++launches_;
         continue;
       }
@@ -1373,7 +1389,7 @@ void GpuFactor::selinv_levels(int B, int slot0) {
       const MiniBand& M = bands_[band_at_[l]];
       if (l != M.l0) continue;
       k_selinv_mini<<<dim3(cdiv(M.ntask, kMiniGroups), B), kMiniThreads, 0, stream_>>>(
-          ds_, d_mptr_.p + M.off, d_mlist_.p, M.ntask, Fp, Sp, fs);
+          ds_, mini_tables(M.off), M.ntask, Fp, Sp, fs);
       ++launches_;
       continue;
     }

@@ -190,7 +190,7 @@ class GpuFactor {
   int persist_wait_limit_selftest(double limit_ms);
 
  private:
-  void plan_levels();
+  void plan_levels(const HostMaps& maps);
   // fuse: per level, 1 = each row CTA factors the diagonal block itself, 0 = one CTA
   // factors it and k_rows64 forms the rows; nullptr = the occupancy rule. ev: events
   // recorded before and after every level's large-front work (2 per level).
@@ -223,8 +223,11 @@ class GpuFactor {
   std::vector<LevelPlan> levels_;
   std::vector<MiniBand> bands_;
   std::vector<int> band_at_;         // band of a level, -1 none
-  DBuf<int> d_mptr_, d_mlist_;       // mini tasks: front ranges, fronts (children before parents)
-  void plan_minis();
+  DBuf<int> d_mptr_, d_mlist_;       // mini tasks (MiniTables)
+  DBuf<MiniFront> d_mfront_;
+  DBuf<MiniChild> d_mchild_;
+  void plan_minis(const HostMaps& maps);
+  MiniTables mini_tables(int off) const { return {d_mptr_.p + off, d_mlist_.p, d_mfront_.p, d_mchild_.p}; }
   DBuf<int> d_first_, d_rowptr_, d_rows_, d_relx_, d_child_ptr_, d_child_list_, d_parent_, d_uoff_, d_perm_, d_rsp_, d_rss_;
   DBuf<int64_t> d_fptr_, d_lptr_, d_dpos_, spos_, spos_full_, d_gptr_;
   DBuf<int2> d_grng_;  // extend-add source-column ranges per (front, chunk, child)

@@ -6,13 +6,20 @@
 // row i), and one launch does all tasks of a band. Everything a front needs from another front of its
 // band was written by the same eight lanes, so warp synchronization orders it.
 //
-// Bounded by the latency of a front's dependent loads (descriptor, structure, values) times the length
-// of a task; 4 fronts per warp and 32 per CTA in 18 KB keep up to 256 fronts per SM in flight instead
-// of 24. A front of a task costs 5 to 6 us however many run beside it, so bands are short: 4 levels
-// take 0.23 ms per factorization of the models below, 8 levels 0.37 (tasks of up to 20 fronts), 16
-// levels 0.58.
-// 96 uneven AR1 + iid models (134 k fronts, 39 levels, B = 2), per call: factorization 465 -> 229 us,
-// forward sweep 349 -> 158, backward sweep 215 -> 99, selected inverse 700 -> 270.
+// Bounded by the instructions and the load latency of one front after the other in a task (2.7 us per
+// front of the factorization with few tasks on the chip; with many, half of the issue slots are taken).
+// So what a front needs besides its children's results is loaded before the front below it is finished:
+// its line of the front table (two ahead), the panel (copied to shared memory without going through
+// registers), its children's lines and its rows' places. Reading these through list, first, rowptr, fptr
+// and child_list when the front's turn came cost 5 to 6 us per front. Bands are short because a task is as
+// long as the fronts that hang together: 4 levels give tasks of up to 9 fronts and 0.17 ms per
+// factorization of the models below, 6 levels 0.25, 8 levels 0.34.
+// Registers: a spill costs more than a resident CTA gains (factorization, 4 / 5 / 6 / 8 CTAs of 128
+// threads: 172 / 179 / 200 / 251 us); leaving the unrolled loops at the warp's largest front costs more
+// than the skipped steps (224 us).
+// 96 uneven AR1 + iid models (134 k fronts, 39 levels, B = 2), per call, level launches -> bands -> with
+// the loads ahead: factorization 465 -> 229 -> 172 us, forward sweep 349 -> 164 -> 106, backward sweep
+// 215 -> 100 -> 82, selected inverse 700 -> 275 -> 158.
 //
 // Per front the arithmetic and its order are those of the one-warp kernels (factor_tiny_warp,
 // fwd_tiny_warp, bwd_tiny_warp, k_selinv_tiny): same bits.
@@ -30,62 +37,90 @@ namespace {
 constexpr int kMiniM = 8;          // rows of a front
 constexpr int kMiniLd = kMiniM + 1;
 constexpr int kMiniLevels = 4;     // levels of a band
-constexpr int kMiniGroups = 32;    // tasks per CTA (8 lanes each)
+constexpr int kMiniGroups = 16;    // tasks per CTA (8 lanes each)
 constexpr int kMiniThreads = kMiniGroups * 8;
 
-// The caller's task: fronts list[f0 .. f0 + len), and the longest task of the warp.
+// The caller's task: fronts f0 .. f0 + len of the table, and the longest task of the warp.
 struct MiniTask {
   int f0, len, longest;
 };
-__device__ __forceinline__ MiniTask mini_task(const DevSym& S, const int* __restrict__ ptr,
-                                              const int* __restrict__ list, int ntask, int b, bool skip) {
+__device__ __forceinline__ MiniTask mini_task(const DevSym& S, const MiniTables& M, int ntask, int b, bool skip) {
   MiniTask t{0, 0, 0};
   const int c = blockIdx.x * kMiniGroups + (threadIdx.x >> 3);
   if (c < ntask) {
-    t.f0 = ptr[c];
-    t.len = ptr[c + 1] - t.f0;
-    if (skip && front_skipped(S, list[t.f0], b)) t.len = 0;  // a task lies within one model
+    t.f0 = M.ptr[c];
+    t.len = M.ptr[c + 1] - t.f0;
+    if (skip && front_skipped(S, M.list[t.f0], b)) t.len = 0;  // a task lies within one model
   }
   t.longest = __reduce_max_sync(0xffffffffu, t.len);
   return t;
 }
+// Front `it` of the task, parents first for `Up` = false; a front without rows past the end.
+template <bool Up>
+__device__ __forceinline__ MiniFront mini_front(const MiniTables& M, const MiniTask& T, int it) {
+  if (it >= T.len) return MiniFront{};
+  return M.front[T.f0 + (Up ? it : T.len - 1 - it)];
+}
 
-__global__ void __launch_bounds__(kMiniThreads) k_factor_mini(DevSym S, const int* __restrict__ ptr,
-                                                              const int* __restrict__ list, int ntask,
+__global__ void __launch_bounds__(kMiniThreads, 4) k_factor_mini(DevSym S, MiniTables M, int ntask,
                                                               double* __restrict__ F, int64_t fstride) {
-  __shared__ double sA[kMiniGroups][kMiniM * kMiniLd];
+  __shared__ double sA[2][kMiniGroups][kMiniM * kMiniLd];
   const int l = threadIdx.x & 7, b = blockIdx.y;
-  double* A = sA[threadIdx.x >> 3];
   double* Fb = F + (int64_t)b * fstride;
-  const MiniTask T = mini_task(S, ptr, list, ntask, b, true);
-  for (int it = 0; it < T.longest; ++it) {
-    const bool on = it < T.len;
-    const int s = on ? list[T.f0 + it] : 0;
-    const int k = on ? sn_k(S, s) : 0, m = on ? sn_m(S, s) : 0;
-    double* Fs = Fb + S.fptr[s];
-    const int q0 = S.child_ptr[s], nch = on ? S.child_ptr[s + 1] - q0 : 0;
-    const int kmax = __reduce_max_sync(0xffffffffu, k), cmax = __reduce_max_sync(0xffffffffu, nch);
+  const MiniTask T = mini_task(S, M, ntask, b, true);
+  MiniFront cur = mini_front<true>(M, T, 0), nxt = mini_front<true>(M, T, 1);
+  MiniChild ch{0, 0, 0};  // child l of the front that comes next
+  auto prefetch = [&](const MiniFront& f, double* A) {
 #pragma unroll
-    for (int j = 0; j < kMiniM; ++j) A[l + j * kMiniLd] = (l < m && j < k) ? Fs[l + j * m] : 0.0;
+    for (int j = 0; j < kMiniM; ++j) {
+      if (l < f.m && j < f.k) cp_async8(&A[l + j * kMiniLd], Fb + f.fptr + l + j * f.m);
+      else A[l + j * kMiniLd] = 0.0;
+    }
+    cp_async_commit();
+    if (l < f.nch) ch = M.child[f.child0 + l];
+  };
+  prefetch(cur, sA[0][threadIdx.x >> 3]);
+  for (int it = 0; it < T.longest; ++it) {
+    const int k = cur.k, m = cur.m, nch = cur.nch, child0 = cur.child0;
+    double* Fs = Fb + cur.fptr;
+    double* A = sA[it & 1][threadIdx.x >> 3];
+    const int kmax = __reduce_max_sync(0xffffffffu, k), cmax = __reduce_max_sync(0xffffffffu, nch);
+    MiniChild mine = ch;
+    double v[kMiniM];  // row l of the update of child q, and its place in the parent
+    int rel, rc;
+    auto fetch = [&](int q) {
+      const int64_t src = __shfl_sync(0xffffffffu, mine.src, q & 7, 8);
+      const int dim = __shfl_sync(0xffffffffu, mine.dim, q & 7, 8);
+      const int r0 = __shfl_sync(0xffffffffu, mine.rel, q & 7, 8);
+      rc = q < nch ? dim & 15 : 0;
+      rel = 0;
+      if (l < rc) {
+        rel = S.relx[r0 + l];
+#pragma unroll
+        for (int j = 0; j < kMiniM; ++j) v[j] = j <= l ? Fb[src + l + (int64_t)j * (dim >> 4)] : 0.0;
+      }
+    };
+    fetch(0);
+    cur = nxt;
+    nxt = mini_front<true>(M, T, it + 2);
+    prefetch(cur, sA[(it + 1) & 1][threadIdx.x >> 3]);
+    cp_async_wait<1>();
     __syncwarp();
     for (int q = 0; q < cmax; ++q) {
-      int rel = 0, rc = 0;
-      double v[kMiniM];
-      if (q < nch) {
-        const int c = S.child_list[q0 + q], kc = sn_k(S, c), mc = sn_m(S, c);
-        rc = mc - kc;
-        const double* Uc = Fb + S.fptr[c] + (int64_t)kc * mc + kc;
-        if (l < rc) {
-          rel = S.relx[S.rowptr[c] + kc + l];
-#pragma unroll
-          for (int j = 0; j < kMiniM; ++j) v[j] = j <= l ? Uc[l + j * mc] : 0.0;
-        }
+      if (q) {
+        if ((q & 7) == 0 && q + l < nch) mine = M.child[child0 + q + l];
+        fetch(q);
       }
+      double t[kMiniM];  // the targets of one child are distinct: all loads before the stores
+      int at[kMiniM];
 #pragma unroll
       for (int j = 0; j < kMiniM; ++j) {
-        const int pc = __shfl_sync(0xffffffffu, rel, j, 8);
-        if (l < rc && j <= l) A[rel + pc * kMiniLd] += v[j];
+        at[j] = rel + __shfl_sync(0xffffffffu, rel, j, 8) * kMiniLd;
+        if (l < rc && j <= l) t[j] = A[at[j]];
       }
+#pragma unroll
+      for (int j = 0; j < kMiniM; ++j)
+        if (l < rc && j <= l) A[at[j]] = t[j] + v[j];
       __syncwarp();
     }
     double a[kMiniM];
@@ -111,30 +146,59 @@ __global__ void __launch_bounds__(kMiniThreads) k_factor_mini(DevSym S, const in
   }
 }
 
-__global__ void __launch_bounds__(kMiniThreads) k_fwd_mini(DevSym S, const int* __restrict__ ptr,
-                                                           const int* __restrict__ list, int ntask,
+__global__ void __launch_bounds__(kMiniThreads, 6) k_fwd_mini(DevSym S, MiniTables M, int ntask,
                                                            const double* __restrict__ F, int64_t fstride, double* xp,
                                                            double* ub, int64_t ustride) {
+  __shared__ double sL[2][kMiniM][kMiniThreads];  // row l of the panels (D at l < k), per thread
   const int l = threadIdx.x & 7, b = blockIdx.y;
   const double* Fb = F + (int64_t)b * fstride;
   double* xb = xp + (int64_t)b * S.n;
   double* ubb = ub + (int64_t)b * ustride;
-  const MiniTask T = mini_task(S, ptr, list, ntask, b, false);
-  for (int it = 0; it < T.longest; ++it) {
-    const bool on = it < T.len;
-    const int s = on ? list[T.f0 + it] : 0;
-    const int k = on ? lg_k(S, s) : 0, m = on ? lg_m(S, s) : 0, f = S.first[s];
-    const double* Fs = Fb + S.fptr[s];
-    const int kmax = __reduce_max_sync(0xffffffffu, k);
-    double L[kMiniM];  // row l of the panel, D at l < k
-#pragma unroll
-    for (int j = 0; j < kMiniM; ++j) L[j] = (l < m && j < k && j <= l) ? Fs[l + j * m] : 0.0;
-    double yi = 0.0;
-    if (l < m) {
-      yi = l < k ? xb[f + l] : 0.0;
-      const int row = S.rowptr[s] + l;
-      for (int q = S.rsp[row], e = S.rsp[row + 1]; q < e; ++q) yi += ubb[S.rss[q]];
+  const MiniTask T = mini_task(S, M, ntask, b, false);
+  // fronts it, it + 1, it + 2; of front it: the right-hand side and the first two of the row's children
+  // entries; of front it + 1: the row's range of entries
+  MiniFront cur = mini_front<true>(M, T, 0), nxt = mini_front<true>(M, T, 1), nx2 = mini_front<true>(M, T, 2);
+  double x = 0.0;
+  int e0 = 0, e1 = 0, n0 = 0, n1 = 0, s0 = 0, s1 = 0;
+  auto range = [&](const MiniFront& f) {
+    n0 = n1 = 0;
+    if (l < f.m) {
+      n0 = S.rsp[f.rowptr + l];
+      n1 = S.rsp[f.rowptr + l + 1];
     }
+  };
+  auto prefetch = [&](const MiniFront& f, int it) {
+    e0 = n0;
+    e1 = n1;
+    if (e0 < e1) s0 = S.rss[e0];
+    if (e0 + 1 < e1) s1 = S.rss[e0 + 1];
+#pragma unroll
+    for (int j = 0; j < kMiniM; ++j)
+      if (l < f.m && j < f.k && j <= l) cp_async8(&sL[it & 1][j][threadIdx.x], Fb + f.fptr + l + j * f.m);
+    cp_async_commit();
+    x = l < f.k ? xb[f.first + l] : 0.0;
+  };
+  range(cur);
+  prefetch(cur, 0);
+  range(nxt);
+  for (int it = 0; it < T.longest; ++it) {
+    const int k = cur.k, m = cur.m, f = cur.first, uo = cur.uoff;
+    const int kmax = __reduce_max_sync(0xffffffffu, k);
+    const double u0 = e0 < e1 ? ubb[s0] : 0.0, u1 = e0 + 1 < e1 ? ubb[s1] : 0.0;
+    double yi = x;
+    const int q0 = e0, q1 = e1;
+    cur = nxt;
+    nxt = nx2;
+    nx2 = mini_front<true>(M, T, it + 3);
+    prefetch(cur, it + 1);
+    range(nxt);
+    if (q0 < q1) yi += u0;
+    if (q0 + 1 < q1) yi += u1;
+    for (int q = q0 + 2; q < q1; ++q) yi += ubb[S.rss[q]];
+    cp_async_wait<1>();
+    double L[kMiniM];
+#pragma unroll
+    for (int j = 0; j < kMiniM; ++j) L[j] = (l < m && j < k && j <= l) ? sL[it & 1][j][threadIdx.x] : 0.0;
     double yd = l < k ? yi : 0.0;
 #pragma unroll
     for (int j = 0; j < kMiniM; ++j) {
@@ -149,42 +213,45 @@ __global__ void __launch_bounds__(kMiniThreads) k_fwd_mini(DevSym S, const int* 
       const double yj = __shfl_sync(0xffffffffu, yd, j, 8);
       if (j < k) a[j & 3] += L[j] * yj;
     }
-    double d = 1.0;
-#pragma unroll
-    for (int j = 0; j < kMiniM; ++j)
-      if (j == l) d = L[j];
-    if (l < k) xb[f + l] = yd / d;
-    else if (l < m) ubb[S.uoff[s] + l - k] = yi - ((a[0] + a[1]) + (a[2] + a[3]));
+    if (l < k) xb[f + l] = yd / sL[it & 1][l][threadIdx.x];
+    else if (l < m) ubb[uo + l - k] = yi - ((a[0] + a[1]) + (a[2] + a[3]));
     __syncwarp();
   }
 }
 
-__global__ void __launch_bounds__(kMiniThreads) k_bwd_mini(DevSym S, const int* __restrict__ ptr,
-                                                           const int* __restrict__ list, int ntask,
+__global__ void __launch_bounds__(kMiniThreads, 6) k_bwd_mini(DevSym S, MiniTables M, int ntask,
                                                            const double* __restrict__ F, int64_t fstride, double* xp) {
+  __shared__ double sB[2][kMiniM][kMiniThreads], sC[2][kMiniM][kMiniThreads];  // L[k + l][j], L[j][l]
   const int l = threadIdx.x & 7, b = blockIdx.y;
   const double* Fb = F + (int64_t)b * fstride;
   double* xb = xp + (int64_t)b * S.n;
-  const MiniTask T = mini_task(S, ptr, list, ntask, b, false);
-  for (int it = 0; it < T.longest; ++it) {  // parents first
-    const bool on = it < T.len;
-    const int s = on ? list[T.f0 + T.len - 1 - it] : 0;
-    const int k = on ? lg_k(S, s) : 0, m = on ? lg_m(S, s) : 0, f = S.first[s];
-    const double* Fs = Fb + S.fptr[s];
-    const int kmax = __reduce_max_sync(0xffffffffu, k);
-    const int ri = k + l;
-    double Lb[kMiniM], Lc[kMiniM];  // L[ri][j] and L[i][l]
+  const MiniTask T = mini_task(S, M, ntask, b, false);
+  MiniFront cur = mini_front<false>(M, T, 0), nxt = mini_front<false>(M, T, 1);
+  int row = 0;
+  auto prefetch = [&](const MiniFront& f, int it) {
+    const double* Fs = Fb + f.fptr;
 #pragma unroll
     for (int j = 0; j < kMiniM; ++j) {
-      Lb[j] = (ri < m && j < k) ? Fs[ri + j * m] : 0.0;
-      Lc[j] = (j < k && l < j) ? Fs[j + l * m] : 0.0;
+      if (f.k + l < f.m && j < f.k) cp_async8(&sB[it & 1][j][threadIdx.x], Fs + f.k + l + j * f.m);
+      if (j < f.k && l < j) cp_async8(&sC[it & 1][j][threadIdx.x], Fs + j + l * f.m);
     }
-    double xl = l < m ? xb[S.rows[S.rowptr[s] + l]] : 0.0;
+    cp_async_commit();
+    if (l < f.m) row = S.rows[f.rowptr + l];
+  };
+  prefetch(cur, 0);
+  for (int it = 0; it < T.longest; ++it) {
+    const int k = cur.k, m = cur.m, f = cur.first, ri = k + l;
+    const int kmax = __reduce_max_sync(0xffffffffu, k);
+    double xl = l < m ? xb[row] : 0.0;
+    cur = nxt;
+    nxt = mini_front<false>(M, T, it + 2);
+    prefetch(cur, it + 1);
+    cp_async_wait<1>();
     const double xs = __shfl_sync(0xffffffffu, xl, ri & 7, 8);
 #pragma unroll
     for (int j = 0; j < kMiniM; ++j) {
       if (j >= kmax) break;
-      double acc = ri < m ? Lb[j] * xs : 0.0;
+      double acc = ri < m && j < k ? sB[it & 1][j][threadIdx.x] * xs : 0.0;
 #pragma unroll
       for (int o = 4; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o, 8);
       acc = __shfl_sync(0xffffffffu, acc, 0, 8);
@@ -194,15 +261,14 @@ __global__ void __launch_bounds__(kMiniThreads) k_bwd_mini(DevSym S, const int* 
     for (int i = kMiniM - 1; i >= 0; --i) {
       if (i >= kmax) continue;
       const double xi = __shfl_sync(0xffffffffu, xl, i, 8);
-      if (i < k && l < i) xl -= Lc[i] * xi;
+      if (i < k && l < i) xl -= sC[it & 1][i][threadIdx.x] * xi;
     }
     if (l < k) xb[f + l] = xl;
     __syncwarp();
   }
 }
 
-__global__ void __launch_bounds__(kMiniThreads) k_selinv_mini(DevSym S, const int* __restrict__ ptr,
-                                                              const int* __restrict__ list, int ntask,
+__global__ void __launch_bounds__(kMiniThreads, 6) k_selinv_mini(DevSym S, MiniTables M, int ntask,
                                                               const double* __restrict__ F, double* Sg,
                                                               int64_t fstride) {
   __shared__ double sS[kMiniGroups][kMiniM * kMiniLd];
@@ -212,34 +278,36 @@ __global__ void __launch_bounds__(kMiniThreads) k_selinv_mini(DevSym S, const in
   double* L = sL[threadIdx.x >> 3];
   const double* Fb = F + (int64_t)b * fstride;
   double* Sb = Sg + (int64_t)b * fstride;
-  const MiniTask T = mini_task(S, ptr, list, ntask, b, false);
-  for (int it = 0; it < T.longest; ++it) {  // parents first
-    const bool on = it < T.len;
-    const int s = on ? list[T.f0 + T.len - 1 - it] : 0;
-    const int k = on ? sn_k(S, s) : 0, m = on ? sn_m(S, s) : 0, r = m - k;
-    const double* Fs = Fb + S.fptr[s];
-    double* Ss = Sb + S.fptr[s];
+  const MiniTask T = mini_task(S, M, ntask, b, false);
+  MiniFront cur = mini_front<false>(M, T, 0), nxt = mini_front<false>(M, T, 1);
+  double pv[kMiniM];  // row l of the panel, and the place of below-row l, of the front that comes next
+  int rel = 0;
+  auto prefetch = [&](const MiniFront& f) {
+#pragma unroll
+    for (int j = 0; j < kMiniM; ++j) pv[j] = (l < f.m && j < f.k) ? Fb[f.fptr + l + j * f.m] : 0.0;
+    if (l < f.m - f.k) rel = S.relx[f.rowptr + f.k + l];
+  };
+  prefetch(cur);
+  for (int it = 0; it < T.longest; ++it) {
+    const int k = cur.k, m = cur.m, r = m - k;
+    double* Ss = Sb + cur.fptr;
     const int kmax = __reduce_max_sync(0xffffffffu, k);
+    double v[kMiniM];
+#pragma unroll
+    for (int j = 0; j < kMiniM; ++j) {
+      const int rj = __shfl_sync(0xffffffffu, rel, j, 8);
+      v[j] = j <= l && l < r ? parent_sigma(Sb + cur.pptr, cur.pm, rel, rj) : 0.0;
+      if (l < m && j < k) L[l + j * kMiniLd] = pv[j];
+    }
+    cur = nxt;
+    nxt = mini_front<false>(M, T, it + 2);
+    prefetch(cur);
 #pragma unroll
     for (int j = 0; j < kMiniM; ++j)
-      if (l < m && j < k) L[l + j * kMiniLd] = Fs[l + j * m];
-    if (r > 0) {
-      const int p = S.parent[s], mp = sn_m(S, p);
-      const double* Sp = Sb + S.fptr[p];
-      const int* rel = S.relx + S.rowptr[s] + k;
-      if (l < r) {
-        const int ri = rel[l];
-        double v[kMiniM];
-#pragma unroll
-        for (int j = 0; j < kMiniM; ++j) v[j] = j <= l ? parent_sigma(Sp, mp, ri, rel[j]) : 0.0;
-#pragma unroll
-        for (int j = 0; j < kMiniM; ++j)
-          if (j <= l) {
-            Sm[(k + l) + (k + j) * kMiniLd] = v[j];
-            Sm[(k + j) + (k + l) * kMiniLd] = v[j];
-          }
+      if (j <= l && l < r) {
+        Sm[(k + l) + (k + j) * kMiniLd] = v[j];
+        Sm[(k + j) + (k + l) * kMiniLd] = v[j];
       }
-    }
     __syncwarp();
     for (int jj = kmax - 1; jj >= 0; --jj) {
       const bool col = jj < k, mine = col && l > jj && l < m;
