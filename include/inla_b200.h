@@ -287,8 +287,8 @@ int inla_set_persistent_schedule(int mode);
  * (default) the autotuner's per-level choice (on the first factorization at a batch size the
  * level sequence is timed in each form and every level keeps the fastest); 0 split (diagonal
  * block, rows, trailing update: three launches per 64-column step); 1 fused (every row CTA
- * factors the diagonal block: two launches); 2 look-ahead (rows, then the trailing update
- * whose first tile also factors the next diagonal block: two launches). All forms give
+ * factors the diagonal block: two launches); 2 look-ahead (rows and trailing update, and beside
+ * them, on a stream of its own, the next diagonal block: three launches). All forms give
  * bit-identical factors. */
 int inla_set_panel_form(int form);
 /* Diagnostic of the bounded waits: runs the persistent factorization once with completion

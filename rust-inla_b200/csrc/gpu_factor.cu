@@ -1073,8 +1073,8 @@ void GpuFactor::run_factor_levels(int B, const std::vector<char>* fuse, cudaEven
 // 64 x 64 diagonal block, k_rows64 forms the rows from the cached factor, then the
 // trailing update: three launches per step), "fused" (each of the nrb row CTAs
 // factors the diagonal block itself, then the update: two launches) and
-// "look-ahead" (rows, then the update whose tile-0 CTAs factor the next diagonal
-// block: two launches per step plus one for the first block). Which is faster
+// "look-ahead" (rows and update, and beside them on a stream of its own k_diag_next, which
+// needs only the previous diagonal block: three launches per step). Which is faster
 // depends on the level's fronts, the batch size and the GPU, so on the first
 // factorization at a batch size B the level sequence runs once in each form
 // (after a fill, untimed warm-up first) with CUDA events around every level's

@@ -6,7 +6,9 @@
 //               dense routine (cta_ldlt, which also forms L_JJ^-1); CTA 0
 //               stores the factored block (dcache) and L_JJ^-1 (the inverse-
 //               block cache, reused by the selected inverse); each CTA forms
-//               its 64 rows L_i = F_i L_JJ^-T D_J^-1 as one tensor-core GEMM;
+//               its 64 rows L_i = F_i L_JJ^-T D_J^-1 as one tensor-core GEMM
+//               (or one CTA per front factors the block and k_rows64 forms the
+//               rows; or k_diag_next factors it while step J - 1 is in work);
 //   update      F[i,j] -= sum_{t in J} L_it d_t L_jt on 64x64 tiles of the lower
 //               trailing matrix (tensor-core tiles, operands staged with cp.async;
 //               update64w8_body in snode_persist.cuh, launched as k_update64w8).
@@ -846,7 +848,8 @@ constexpr int kSiT = 64;  // rows of B per tile
 //
 // X and W live transposed in the strictly upper triangle of the front's Sigma buffer (block (I, J) of X
 // at (J, I), W at (K, B)), which nothing else uses; the products L_21 X_11 in the lower block that
-// Sigma_KK takes at the end. One CTA per 64 x 64 tile, K in chunks of 32 through three cp.async stages.
+// Sigma_KK takes at the end. One CTA per 64 x 64 tile, K in chunks of 32 through two cp.async stages (three
+// CTAs per SM; a third stage would leave two).
 // ---------------------------------------------------------------------------
 enum SiMode : int {
   SI_T = 0,      // T = L_21 X_11                      (lower block (I, J))

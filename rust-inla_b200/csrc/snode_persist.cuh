@@ -231,7 +231,8 @@ __device__ __forceinline__ void update64w8_body(const DevSym& S, int s, int b, i
 // j0 (as tile 0 of the update would), factors the tile's pivot columns and writes the block into the
 // front and L^-1 to the inverse-block cache. Same arithmetic in the same order as the separate tasks:
 // bit-identical. 256 threads; smu: kPanelSmem bytes. What bounds it is the factorization of the 64
-// pivots (7.3 us of about 13).
+// pivots (7.5 us) and the four dependent passes around it (loads, two products, write-back); a task takes
+// 13 us alone and 17 beside the update tiles of its step.
 __device__ __forceinline__ void diag_next_body(const DevSym& S, int s, int b, int j0, double* __restrict__ F,
                                                int64_t fstride, double* __restrict__ linv, double* smu) {
   if (front_skipped(S, s, b)) return;
