@@ -4,6 +4,13 @@
 
 namespace inla {
 
+// A column of a child's update block: F offset of its first entry (the diagonal one), its rows and the
+// offset of their places in relx.
+struct alignas(16) GatherCol {
+  int64_t src;
+  int len, rel;
+};
+
 struct DevSym {
   int n = 0, ns = 0;
   const int* first = nullptr;      // ns+1
@@ -20,6 +27,10 @@ struct DevSym {
   // rss[rsp[i] .. rsp[i + 1]) of the update vectors for row i of the concatenated structures
   const int* rsp = nullptr;        // sum m + 1
   const int* rss = nullptr;        // sum r
+  // the children's columns that add into each column of the large fronts, in child order: rsp's ranges
+  // for front s, moved by gptr[s]
+  const GatherCol* gcol = nullptr;
+  const int64_t* gptr = nullptr;   // ns
   const int64_t* dpos = nullptr;   // n : front offset of D_j
   const int* perm = nullptr;       // n : perm[new] = old
   // 64 x 64 inverse-block cache of the large fronts: block (s, j0 / 64) of

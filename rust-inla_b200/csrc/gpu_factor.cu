@@ -309,34 +309,29 @@ GpuFactor::GpuFactor(const Symbolic& sym, int max_batch, cudaStream_t stream)
 
   const auto tm3 = std::chrono::steady_clock::now();
   plan_levels(M);
-  // extend-add range table: for every large front, column chunk z (of the
-  // level's gcols columns) and child, the child's source columns whose parent
-  // column lies in the chunk
+  // children's columns of the large fronts (DevSym::gcol)
   {
     std::vector<int64_t> gptr(ns, 0);
-    std::vector<int2> grng;
-    for (const LevelPlan& P : levels_) {
-      if (P.large.empty()) continue;
-      const int gcols = gather_cols(P.mmax_large);
+    std::vector<GatherCol> gcol;
+    std::vector<int> cursor;
+    for (const LevelPlan& P : levels_)
       for (int s : P.large) {
+        const int* rsp = M.rsp.data() + rowptr[s];
         const int m = rowptr[s + 1] - rowptr[s];
-        gptr[s] = (int64_t)grng.size();
-        for (int z = 0; z < cdiv(m, gcols); ++z) {
-          const int c0 = z * gcols, c1 = std::min(c0 + gcols, m);
-          for (int64_t q = S.child_ptr[s]; q < S.child_ptr[s + 1]; ++q) {
-            const int c = (int)S.child_list[q];
-            const int kc = first[c + 1] - first[c], rc = (rowptr[c + 1] - rowptr[c]) - kc;
-            const int* rel = relx.data() + rowptr[c] + kc;
-            const int lo = (int)(std::lower_bound(rel, rel + rc, c0) - rel);
-            const int hi = (int)(std::lower_bound(rel, rel + rc, c1) - rel);
-            grng.push_back(make_int2(lo, hi));
-          }
+        gptr[s] = (int64_t)gcol.size() - rsp[0];
+        gcol.resize(gcol.size() + (rsp[m] - rsp[0]));
+        cursor.assign(rsp, rsp + m);
+        for (int64_t q = S.child_ptr[s]; q < S.child_ptr[s + 1]; ++q) {
+          const int c = (int)S.child_list[q];
+          const int kc = first[c + 1] - first[c], mc = rowptr[c + 1] - rowptr[c];
+          for (int i = kc; i < mc; ++i)
+            gcol[gptr[s] + cursor[relx[rowptr[c] + i]]++] = {fptr[c] + (int64_t)i * mc + i, mc - i, rowptr[c] + i};
         }
       }
-    }
-    if (grng.empty()) grng.push_back(make_int2(0, 0));
     d_gptr_.upload(gptr, stream_);
-    d_grng_.upload(grng, stream_);
+    d_gcol_.upload(gcol, stream_);
+    ds_.gptr = d_gptr_.p;
+    ds_.gcol = d_gcol_.p;
   }
 
   INLA_CUDA(cudaStreamCreateWithFlags(&chain_stream_, cudaStreamNonBlocking));
@@ -585,7 +580,6 @@ bool make_persist_plan(const Symbolic& S, const std::vector<LevelPlan>& levels, 
   pl = PersistPlan();
   pl.gstart = {0};
   pl.total.assign(ns, 0);
-  pl.gptr.assign(ns, 0);
   auto push = [&](int type, int sn, int sub, int need, int j0, int arg) {
     pl.task.insert(pl.task.end(), {type, sn, sub, need, j0, arg});
   };
@@ -624,19 +618,6 @@ bool make_persist_plan(const Symbolic& S, const std::vector<LevelPlan>& levels, 
       smem = std::max(smem, gcols * m * 8);
       ++pl.nlarge;
       const int nz = cdiv(m, gcols);
-      pl.gptr[sn] = (int64_t)pl.grng.size();
-      for (int z = 0; z < nz; ++z) {
-        const int c0 = z * gcols, c1 = std::min(c0 + gcols, m);
-        for (int64_t q = S.child_ptr[sn]; q < S.child_ptr[sn + 1]; ++q) {
-          const int c = (int)S.child_list[q];
-          const int kc = (int)(S.sn_first[c + 1] - S.sn_first[c]);
-          const int rc = (int)(S.sn_rowptr[c + 1] - S.sn_rowptr[c]) - kc;
-          const int32_t* rel = S.rel.data() + S.rel_ptr[c];
-          const int lo = (int)(std::lower_bound(rel, rel + rc, c0) - rel);
-          const int hi = (int)(std::lower_bound(rel, rel + rc, c1) - rel);
-          pl.grng.push_back(make_int2(lo, hi));
-        }
-      }
       ph[f].push_back({PT_GATHER, nz, 0, 0, 0, gcols});
       ph[f].push_back({PT_DIAG, 1, 0, 0, nz, 0});
       int done = nz;  // extend-add, row and update tasks so far
@@ -666,7 +647,6 @@ bool make_persist_plan(const Symbolic& S, const std::vector<LevelPlan>& levels, 
   }
   pl.smem = smem;
   if (pl.tiny.empty()) pl.tiny.push_back(0);
-  if (pl.grng.empty()) pl.grng.push_back(make_int2(0, 0));
   return smem <= 227 * 1024 && pl.gstart.size() > 1;
 }
 
@@ -711,10 +691,9 @@ std::string check_persist_plan(const Symbolic& S, const PersistPlan& pl) {
       if (!children_done(sn)) return at + "small front before its children";
     } else if (type == PT_GATHER) {
       if (m <= GpuFactor::kSmallB || !children_done(sn)) return at + "extend-add before the children";
-      const int gcols = T[5], nch = (int)(S.child_ptr[sn + 1] - S.child_ptr[sn]);
+      const int gcols = T[5];
       if (gcols < 1 || (int64_t)gcols * m * 8 > pl.smem) return at + "extend-add slice exceeds shared memory";
-      if (sub >= cdiv(m, gcols) || pl.gptr[sn] + (int64_t)(sub + 1) * nch > (int64_t)pl.grng.size())
-        return at + "extend-add chunk out of range";
+      if (sub >= cdiv(m, gcols)) return at + "extend-add chunk out of range";
       if (need != 0 || prog[sn] != sub) return at + "extend-add count";
     } else if (type == PT_DIAG || type == PT_NEXT || type == PT_ROWS || type == PT_UPDATE) {
       if (m <= GpuFactor::kSmallB) return at + "step of a front that is not large";
@@ -843,8 +822,6 @@ void GpuFactor::plan_persist() {
   d_ptask_.upload(pl.task, stream_);
   d_ptiny_.upload(pl.tiny, stream_);
   d_ptotal_.upload(pl.total, stream_);
-  d_pgptr_.upload(pl.gptr, stream_);
-  d_pgrng_.upload(pl.grng, stream_);
   d_pstate_.alloc(2 + 2 * (size_t)max_batch_ * ns);
   INLA_CUDA(cudaMemsetAsync(d_pstate_.p, 0, sizeof(int) * (2 + 2 * (size_t)max_batch_ * ns), stream_));
   persist_smem_ = pl.smem;
@@ -877,8 +854,6 @@ void GpuFactor::run_factor_persist(int B, const int* total_override, long long l
   a.head = reinterpret_cast<unsigned*>(d_pstate_.p + 1);
   a.err = d_pstate_.p;
   a.linv = linv_.p;
-  a.gptr = d_pgptr_.p;
-  a.grng = d_pgrng_.p;
   a.limit_ns = limit_ns > 0 ? limit_ns : persist_limit_ns_;
   if (active) {
     a.S.active = active;
@@ -1011,7 +986,7 @@ void GpuFactor::run_factor_levels(int B, const std::vector<char>* fuse, cudaEven
       const int* lst = d_lists_.p + P.off_large;
       const int gcols = gather_cols(P.mmax_large);
       k_gather8<<<dim3(nl, B, cdiv(P.mmax_large, gcols)), 256, gcols * P.mmax_large * 8, stream_>>>(
-          ds_, lst, F_.p, fs, gcols, d_gptr_.p, d_grng_.p);
+          ds_, lst, F_.p, fs, gcols);
       ++launches_;
       const int form = fuse ? (*fuse)[li] : -1;
       for (int j0 = 0; j0 < P.kmax_large; j0 += kB64) {

@@ -87,11 +87,9 @@ struct MiniBand {
 
 // Task queue of the persistent schedule for one problem (snode_persist.cuh): 6 ints per task
 // {type, front, sub, need, j0, arg}, group starts, tiny-front list, completion counts per
-// front, extend-add chunk table, shared memory in bytes.
+// front, shared memory in bytes.
 struct PersistPlan {
   std::vector<int> gstart, task, tiny, total;
-  std::vector<int64_t> gptr;
-  std::vector<int2> grng;
   int nlarge = 0, smem = 0;
 };
 // Host tables of an analysis that an engine uploads: 32-bit copies of the supernode arrays,
@@ -230,7 +228,7 @@ class GpuFactor {
   MiniTables mini_tables(int off) const { return {d_mptr_.p + off, d_mlist_.p, d_mfront_.p, d_mchild_.p}; }
   DBuf<int> d_first_, d_rowptr_, d_rows_, d_relx_, d_child_ptr_, d_child_list_, d_parent_, d_uoff_, d_perm_, d_rsp_, d_rss_;
   DBuf<int64_t> d_fptr_, d_lptr_, d_dpos_, spos_, spos_full_, d_gptr_;
-  DBuf<int2> d_grng_;  // extend-add source-column ranges per (front, chunk, child)
+  DBuf<GatherCol> d_gcol_;
   DBuf<int> d_pmap_, d_lists_, d_csn_, d_csnm_, d_lbo_;
   DBuf<double> F_, Sg_, xp_, ub_, logdet_, dcache_, linv_, ldpart_;
   DBuf<int> status_, ldflag_;
@@ -246,8 +244,6 @@ class GpuFactor {
   int persist_smem_ = 0, persist_grid_ = 0, persist_groups_ = 0;
   long long persist_limit_ns_ = 2000000000LL;
   DBuf<int> d_pgstart_, d_ptask_, d_ptiny_, d_ptotal_, d_pstate_;  // pstate: err, head, prog[B][ns], dprog[B][ns]
-  DBuf<int64_t> d_pgptr_;
-  DBuf<int2> d_pgrng_;
   cudaStream_t chain_stream_ = nullptr;  // pivot chain of the look-ahead form, joined with stream_
   cudaEvent_t chain_ev_[2] = {nullptr, nullptr};
   int panel_form_ = -1;  // forced panel form (set_panel_form at construction), -1 autotuned

@@ -40,29 +40,20 @@ __device__ __forceinline__ const double* linv_block(const DevSym& S, const doubl
   return linv + (int64_t)b * S.lstride + ((int64_t)S.lbo[s] + blk) * (kB64 * kB64);
 }
 
-// Extend-add of the children's updates into parent columns [c0, c1) (gcols
-// columns per CTA, at most kGatherCols, fewer when the slice would not fit;
-// grng[gptr[s] + z * nchildren + q] = the child's source columns whose parent
-// column falls in chunk z, from a host table): every warp assembles columns of its own in
-// shared memory (panel columns start from the filled values, update columns from zero), adds
-// its column of every child that has it in child order (targets are distinct within one child,
-// so an entry's sum has a fixed order) and writes the column's lower part back once. No warp
-// waits for another. The children's descriptors are read 32 at a time, one per lane, so a child
-// without the column costs nothing and the dependent descriptor loads are paid once per 32
-// children: with one child after the other for the whole CTA and two barriers each, the
-// fronts of grouped models (20 to 324 iid children) spent 2 ms per factorization here.
-// What bounds it is the latency of the loads: a lane keeps eight of a long child column in
-// flight, or those of four short columns. Measured (before -> after): persistent factorization of the
-// grouped model 24x24x14 (B = 2) 2.72 -> 1.69 ms; the level launches of SPDE 200^2 at B = 10 / 15
-// 1.20 -> 1.12 / 3.40 -> 3.20 ms.
+// Extend-add of the children's updates into parent columns [c0, c1) (gcols columns per CTA, at most
+// kGatherCols, fewer when the slice would not fit): every warp assembles columns of its own in shared
+// memory (panel columns start from the filled values, update columns from zero), adds the children's
+// columns that fall on it in child order (targets are distinct within one child, so an entry's sum has a
+// fixed order) and writes the column's lower part back once. No warp waits for another. A host table
+// lists these columns (DevSym::gcol), 32 read at a time, one per lane, so a child without the column
+// costs nothing and there is one dependent load between the list and the values. What bounds it is the
+// latency of the loads: eight per lane are in flight, of one long column or of up to eight short ones.
+// Measured (one child after the other for the whole CTA, two barriers each -> a warp per column searching
+// every child's range -> lists and eight pieces): level launches of SPDE 200^2 at B = 10 1.20 -> 1.12 ->
+// 0.70 ms, at B = 30 3.40 -> 2.58 -> 2.00 ms. Fronts of the grouped model 24x24x14 have 20 to 324 iid
+// children (B = 2): persistent factorization 2.72 -> 1.69 ms before the lists.
 constexpr int kGatherCols = 8;
 
-// Descriptor of one child's column for the warp: F offset of its first entry (row jj), its row
-// count from there and the offset of its parent rows.
-struct GatherCol {
-  int64_t src;
-  int len, rel;
-};
 __device__ __forceinline__ GatherCol gather_shfl(const GatherCol& d, int lane) {
   GatherCol r;
   r.src = __shfl_sync(0xffffffffu, d.src, lane);
@@ -73,84 +64,46 @@ __device__ __forceinline__ GatherCol gather_shfl(const GatherCol& d, int lane) {
 
 // One warp: column `col` of front s (ld m) of problem b in g[0 .. m).
 __device__ __forceinline__ void gather_column(const DevSym& S, int s, double* Fb, double* Fs, int k, int m, int col,
-                                              const int2* __restrict__ rng, double* g) {
+                                              double* g) {
   const int lane = threadIdx.x & 31;
   for (int row = col + lane; row < m; row += 32) {
     if (col < k) cp_async8(&g[row], Fs + row + (int64_t)col * m);
     else g[row] = 0.0;
   }
   cp_async_commit();
-  const int q0 = S.child_ptr[s], nch = S.child_ptr[s + 1] - q0;
+  const int row0 = S.rowptr[s] + col, e0 = S.rsp[row0], n = S.rsp[row0 + 1] - e0;
+  const GatherCol* list = S.gcol + S.gptr[s] + e0;
   bool ready = false;  // the panel values have landed
   auto settle = [&] {
     if (!ready) cp_async_wait<0>();
     ready = true;
     __syncwarp();
   };
-  for (int qb = 0; qb < nch; qb += 32) {
-    GatherCol mine{0, 0, 0};
-    if (qb + lane < nch) {
-      const int2 lh = rng[qb + lane];
-      if (lh.x < lh.y) {
-        const int c = S.child_list[q0 + qb + lane];
-        const int kc = lg_k(S, c), mc = lg_m(S, c), rp = S.rowptr[c] + kc;
-        for (int jj = lh.x; jj < lh.y; ++jj)
-          if (S.relx[rp + jj] == col) {
-            mine.src = S.fptr[c] + (int64_t)(kc + jj) * mc + kc + jj;
-            mine.len = mc - kc - jj;
-            mine.rel = rp + jj;
-          }
+  for (int qb = 0; qb < n; qb += 32) {
+    const GatherCol mine = qb + lane < n ? list[qb + lane] : GatherCol{0, 0, 0};
+    const int cnt = min(32, n - qb);
+    GatherCol d = gather_shfl(mine, 0);
+    for (int at = 0, off = lane; at < cnt;) {  // 32 rows of a column at a time, eight such pieces in flight
+      double v[8];
+      int dst[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        dst[u] = -1;
+        if (at >= cnt) continue;
+        if (off < d.len) {
+          v[u] = Fb[d.src + off];
+          dst[u] = S.relx[d.rel + off];
+        }
+        off += 32;
+        if (off - lane >= d.len) {
+          off = lane;
+          if (++at < cnt) d = gather_shfl(mine, at);
+        }
       }
-    }
-    unsigned todo = __ballot_sync(0xffffffffu, mine.len > 0);
-    const unsigned shortc = __ballot_sync(0xffffffffu, mine.len > 0 && mine.len <= 64);
-    while (todo) {
-      const int first = __ffs(todo) - 1;
-      if (shortc >> first & 1u) {  // up to four short columns, loads together, added in order
-        double v[4][2];
-        int dst[4][2], n = 0;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          dst[u][0] = dst[u][1] = -1;
-          const int at = __ffs(todo) - 1;
-          if (at < 0 || !(shortc >> at & 1u) || n < u) continue;
-          todo &= todo - 1;
-          n = u + 1;
-          const GatherCol d = gather_shfl(mine, at);
-#pragma unroll
-          for (int h = 0; h < 2; ++h)
-            if (lane + 32 * h < d.len) {
-              v[u][h] = Fb[d.src + lane + 32 * h];
-              dst[u][h] = S.relx[d.rel + lane + 32 * h];
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          if (u >= n) break;
-          settle();
-#pragma unroll
-          for (int h = 0; h < 2; ++h)
-            if (dst[u][h] >= 0) g[dst[u][h]] += v[u][h];
-        }
-        continue;
-      }
-      todo &= todo - 1;
-      const GatherCol d = gather_shfl(mine, first);
-      for (int i0 = lane; i0 - lane < d.len; i0 += 256) {
-        double v[8];
-        int dst[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          dst[u] = -1;
-          if (i0 + 32 * u < d.len) {
-            v[u] = Fb[d.src + i0 + 32 * u];
-            dst[u] = S.relx[d.rel + i0 + 32 * u];
-          }
-        }
+      for (int u = 0; u < 8; ++u) {
         settle();
-#pragma unroll
-        for (int u = 0; u < 8; ++u)
-          if (dst[u] >= 0) g[dst[u]] += v[u];
+        if (dst[u] >= 0) g[dst[u]] += v[u];
       }
     }
   }
@@ -160,26 +113,23 @@ __device__ __forceinline__ void gather_column(const DevSym& S, int s, double* Fb
 
 // Chunk z of front s, problem b (any block size; gsl: [gcols][m] doubles of shared memory).
 __device__ __forceinline__ void gather8_body(const DevSym& S, int s, int b, int z, double* __restrict__ F,
-                                             int64_t fstride, int gcols, const int64_t* __restrict__ gptr,
-                                             const int2* __restrict__ grng, double* gsl) {
+                                             int64_t fstride, int gcols, double* gsl) {
   if (front_skipped(S, s, b)) return;
   const int k = lg_k(S, s), m = lg_m(S, s);
   const int c0 = z * gcols;
   if (c0 >= m) return;
   const int c1 = min(c0 + gcols, m);
   double* Fb = F + (int64_t)b * fstride;
-  const int2* rng = grng + gptr[s] + (int64_t)z * (S.child_ptr[s + 1] - S.child_ptr[s]);
   for (int cc = threadIdx.x >> 5; cc < c1 - c0; cc += blockDim.x >> 5)
-    gather_column(S, s, Fb, Fb + S.fptr[s], k, m, c0 + cc, rng, gsl + (int64_t)cc * m);
+    gather_column(S, s, Fb, Fb + S.fptr[s], k, m, c0 + cc, gsl + (int64_t)cc * m);
 }
 
-// 48 registers: five CTAs per SM even with a few spills (79 registers, three CTAs: 3.20 ms instead of
-// 2.58 in the SPDE 200^2 factorization at B = 30; 64 and four: 2.73).
+// 48 registers, five CTAs per SM (measured with the ranges searched, SPDE 200^2 at B = 30: five CTAs 2.58
+// ms, four 2.73, three 3.20).
 __global__ void __launch_bounds__(256, 5) k_gather8(DevSym S, const int* __restrict__ list, double* __restrict__ F,
-                                                 int64_t fstride, int gcols, const int64_t* __restrict__ gptr,
-                                                 const int2* __restrict__ grng) {
+                                                 int64_t fstride, int gcols) {
   extern __shared__ double gsl[];  // [gcols][m] column slice
-  gather8_body(S, list[blockIdx.x], blockIdx.y, blockIdx.z, F, fstride, gcols, gptr, grng, gsl);
+  gather8_body(S, list[blockIdx.x], blockIdx.y, blockIdx.z, F, fstride, gcols, gsl);
 }
 
 // Sigma restricted to the below-rows of s, gathered from the parent's Sigma

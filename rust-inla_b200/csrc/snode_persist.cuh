@@ -72,8 +72,6 @@ struct PersistArgs {
   unsigned* head;           // next task to claim
   int* err;                 // 0, or the reason the launch stopped early
   double* linv;
-  const int64_t* gptr;      // extend-add chunk table of this schedule
-  const int2* grng;
   long long limit_ns;       // longest wait for one dependency
 };
 
@@ -401,7 +399,7 @@ __global__ void __launch_bounds__(kPersistThreads, 2) k_factor_persist(PersistAr
         factor_small_body<kPersistThreads>(S, T.s, b, a.F, a.fstride, psm);
         break;
       case PT_GATHER:
-        gather8_body(S, T.s, b, T.sub, a.F, a.fstride, T.arg, a.gptr, a.grng, psm);
+        gather8_body(S, T.s, b, T.sub, a.F, a.fstride, T.arg, psm);
         break;
       case PT_DIAG:
         panel64_body(S, T.s, b, 0, T.j0, 0, a.F, a.fstride, nullptr, a.linv, psm);
