@@ -314,8 +314,10 @@ GpuFactor::GpuFactor(const Symbolic& sym, int max_batch, cudaStream_t stream)
     std::vector<int64_t> gptr(ns, 0);
     std::vector<GatherCol> gcol;
     std::vector<int> cursor;
+    bool large = false;
     for (const LevelPlan& P : levels_)
       for (int s : P.large) {
+        large = true;
         const int* rsp = M.rsp.data() + rowptr[s];
         const int m = rowptr[s + 1] - rowptr[s];
         gptr[s] = (int64_t)gcol.size() - rsp[0];
@@ -328,14 +330,19 @@ GpuFactor::GpuFactor(const Symbolic& sym, int max_batch, cudaStream_t stream)
             gcol[gptr[s] + cursor[relx[rowptr[c] + i]]++] = {fptr[c] + (int64_t)i * mc + i, mc - i, rowptr[c] + i};
         }
       }
-    d_gptr_.upload(gptr, stream_);
-    d_gcol_.upload(gcol, stream_);
-    ds_.gptr = d_gptr_.p;
-    ds_.gcol = d_gcol_.p;
+    if (large) {  // also where no large front has children: the kernel reads gptr
+      d_gptr_.upload(gptr, stream_);
+      d_gcol_.upload(gcol, stream_);
+      ds_.gptr = d_gptr_.p;
+      ds_.gcol = d_gcol_.p;
+    }
   }
 
-  INLA_CUDA(cudaStreamCreateWithFlags(&chain_stream_, cudaStreamNonBlocking));
-  for (auto& e : chain_ev_) INLA_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  // the look-ahead form needs its stream where a large front has more than one block of pivots
+  if (std::any_of(levels_.begin(), levels_.end(), [](const LevelPlan& P) { return P.kmax_large > kB64; })) {
+    INLA_CUDA(cudaStreamCreateWithFlags(&chain_stream_, cudaStreamNonBlocking));
+    for (auto& e : chain_ev_) INLA_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  }
   panel_form_ = g_panel_form.load();
   plan_persist();
   const auto ta = std::chrono::steady_clock::now();
