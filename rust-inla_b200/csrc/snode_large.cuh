@@ -124,8 +124,8 @@ __device__ __forceinline__ void gather8_body(const DevSym& S, int s, int b, int 
     gather_column(S, s, Fb, Fb + S.fptr[s], k, m, c0 + cc, gsl + (int64_t)cc * m);
 }
 
-// 48 registers, five CTAs per SM (measured with the ranges searched, SPDE 200^2 at B = 30: five CTAs 2.58
-// ms, four 2.73, three 3.20).
+// 48 registers, five CTAs per SM: SPDE 200^2 at B = 10 / 30 0.70 / 2.00 ms per factorization (four CTAs
+// 0.76 / 2.16, six with spills 0.79 / 2.22).
 __global__ void __launch_bounds__(256, 5) k_gather8(DevSym S, const int* __restrict__ list, double* __restrict__ F,
                                                  int64_t fstride, int gcols) {
   extern __shared__ double gsl[];  // [gcols][m] column slice
