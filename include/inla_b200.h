@@ -278,6 +278,11 @@ int inla_batch_schedule(inla_batch* h, int* persistent);
  * info3 = {tasks per problem, shared memory bytes, 1 if the schedule fits}. INLA_ERR_INTERNAL
  * with the first violation otherwise. */
 int inla_solver_check_schedule(const inla_solver* s, int64_t* info3);
+/* Host-only check of the bands of levels whose fronts all have at most eight rows (after
+ * inla_solver_analyze; no device use): every front of a band belongs to one task, with its
+ * children of the band before it. info3 = {bands, tasks, fronts of the longest task}.
+ * INLA_ERR_INTERNAL with the first violation. */
+int inla_solver_check_bands(const inla_solver* s, int64_t* info3);
 /* Process-wide choice for engines (solver, batch, Laplace, many-model handles) created after
  * the call: 0 the level launches; 1 (default) measured per batch size -- on its first
  * factorization at a batch size an engine times both schedules and keeps the faster for that

@@ -356,6 +356,26 @@ int inla_solver_check_schedule(const inla_solver* s, int64_t* info3) {
   }
 }
 
+int inla_solver_check_bands(const inla_solver* s, int64_t* info3) {
+  try {
+    if (!s || !s->sym) return fail(INLA_ERR_NOT_FACTORED, "no symbolic analysis yet");
+    std::vector<int> flat;
+    const std::vector<LevelPlan> levels = make_level_plans(*s->sym, flat);
+    MiniPlan pl;
+    make_mini_plan(*s->sym, levels, pl);
+    if (info3) {
+      info3[0] = (int64_t)pl.bands.size();
+      info3[1] = (int64_t)pl.ptr.size() - 1;
+      info3[2] = pl.longest;
+    }
+    const std::string err = check_mini_plan(*s->sym, levels, pl);
+    if (!err.empty()) return fail(INLA_ERR_INTERNAL, "bands of small fronts: " + err);
+    return INLA_OK;
+  } catch (...) {
+    return map_exception();
+  }
+}
+
 int inla_solver_colcounts(const inla_solver* s, int64_t* counts) {
   if (!s || !s->sym) return fail(INLA_ERR_NOT_FACTORED, "no symbolic analysis yet");
   std::memcpy(counts, s->sym->colcount.data(), sizeof(int64_t) * s->sym->n);

@@ -495,27 +495,40 @@ void GpuFactor::plan_levels(const HostMaps& maps) {
 
 // Bands of up to kMiniLevels consecutive levels whose fronts all have at most kMiniM rows, cut into the
 // tasks of snode_mini.cuh: the fronts of a band that are connected through parent links, children
-// first. (INLA_NO_TINY_FRONTS switches these off with the other small-front kernels.)
-void GpuFactor::plan_minis(const HostMaps& maps) {
-  const Symbolic& S = sym_;
-  const int L = (int)levels_.size();
-  band_at_.assign(L, -1);
+// first. A level joins the band below it only while no task's cost exceeds kMiniTask fronts, a child from
+// outside the band counting 1 / kMiniChildren of a front.
+// (INLA_NO_TINY_FRONTS switches these off with the other small-front kernels.)
+void make_mini_plan(const Symbolic& S, const std::vector<LevelPlan>& levels, MiniPlan& pl) {
+  const int L = (int)levels.size();
+  pl = MiniPlan();
+  pl.at.assign(L, -1);
   static const bool on = std::getenv("INLA_NO_TINY_FRONTS") == nullptr;
   if (!on) return;
-  std::vector<int> task(S.nsuper, -1);  // task of a front within the band being built
-  std::vector<int> ptr{0}, list;
+  std::vector<int64_t> cost(S.nsuper, 0);  // of the band's fronts in the subtree of a front of the band
+  std::vector<int> task(S.nsuper, -1);     // task of a front within the band being built
   for (int l = 0; l < L;) {
     int e = l;
-    while (e < L && e - l < kMiniLevels && levels_[e].mmax_all <= kMiniM) ++e;
+    for (; e < L && e - l < kMiniLevels && levels[e].mmax_all <= kMiniM; ++e) {
+      int64_t most = 0;
+      for (int s : levels[e].all) {
+        cost[s] = kMiniChildren;
+        for (int64_t q = S.child_ptr[s]; q < S.child_ptr[s + 1]; ++q)
+          cost[s] += std::max<int64_t>(cost[S.child_list[q]], 1);
+        most = std::max(most, cost[s]);
+      }
+      if (most > kMiniTask * kMiniChildren) break;
+    }
+    for (int q = l; q < std::min(L, e + 1); ++q)
+      for (int s : levels[q].all) cost[s] = 0;
     if (e - l < 2) {  // a single level gains nothing over the level kernels
       l = std::max(e, l + 1);
       continue;
     }
     // from the top level down: a front joins its parent's task if the parent lies in the band
-    const int off = (int)ptr.size() - 1;
+    const int off = (int)pl.ptr.size() - 1;
     std::vector<std::vector<int>> tasks;
     for (int q = e - 1; q >= l; --q)
-      for (int s : levels_[q].all) {
+      for (int s : levels[q].all) {
         const int64_t p = S.sn_parent[s];
         task[s] = p >= 0 && task[p] >= 0 ? task[p] : (int)tasks.size();
         if (task[s] == (int)tasks.size()) tasks.emplace_back();
@@ -524,17 +537,57 @@ void GpuFactor::plan_minis(const HostMaps& maps) {
     // similar lengths side by side: the four tasks of a warp run for the longest of them
     std::stable_sort(tasks.begin(), tasks.end(),
                      [](const std::vector<int>& a, const std::vector<int>& b) { return a.size() > b.size(); });
+    pl.longest = std::max(pl.longest, (int)tasks[0].size());
     for (const std::vector<int>& t : tasks) {
-      list.insert(list.end(), t.rbegin(), t.rend());
-      ptr.push_back((int)list.size());
+      pl.list.insert(pl.list.end(), t.rbegin(), t.rend());
+      pl.ptr.push_back((int)pl.list.size());
     }
     for (int q = l; q < e; ++q) {
-      band_at_[q] = (int)bands_.size();
-      for (int s : levels_[q].all) task[s] = -1;
+      pl.at[q] = (int)pl.bands.size();
+      for (int s : levels[q].all) task[s] = -1;
     }
-    bands_.push_back({l, e, off, (int)tasks.size()});
+    pl.bands.push_back({l, e, off, (int)tasks.size()});
     l = e;
   }
+}
+
+// Host check of the bands: every front of a band's levels in exactly one of its tasks, after its
+// children of the band, which lie in the same task; no task longer than kMiniTask. Returns an empty
+// string or the first violation.
+std::string check_mini_plan(const Symbolic& S, const std::vector<LevelPlan>& levels, const MiniPlan& pl) {
+  std::vector<int> band(S.nsuper, -1), task(S.nsuper, -1);
+  for (size_t i = 0; i < pl.bands.size(); ++i)
+    for (int q = pl.bands[i].l0; q < pl.bands[i].l1; ++q)
+      for (int s : levels[q].all) band[s] = (int)i;
+  for (size_t i = 0; i < pl.bands.size(); ++i) {
+    const MiniBand& M = pl.bands[i];
+    const std::string at = "band " + std::to_string(i) + ": ";
+    for (int t = M.off; t < M.off + M.ntask; ++t) {
+      const int len = pl.ptr[t + 1] - pl.ptr[t];
+      if (len < 1 || len > kMiniTask || len > pl.longest) return at + "task of " + std::to_string(len) + " fronts";
+      for (int f = pl.ptr[t]; f < pl.ptr[t + 1]; ++f) {
+        const int s = pl.list[f];
+        if (band[s] != (int)i || task[s] >= 0) return at + "front of another band or twice";
+        if (S.sn_rowptr[s + 1] - S.sn_rowptr[s] > kMiniM) return at + "front too large";
+        for (int64_t q = S.child_ptr[s]; q < S.child_ptr[s + 1]; ++q) {
+          const int c = (int)S.child_list[q];
+          if (band[c] == (int)i && task[c] != t) return at + "front before its children";
+        }
+        task[s] = t;
+      }
+    }
+  }
+  for (int64_t s = 0; s < S.nsuper; ++s)
+    if (band[s] >= 0 && task[s] < 0) return "front " + std::to_string(s) + " in no task";
+  return std::string();
+}
+
+void GpuFactor::plan_minis(const HostMaps& maps) {
+  MiniPlan pl;
+  make_mini_plan(sym_, levels_, pl);
+  bands_ = pl.bands;
+  band_at_ = pl.at;
+  const std::vector<int>& list = pl.list;
   if (bands_.empty()) return;
   std::vector<MiniFront> front;
   std::vector<MiniChild> child;
@@ -550,7 +603,7 @@ void GpuFactor::plan_minis(const HostMaps& maps) {
       child.push_back({maps.fptr[c] + (int64_t)kc * mc + kc, maps.rowptr[c] + kc, mc * 16 + (mc - kc)});
     }
   }
-  d_mptr_.upload(ptr, stream_);
+  d_mptr_.upload(pl.ptr, stream_);
   d_mlist_.upload(list, stream_);
   d_mfront_.upload(front, stream_);
   d_mchild_.upload(child, stream_);

@@ -84,6 +84,13 @@ struct LevelPlan {
 struct MiniBand {
   int l0, l1, off, ntask;
 };
+// Bands of an analysis: band of every level (-1 none), task ranges, fronts in task order, and the fronts
+// of the longest task.
+struct MiniPlan {
+  std::vector<MiniBand> bands;
+  std::vector<int> at, ptr{0}, list;
+  int longest = 0;
+};
 
 // Task queue of the persistent schedule for one problem (snode_persist.cuh): 6 ints per task
 // {type, front, sub, need, j0, arg}, group starts, tiny-front list, completion counts per
@@ -105,6 +112,8 @@ struct HostMaps {
 std::shared_ptr<const HostMaps> host_maps(const Symbolic& S);
 void release_host_maps();
 std::vector<LevelPlan> make_level_plans(const Symbolic& S, std::vector<int>& flat);
+void make_mini_plan(const Symbolic& S, const std::vector<LevelPlan>& levels, MiniPlan& pl);
+std::string check_mini_plan(const Symbolic& S, const std::vector<LevelPlan>& levels, const MiniPlan& pl);
 bool make_persist_plan(const Symbolic& S, const std::vector<LevelPlan>& levels, PersistPlan& out);
 std::string check_persist_plan(const Symbolic& S, const PersistPlan& pl);
 // Task queue of the persistent triangular solve (forward sweep bottom-up, then backward).
@@ -220,7 +229,7 @@ class GpuFactor {
   DevSym ds_;
   std::vector<LevelPlan> levels_;
   std::vector<MiniBand> bands_;
-  std::vector<int> band_at_;         // band of a level, -1 none
+  std::vector<int> band_at_;         // MiniPlan::at
   DBuf<int> d_mptr_, d_mlist_;       // mini tasks (MiniTables)
   DBuf<MiniFront> d_mfront_;
   DBuf<MiniChild> d_mchild_;

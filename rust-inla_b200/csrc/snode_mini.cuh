@@ -14,6 +14,15 @@
 // and child_list when the front's turn came cost 5 to 6 us per front. Bands are short because a task is as
 // long as the fronts that hang together: 4 levels give tasks of up to 9 fronts and 0.17 ms per
 // factorization of the models below, 6 levels 0.25, 8 levels 0.34.
+// Those are chains. Where fronts branch, a band stops before the level that would make a task longer than
+// kMiniTask fronts: a star or a nested grouping is one component, and without the limit one task. Star of
+// 24 000 leaves, factorization / solve / selected inverse without the limit 25.6 / 24.9 / 23.5 ms, with it
+// 12.6 / 0.98 / 0.04 ms (12.6 for 4 to 40 fronts). 1000 stars of 12 leaves, one task each: selected inverse
+// 23 us, in level launches 28; 200 of 60: 101 / 88 / 71 us as tasks, 79 / 30 / 30 in level launches; one of
+// 40: 65 / 51 / 50 and 47 / 20 / 14. Adding a child from outside the band takes a quarter of a front's time:
+// chain of 100 hubs with 400 leaves each 2.49 / 0.35 / 0.09 ms with fronts counted alone, 1.83 / 0.23 / 0.10
+// with the children counted; 2000 hubs of 10 leaves 241 / 127 / 82 and 154 / 96 / 60 us (weights 1 / 2 and
+// 1 / 8: 166 and 187 us). 96 uneven AR1 + iid models: the same within 2 % for every limit and weight.
 // Registers: a spill costs more than a resident CTA gains (factorization, 4 / 5 / 6 / 8 CTAs of 128
 // threads: 172 / 179 / 200 / 251 us); leaving the unrolled loops at the warp's largest front costs more
 // than the skipped steps (224 us).
@@ -37,6 +46,8 @@ namespace {
 constexpr int kMiniM = 8;          // rows of a front
 constexpr int kMiniLd = kMiniM + 1;
 constexpr int kMiniLevels = 4;     // levels of a band
+constexpr int kMiniTask = 16;      // fronts of a task
+constexpr int kMiniChildren = 4;   // children from outside the band that count as a front
 constexpr int kMiniGroups = 16;    // tasks per CTA (8 lanes each)
 constexpr int kMiniThreads = kMiniGroups * 8;
 
