@@ -283,6 +283,11 @@ int inla_solver_check_schedule(const inla_solver* s, int64_t* info3);
  * children of the band before it. info3 = {bands, tasks, fronts of the longest task}.
  * INLA_ERR_INTERNAL with the first violation. */
 int inla_solver_check_bands(const inla_solver* s, int64_t* info3);
+/* Host-only check of the selected inverse's launches over the large fronts at a batch size (after
+ * inla_solver_analyze; no device use): grids within the device's limits, and every tile of every
+ * product computed once. info3 = {launches, tiles of the largest grid, tiles of all grids}.
+ * INLA_ERR_INTERNAL with the first violation. */
+int inla_solver_check_selinv(const inla_solver* s, int batch, int64_t* info3);
 /* Process-wide choice for engines (solver, batch, Laplace, many-model handles) created after
  * the call: 0 the level launches; 1 (default) measured per batch size -- on its first
  * factorization at a batch size an engine times both schedules and keeps the faster for that

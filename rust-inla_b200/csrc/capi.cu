@@ -376,6 +376,20 @@ int inla_solver_check_bands(const inla_solver* s, int64_t* info3) {
   }
 }
 
+int inla_solver_check_selinv(const inla_solver* s, int batch, int64_t* info3) {
+  try {
+    if (!s || !s->sym) return fail(INLA_ERR_NOT_FACTORED, "no symbolic analysis yet");
+    if (batch < 1) return fail(INLA_ERR_INVALID, "batch must be >= 1");
+    std::vector<int> flat;
+    const std::vector<LevelPlan> levels = make_level_plans(*s->sym, flat);
+    const std::string err = check_selinv_launches(*s->sym, levels, batch, 148, info3);
+    if (!err.empty()) return fail(INLA_ERR_INTERNAL, "selected inverse: " + err);
+    return INLA_OK;
+  } catch (...) {
+    return map_exception();
+  }
+}
+
 int inla_solver_colcounts(const inla_solver* s, int64_t* counts) {
   if (!s || !s->sym) return fail(INLA_ERR_NOT_FACTORED, "no symbolic analysis yet");
   std::memcpy(counts, s->sym->colcount.data(), sizeof(int64_t) * s->sym->n);

@@ -1407,6 +1407,100 @@ void GpuFactor::solve(double* d_x, int64_t xstride, int B, int slot0) {
   });
 }
 
+// Launches of the products of a level whose large fronts have at most kmax pivots and rmax rows below them,
+// for `pairs` (front, problem) pairs. Only tiles that exist are counted: the count decides between whole
+// tiles and 32-row halves, and a launch takes at most kMaxGridZ of them.
+constexpr int kMaxGridZ = 65535;
+std::vector<SiLaunch> si_launches(int kmax, int rmax, int64_t pairs, int sms) {
+  std::vector<SiLaunch> out;
+  auto add = [&](int mode, int hb, int64_t tiles) {
+    const bool half = pairs * tiles <= sms;
+    for (int64_t z0 = 0; z0 < tiles; z0 += kMaxGridZ)
+      out.push_back({mode, hb, (int)z0, (int)std::min<int64_t>(kMaxGridZ, tiles - z0), half});
+  };
+  const int nblk = cdiv(kmax, kB64);
+  for (int hb = 1; hb < nblk; hb *= 2) {
+    add(SI_T, hb, si_join_tiles(nblk, hb));
+    add(SI_X, hb, si_join_tiles(nblk, hb));
+  }
+  const int64_t below = (int64_t)cdiv(rmax, kSiT) * nblk;
+  add(SI_W, 0, below);
+  add(SI_BK, 0, below);
+  add(SI_KK, 0, (int64_t)nblk * (nblk + 1) / 2);
+  return out;
+}
+
+// Host check of those launches for every front of an analysis at batch size B: grids within the limits, and
+// every tile of every product computed exactly once.
+std::string check_selinv_launches(const Symbolic& S, const std::vector<LevelPlan>& levels, int B, int sms,
+                                  int64_t* info3) {
+  int64_t nlaunch = 0, zmax = 0, ctas = 0;
+  for (const LevelPlan& P : levels) {
+    if (P.si_large.empty()) continue;
+    const std::vector<SiLaunch> launches =
+        si_launches(P.kmax_si_large, P.rmax_si_large, (int64_t)P.si_large.size() * B, sms);
+    for (const SiLaunch& x : launches) {
+      const int64_t z = x.half ? 2 * (int64_t)x.tiles : x.tiles;
+      if (z < 1 || z > kMaxGridZ || (x.hb > 0 && x.z0 > 0)) return "grid of " + std::to_string(z) + " tiles";
+      ++nlaunch;
+      zmax = std::max(zmax, z);
+      ctas += z;
+    }
+    for (int s : P.si_large) {
+      const int k = (int)(S.sn_first[s + 1] - S.sn_first[s]), m = (int)(S.sn_rowptr[s + 1] - S.sn_rowptr[s]);
+      const int nblk = cdiv(k, kB64), rt = cdiv(m - k, kSiT);
+      std::map<std::pair<int, int>, std::vector<int64_t>> rows;  // (mode, hb): rows done of every 64-column block
+      for (const SiLaunch& x : launches) {
+        std::vector<int64_t>& seen = rows[{x.mode, x.hb}];
+        seen.resize((size_t)nblk * (nblk + rt), 0);
+        for (int z = 0; z < (x.half ? 2 : 1) * x.tiles; ++z) {
+          auto tile = [&](auto mode) {
+            constexpr int M = decltype(mode)::value;
+            SiTile t;
+            const bool ok = x.half ? si_tile<M, 32>(x.z0 + z, x.hb, k, m, t) : si_tile<M, 64>(x.z0 + z, x.hb, k, m, t);
+            if (!ok) return true;
+            const bool below = M == SI_W || M == SI_BK;
+            if (t.i0 < 0 || t.i1 > (below ? m : k) || t.j0 < 0 || t.j0 >= k || t.t0 > t.t1 || t.t1 > m) return false;
+            const int I = below ? nblk + (t.i0 - k) / kSiT : t.i0 / kB64;
+            seen[(size_t)I * nblk + t.j0 / kB64] += t.i1 - t.i0;
+            return true;
+          };
+          bool ok = true;
+          if (x.mode == SI_T) ok = tile(std::integral_constant<int, SI_T>());
+          else if (x.mode == SI_X) ok = tile(std::integral_constant<int, SI_X>());
+          else if (x.mode == SI_W) ok = tile(std::integral_constant<int, SI_W>());
+          else if (x.mode == SI_BK) ok = tile(std::integral_constant<int, SI_BK>());
+          else ok = tile(std::integral_constant<int, SI_KK>());
+          if (!ok) return "tile out of range";
+        }
+      }
+      for (int hb = 1; hb < nblk; hb *= 2)
+        if (!rows.count({SI_T, hb}) || !rows.count({SI_X, hb})) return "a join is missing";
+      if (!rows.count({SI_KK, 0}) || (rt > 0 && (!rows.count({SI_W, 0}) || !rows.count({SI_BK, 0}))))
+        return "a product is missing";
+      for (const auto& r : rows) {
+        const int mode = r.first.first, hb = r.first.second;
+        for (int I = 0; I < nblk + rt; ++I)
+          for (int J = 0; J < nblk; ++J) {
+            bool want = I < nblk && I >= J;  // SI_KK
+            if (mode == SI_T || mode == SI_X) want = I < nblk && I / (2 * hb) == J / (2 * hb) && (I / hb) % 2 == 1 && (J / hb) % 2 == 0;
+            if (mode == SI_W || mode == SI_BK) want = I >= nblk;
+            const int len = I < nblk ? std::min(kB64, k - I * kB64) : std::min(kSiT, m - k - (I - nblk) * kSiT);
+            if (r.second[(size_t)I * nblk + J] != (want ? len : 0))
+              return "front " + std::to_string(s) + ", product " + std::to_string(mode) + ": tile (" +
+                     std::to_string(I) + ", " + std::to_string(J) + ") not computed once";
+          }
+      }
+    }
+  }
+  if (info3) {
+    info3[0] = nlaunch;
+    info3[1] = zmax;
+    info3[2] = ctas;
+  }
+  return std::string();
+}
+
 void GpuFactor::selinv(int B, int slot0) {
   if (B < 1 || slot0 < 0 || slot0 + B > max_batch_) throw std::runtime_error("batch size out of range");
   Sg_.alloc((size_t)max_batch_ * ftotal_);  // outside any capture
@@ -1448,24 +1542,18 @@ void GpuFactor::selinv_levels(int B, int slot0) {
         k_si_gather8<<<dim3(nl, B, cdiv(P.rmax_si_large, kGatherCols)), 256, 0, stream_>>>(ds_, lst, Sp, fs);
         ++launches_;
       }
-      const int nblk = cdiv(P.kmax_si_large, kB64);
-      auto go = [&](auto full, auto half, int tiles, int hb) {
-        if (tiles <= 0) return;
-        if ((int64_t)nl * B * tiles <= num_sms_)
-          half<<<dim3(nl, B, 2 * tiles), 256, kSiGemmSmem, stream_>>>(ds_, lst, hb, Fp, Sp, fs, Lp);
-        else
-          full<<<dim3(nl, B, tiles), 256, kSiGemmSmem, stream_>>>(ds_, lst, hb, Fp, Sp, fs, Lp);
-        ++launches_;
-      };
-      for (int hb = 1; hb < nblk; hb *= 2) {
-        const int tiles = cdiv(nblk, 2 * hb) * hb * hb;
-        go(k_si_gemm<SI_T, 64>, k_si_gemm<SI_T, 32>, tiles, hb);
-        go(k_si_gemm<SI_X, 64>, k_si_gemm<SI_X, 32>, tiles, hb);
+      for (const SiLaunch& x : si_launches(P.kmax_si_large, P.rmax_si_large, (int64_t)nl * B, num_sms_)) {
+        auto go = [&](auto full, auto half) {
+          (x.half ? half : full)<<<dim3(nl, B, x.half ? 2 * x.tiles : x.tiles), 256, kSiGemmSmem, stream_>>>(
+              ds_, lst, x.hb > 0 ? x.hb : x.z0, Fp, Sp, fs, Lp);
+          ++launches_;
+        };
+        if (x.mode == SI_T) go(k_si_gemm<SI_T, 64>, k_si_gemm<SI_T, 32>);
+        else if (x.mode == SI_X) go(k_si_gemm<SI_X, 64>, k_si_gemm<SI_X, 32>);
+        else if (x.mode == SI_W) go(k_si_gemm<SI_W, 64>, k_si_gemm<SI_W, 32>);
+        else if (x.mode == SI_BK) go(k_si_gemm<SI_BK, 64>, k_si_gemm<SI_BK, 32>);
+        else go(k_si_gemm<SI_KK, 64>, k_si_gemm<SI_KK, 32>);
       }
-      const int rtiles = cdiv(P.rmax_si_large, kSiT) * nblk;
-      go(k_si_gemm<SI_W, 64>, k_si_gemm<SI_W, 32>, rtiles, 0);
-      go(k_si_gemm<SI_BK, 64>, k_si_gemm<SI_BK, 32>, rtiles, 0);
-      go(k_si_gemm<SI_KK, 64>, k_si_gemm<SI_KK, 32>, nblk * (nblk + 1) / 2, 0);
     }
   }
 }

@@ -809,6 +809,70 @@ enum SiMode : int {
   SI_KK = 4,     // Sigma_KK = X^T D^-1 X - W^T Sigma_BK
 };
 
+// A launch of k_si_gemm over the large fronts of a level: tiles z0 .. z0 + tiles of every front, in 32-row
+// halves or whole (SI_T, SI_X: z0 = 0).
+struct SiLaunch {
+  int mode, hb, z0, tiles;
+  bool half;
+};
+
+// Tiles of the joins of ranges of hb blocks (SI_T, SI_X) of a front of nblk blocks: hb x hb per pair of whole
+// ranges, and the rows that exist of a last, partial pair.
+__host__ __device__ inline int si_join_tiles(int nblk, int hb) {
+  const int pairs = nblk / (2 * hb), rest = nblk - 2 * hb * pairs - hb;
+  return pairs * hb * hb + (rest > 0 ? rest * hb : 0);
+}
+
+// Rows i0 .. i1, columns from j0 and K range t0 .. t1 of tile z (all in rows of a front of k pivots and m
+// rows); TM = 32: z counts halves. False: the front has no such tile. Within a join the tiles with the longest
+// K range come first: in an order that mixes them the launch waits for SMs that got several long ones (SI_T
+// of the last join, 900 pivots at B = 7 72 -> 56 us; all joins of 6000 pivots, SI_T 2.20 -> 1.93 ms, SI_X 1.62 ->
+// 1.42 ms).
+struct SiTile {
+  int i0, i1, j0, t0, t1;
+};
+template <int MODE, int TM>
+__host__ __device__ __forceinline__ bool si_tile(int z, int hb, int k, int m, SiTile& o) {
+  const int nblk = (k + kB64 - 1) / kB64, rt = (m - k + kSiT - 1) / kSiT;
+  const int half = TM == 32 ? (z & 1) : 0;
+  if (TM == 32) z >>= 1;
+  auto lower = [](int a, int b) { return a < b ? a : b; };
+  if (MODE == SI_T || MODE == SI_X) {
+    const int pr = z / (hb * hb), q = z - pr * hb * hb, first = 2 * pr * hb;
+    const int rows = lower(hb, nblk - first - hb);
+    if (q >= rows * hb) return false;
+    const int I = first + hb + (MODE == SI_T ? q % rows : rows - 1 - q / hb);
+    const int J = first + (MODE == SI_T ? q / rows : q % hb);
+    o.i0 = I * kB64;
+    o.i1 = lower(k, o.i0 + kB64);
+    o.j0 = J * kB64;
+    o.t0 = MODE == SI_T ? o.j0 : (first + hb) * kB64;
+    o.t1 = MODE == SI_T ? (first + hb) * kB64 : o.i1;
+  } else if (MODE == SI_W || MODE == SI_BK) {
+    const int I = z / nblk, J = z - I * nblk;
+    if (I >= rt) return false;
+    o.i0 = k + I * kSiT;
+    o.i1 = lower(m, o.i0 + kSiT);
+    o.j0 = J * kB64;
+    o.t0 = MODE == SI_W ? o.j0 : k;
+    o.t1 = MODE == SI_W ? k : m;
+  } else {
+    if (z >= nblk * (nblk + 1) / 2) return false;
+    int I = 0, rem = z;
+    while (rem > I) rem -= ++I;
+    o.i0 = I * kB64;
+    o.i1 = lower(k, o.i0 + kB64);
+    o.j0 = rem * kB64;
+    o.t0 = o.i0 + 32 * half;  // X is lower triangular
+    o.t1 = m;
+  }
+  if (TM == 32) {
+    o.i0 += 32 * half;
+    o.i1 = lower(o.i1, o.i0 + 32);
+  }
+  return o.i0 < o.i1;
+}
+
 // Tile z of front s, problem b. hb: block count of the ranges joined (SI_T, SI_X). TM = 32 cuts every
 // tile into two CTAs of 32 rows, for launches whose 64-row tiles would leave SMs idle (the K loop of
 // one 64 x 64 tile is 1.1 us per chunk at the tensor-core rate of one SM); an entry's sum is the same.
@@ -819,43 +883,9 @@ __device__ __forceinline__ void si_gemm_body(const DevSym& S, int s, int b, int 
   constexpr int ld = kLd64, kBuf = 64 * kLd64;  // one stage: As[32][ld], Bs[32][ld]
   __shared__ double scale[kSiStages][32];
   const int k = lg_k(S, s), m = lg_m(S, s);
-  const int nblk = (k + kB64 - 1) / kB64, rt = (m - k + kSiT - 1) / kSiT;
-  const int half = TM == 32 ? (z & 1) : 0;
-  if (TM == 32) z >>= 1;
-  // tile (rows i0 .. i1, columns j0 .. j1) and the K range t0 .. t1, all in rows of the front
-  int i0, i1, j0, t0, t1;
-  if (MODE == SI_T || MODE == SI_X) {
-    const int pr = z / (hb * hb), q = z - pr * hb * hb, first = 2 * pr * hb;
-    const int I = first + hb + q / hb, J = first + q % hb;
-    if (I >= nblk) return;
-    i0 = I * kB64;
-    i1 = min(k, i0 + kB64);
-    j0 = J * kB64;
-    t0 = MODE == SI_T ? j0 : (first + hb) * kB64;
-    t1 = MODE == SI_T ? (first + hb) * kB64 : i1;
-  } else if (MODE == SI_W || MODE == SI_BK) {
-    const int I = z / nblk, J = z - I * nblk;
-    if (I >= rt) return;
-    i0 = k + I * kSiT;
-    i1 = min(m, i0 + kSiT);
-    j0 = J * kB64;
-    t0 = MODE == SI_W ? j0 : k;
-    t1 = MODE == SI_W ? k : m;
-  } else {
-    if (z >= nblk * (nblk + 1) / 2) return;
-    int I = 0, rem = z;
-    while (rem > I) rem -= ++I;
-    i0 = I * kB64;
-    i1 = min(k, i0 + kB64);
-    j0 = rem * kB64;
-    t0 = i0 + 32 * half;  // X is lower triangular
-    t1 = m;
-  }
-  if (TM == 32) {
-    i0 += 32 * half;
-    i1 = min(i1, i0 + 32);
-    if (i0 >= i1) return;
-  }
+  SiTile tile;
+  if (!si_tile<MODE, TM>(z, hb, k, m, tile)) return;
+  const int i0 = tile.i0, i1 = tile.i1, j0 = tile.j0, t0 = tile.t0, t1 = tile.t1;
   const int j1 = min(k, j0 + kB64);
   const double* Fs = F + (int64_t)b * fstride + S.fptr[s];
   double* Ss = Sg + (int64_t)b * fstride + S.fptr[s];
@@ -982,12 +1012,18 @@ __device__ __forceinline__ void si_gemm_body(const DevSym& S, int s, int b, int 
       }
 }
 
+// arg: hb (SI_T, SI_X: always one launch), else the launch's first tile (a parameter of its own for all modes
+// spills in SI_T and SI_X; without the assumption SI_KK is 3 % slower).
 template <int MODE, int TM>
-__global__ void __launch_bounds__(256, kSiCtas) k_si_gemm(DevSym S, const int* __restrict__ list, int hb,
+__global__ void __launch_bounds__(256, kSiCtas) k_si_gemm(DevSym S, const int* __restrict__ list, int arg,
                                                     const double* __restrict__ F, double* __restrict__ Sg,
                                                     int64_t fstride, const double* __restrict__ linv) {
   extern __shared__ double smem64[];
-  si_gemm_body<MODE, TM>(S, list[blockIdx.x], blockIdx.y, blockIdx.z, hb, F, Sg, fstride, linv, smem64);
+  constexpr bool join = MODE == SI_T || MODE == SI_X;
+  const int z = join ? blockIdx.z : arg + blockIdx.z;
+  __builtin_assume(z >= 0);
+  si_gemm_body<MODE, TM>(S, list[blockIdx.x], blockIdx.y, z, join ? arg : 0, F, Sg,
+                         fstride, linv, smem64);
 }
 
 }  // namespace
