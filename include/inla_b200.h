@@ -278,6 +278,10 @@ int inla_batch_schedule(inla_batch* h, int* persistent);
  * info3 = {tasks per problem, shared memory bytes, 1 if the schedule fits}. INLA_ERR_INTERNAL
  * with the first violation otherwise. */
 int inla_solver_check_schedule(const inla_solver* s, int64_t* info3);
+/* The factorization part of that check on the queue with `delta` added to one field of one task (0 type,
+ * 1 front, 2 part, 3 extend-add, row and update tasks to wait for, 4 first column, 5 diagonal blocks to
+ * wait for), to show that the check sees it; entry6 (may be NULL) = the task as built. */
+int inla_solver_check_schedule_edit(const inla_solver* s, int64_t task, int field, int delta, int32_t* entry6);
 /* Host-only check of the bands of levels whose fronts all have at most eight rows (after
  * inla_solver_analyze; no device use): every front of a band belongs to one task, with its
  * children of the band before it. info3 = {bands, tasks, fronts of the longest task}.

@@ -356,6 +356,25 @@ int inla_solver_check_schedule(const inla_solver* s, int64_t* info3) {
   }
 }
 
+int inla_solver_check_schedule_edit(const inla_solver* s, int64_t task, int field, int delta, int32_t* entry6) {
+  try {
+    if (!s || !s->sym) return fail(INLA_ERR_NOT_FACTORED, "no symbolic analysis yet");
+    std::vector<int> flat;
+    const std::vector<LevelPlan> levels = make_level_plans(*s->sym, flat);
+    PersistPlan pl;
+    make_persist_plan(*s->sym, levels, pl);
+    if (task < 0 || task >= (int64_t)(pl.task.size() / 6) || field < 0 || field > 5)
+      return fail(INLA_ERR_INVALID, "no such task or field");
+    if (entry6) std::copy_n(pl.task.data() + 6 * task, 6, entry6);
+    pl.task[6 * task + field] += delta;
+    const std::string err = check_persist_plan(*s->sym, pl);
+    if (!err.empty()) return fail(INLA_ERR_INTERNAL, "persistent schedule: " + err);
+    return INLA_OK;
+  } catch (...) {
+    return map_exception();
+  }
+}
+
 int inla_solver_check_bands(const inla_solver* s, int64_t* info3) {
   try {
     if (!s || !s->sym) return fail(INLA_ERR_NOT_FACTORED, "no symbolic analysis yet");

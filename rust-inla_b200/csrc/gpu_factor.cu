@@ -712,15 +712,17 @@ bool make_persist_plan(const Symbolic& S, const std::vector<LevelPlan>& levels, 
 
 // Host check of the schedule's invariants: processed one task at a time in queue order (one
 // problem), every task's dependencies are complete when it is reached (so the smallest
-// unfinished task of the GPU queue can always run), every front ends with its completion count,
-// and every table index is in range. Returns an empty string or the first violation.
+// unfinished task of the GPU queue can always run), the counts that a task of a large front waits for
+// cover everything it reads (derived here from the front's shape, not from the queue), every part of a
+// step is there once, every front ends with its completion count, and every table index is in range.
+// Returns an empty string or the first violation.
 std::string check_persist_plan(const Symbolic& S, const PersistPlan& pl) {
   const int ns = (int)S.nsuper;
   const int ntask = (int)(pl.task.size() / 6);
   if (pl.gstart.back() != ntask) return "group table does not cover the tasks";
   for (size_t g = 0; g + 1 < pl.gstart.size(); ++g)
     if (pl.gstart[g + 1] <= pl.gstart[g]) return "empty or decreasing group " + std::to_string(g);
-  std::vector<int> prog(ns, 0), diag(ns, 0), step(ns, -1);
+  std::vector<int> prog(ns, 0), diag(ns, 0);
   auto children_done = [&](int sn) {
     for (int64_t q = S.child_ptr[sn]; q < S.child_ptr[sn + 1]; ++q) {
       const int c = (int)S.child_list[q];
@@ -728,7 +730,22 @@ std::string check_persist_plan(const Symbolic& S, const PersistPlan& pl) {
     }
     return true;
   };
-  auto blocks = [&](int sn) { return cdiv(S.sn_first[sn + 1] - S.sn_first[sn], kB64); };
+  auto pivots = [&](int sn) { return (int)(S.sn_first[sn + 1] - S.sn_first[sn]); };
+  auto height = [&](int sn) { return (int)(S.sn_rowptr[sn + 1] - S.sn_rowptr[sn]); };
+  auto blocks = [&](int sn) { return cdiv(pivots(sn), kB64); };
+  // large fronts: columns per extend-add task, and tasks of every (step, type) reached so far
+  std::vector<int> gcols_of(ns, 0);
+  std::map<std::pair<int, int>, std::pair<int, int>> parts;  // (front, step) -> rows, tiles
+  auto below = [&](int sn, int J) { return std::max(height(sn) - std::min((J + 1) * kB64, pivots(sn)), 0); };
+  auto row_tasks = [&](int sn, int J) { return cdiv(below(sn, J), kPanelRows); };
+  // the first 64 x 64 tile below step J is the next diagonal block's while there is one
+  auto first_tile = [&](int sn, int J) { return J + 1 < blocks(sn) ? 1 : 0; };
+  auto end_tile = [&](int sn, int J) { return cdiv(below(sn, J), kUT64) * (cdiv(below(sn, J), kUT64) + 1) / 2; };
+  auto before = [&](int sn, int J) {  // extend-add tasks, and rows and tiles of the steps before J
+    int c = cdiv(height(sn), std::max(gcols_of[sn], 1));
+    for (int q = 0; q < J; ++q) c += row_tasks(sn, q) + end_tile(sn, q) - first_tile(sn, q);
+    return c;
+  };
   for (int t = 0; t < ntask; ++t) {
     const int* T = pl.task.data() + 6 * t;
     const int type = T[0], sn = T[1], sub = T[2], need = T[3];
@@ -738,14 +755,13 @@ std::string check_persist_plan(const Symbolic& S, const PersistPlan& pl) {
       for (int u = 0; u < sub; ++u) {
         const int f = pl.tiny[sn + u];
         if (f < 0 || f >= ns || !children_done(f)) return at + "tiny front before its children";
-        const int m = (int)(S.sn_rowptr[f + 1] - S.sn_rowptr[f]);
-        if (m > kTinyM) return at + "front too large for a warp";
+        if (height(f) > kTinyM) return at + "front too large for a warp";
       }
       for (int u = 0; u < sub; ++u) ++prog[pl.tiny[sn + u]];
       continue;
     }
     if (sn < 0 || sn >= ns) return at + "front out of range";
-    const int k = (int)(S.sn_first[sn + 1] - S.sn_first[sn]), m = (int)(S.sn_rowptr[sn + 1] - S.sn_rowptr[sn]);
+    const int k = pivots(sn), m = height(sn);
     if (type == PT_SMALL) {
       if (m > GpuFactor::kSmallB) return at + "front too large for the small body";
       if (!children_done(sn)) return at + "small front before its children";
@@ -753,6 +769,8 @@ std::string check_persist_plan(const Symbolic& S, const PersistPlan& pl) {
       if (m <= GpuFactor::kSmallB || !children_done(sn)) return at + "extend-add before the children";
       const int gcols = T[5];
       if (gcols < 1 || (int64_t)gcols * m * 8 > pl.smem) return at + "extend-add slice exceeds shared memory";
+      if (gcols_of[sn] == 0) gcols_of[sn] = gcols;
+      if (gcols != gcols_of[sn]) return at + "extend-add slices of different widths";
       if (sub >= cdiv(m, gcols)) return at + "extend-add chunk out of range";
       if (need != 0 || prog[sn] != sub) return at + "extend-add count";
     } else if (type == PT_DIAG || type == PT_NEXT || type == PT_ROWS || type == PT_UPDATE) {
@@ -761,14 +779,21 @@ std::string check_persist_plan(const Symbolic& S, const PersistPlan& pl) {
       if (prog[sn] < need || diag[sn] < T[5]) return at + "phase before its predecessors";
       const int J = T[4] / kB64;
       if (type == PT_DIAG || type == PT_NEXT) {
-        // block J after block J - 1; its mirror rows and its tile after the updates of step J - 2
-        if (J != diag[sn] || (type == PT_DIAG) != (J == 0) || (J > 0 && T[5] < J)) return at + "diagonal block order";
-        if (J >= 2 && step[sn] < J - 2) return at + "diagonal block before its updates";
+        // the first block after the extend-add; block J after block J - 1 and, for its tile and its mirror
+        // rows, after the updates of step J - 2
+        if (J != diag[sn] || (type == PT_DIAG) != (J == 0) || T[5] < J) return at + "diagonal block order";
+        if (need < before(sn, std::max(J - 1, 0))) return at + "diagonal block does not wait for its updates";
         ++diag[sn];
         continue;
       }
-      if (type == PT_ROWS && T[5] < J + 1) return at + "rows before their diagonal block";
-      if (type == PT_UPDATE) step[sn] = J;
+      std::pair<int, int>& part = parts[{sn, J}];
+      if (type == PT_ROWS) {
+        if (T[5] < J + 1 || need < before(sn, J)) return at + "rows do not wait for their diagonal block or updates";
+        if (sub != part.first++ || sub >= row_tasks(sn, J)) return at + "row block out of order or range";
+      } else {
+        if (need < before(sn, J) + row_tasks(sn, J)) return at + "update does not wait for its rows";
+        if (sub != first_tile(sn, J) + part.second++ || sub >= end_tile(sn, J)) return at + "tile out of order or range";
+      }
     } else {
       return at + "unknown task type";
     }
@@ -776,7 +801,7 @@ std::string check_persist_plan(const Symbolic& S, const PersistPlan& pl) {
   }
   for (int sn = 0; sn < ns; ++sn)
     if (pl.total[sn] < 1 || prog[sn] != pl.total[sn] ||
-        (S.sn_rowptr[sn + 1] - S.sn_rowptr[sn] > GpuFactor::kSmallB && diag[sn] != blocks(sn)))
+        (height(sn) > GpuFactor::kSmallB && (diag[sn] != blocks(sn) || prog[sn] != before(sn, blocks(sn)))))
       return "front " + std::to_string(sn) + " incomplete";
   return std::string();
 }

@@ -92,6 +92,7 @@ SIGNATURES = [
     ("inla_batch_factorize_dev", C.c_int, [P, C.c_int, P, P, P, P]),
     ("inla_batch_schedule", C.c_int, [P, IP]),
     ("inla_solver_check_schedule", C.c_int, [P, LP]),
+    ("inla_solver_check_schedule_edit", C.c_int, [P, C.c_int64, C.c_int, C.c_int, IP]),
     ("inla_solver_check_bands", C.c_int, [P, LP]),
     ("inla_solver_check_selinv", C.c_int, [P, C.c_int, LP]),
     ("inla_set_persistent_schedule", C.c_int, [C.c_int]),
