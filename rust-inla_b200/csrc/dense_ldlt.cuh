@@ -98,6 +98,7 @@ __device__ __forceinline__ void warp_ldlt8(double* A, int lda, int w, double* La
       for (int i = j; i < 8; ++i)
         if (i >= w) a[i][j] = (i == j) ? 1.0 : 0.0;
   }
+  __syncwarp();  // every lane has read the block that lane 0 overwrites
   // Right-looking elimination of the block and of the columns tg and tg + 4 of L^-1 (x0, x1: rows 4 to 7
   // of the latter). A finished column leaves for shared memory at once (lane 0), which frees its registers.
   double x0[8], x1[4];
