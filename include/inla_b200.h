@@ -310,6 +310,9 @@ int inla_set_panel_form(int form);
  * the launch recorded (1: a wait ran out and the launch ended). The handle stays usable;
  * factorize again before solving. */
 int inla_batch_wait_limit_selftest(inla_batch* h, double limit_ms, int* code);
+/* Diagnostic of the reciprocal of the pivots: y[i] = 1 / x[i] (host arrays) as the dense factorization
+ * forms it on the device. */
+int inla_reciprocal_selftest(int64_t n, const double* x, double* y);
 int inla_batch_solve_dev(inla_batch* h, int B, double* d_x, void* stream);
 int inla_batch_diag_inv_dev(inla_batch* h, int B, double* d_diag, void* stream);
 int inla_batch_selinv_pattern_dev(inla_batch* h, int B, double* d_sigma, void* stream);

@@ -467,6 +467,16 @@ int inla_batch_schedule(inla_batch* h, int* persistent) {
   return INLA_OK;
 }
 
+int inla_reciprocal_selftest(int64_t n, const double* x, double* y) {
+  try {
+    if (n < 0 || (n > 0 && (!x || !y))) return fail(INLA_ERR_INVALID, "invalid argument");
+    reciprocal_selftest(n, x, y);
+    return INLA_OK;
+  } catch (...) {
+    return map_exception();
+  }
+}
+
 int inla_batch_wait_limit_selftest(inla_batch* h, double limit_ms, int* code) {
   try {
     if (!h || !h->eng || !code || !(limit_ms > 0.0)) return fail(INLA_ERR_INVALID, "invalid argument");

@@ -58,11 +58,13 @@ __device__ __forceinline__ void bar_arrive_id(int id, int threads) {
   asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
-// 1 / d for 1e-300 <= |d| < 1e300 without a branch: the hardware approximation y (relative error e <
-// 2^-20) and one step of the third-order Householder iteration y (1 + e + e^2), whose error e^3 is below
-// the rounding of the last product. d = 0 gives NaN. The operator's slow path for special operands is a
-// branch that keeps the compiler from moving anything across it (90 cycles per division and the block's
-// products in between exposed); this is 65 cycles and leaves one straight line.
+// 1 / d for 2^-1000 <= |d| < 2^1000 (rcp_in_range) without a branch: the hardware approximation y and one step
+// of the third-order Householder iteration y (1 + e + e^2). PTX has y look at the 20 leading mantissa bits of d
+// and set as many, so |e| < 2^-18, and the neglected e^3 y is below half a unit in the last place: the result
+// lies within one unit of the correctly rounded 1 / d (measured over two million mantissas: 0.03 % differ, the
+// worst is 0.506 units off). Outside the range y may be flushed; warp_ldlt8 then
+// repeats the block with 1.0 / d. With 1.0 / d throughout the 64 x 64 block of cta_ldlt takes 14.9 k cycles with
+// the inverse and 13.3 k without, with this 13.3 k and 11.9 k.
 __device__ __forceinline__ double rcp_straight(double d) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
@@ -70,12 +72,16 @@ __device__ __forceinline__ double rcp_straight(double d) {
   return fma(y, fma(e, e, e), y);
 }
 
+__device__ __forceinline__ bool rcp_in_range(double d) {  // by the high word of |d|
+  return (unsigned)(__double2hiint(d) & 0x7fffffff) - 0x01700000u < 0x7d000000u;
+}
+
 // One warp: LDL^T and inverse of the w x w (w <= 8) leading block of A (shared memory, column-major,
 // even leading dimension lda, 16-byte aligned; lower triangle read). On exit A holds L strictly below
 // the diagonal and D on it (inside w x w only); Lam (ld kLam8Ld) holds L^-1 as an 8 x 8 unit lower
 // triangle (identity beyond w), di[t] = 1 / d_t (1 beyond w), and lam0 / lam1 the lane's entries
 // (g, tg) and (g, tg + 4) of Lam (g = lane / 4, tg = lane % 4: its tensor-core fragments).
-// The chain per pivot is a reciprocal (65 cycles) and two dependent FMAs (12 each). Exchanging the
+// The chain per pivot is a reciprocal and two dependent FMAs. Exchanging the
 // pivot column between lanes put a store -> __syncwarp -> load (40 cycles) and the issue of the
 // exchanged row's loads on it as well: 360 cycles per pivot for 16 x 16 blocks. So every lane repeats
 // the block's 112 products instead, which fit in the shadow of the reciprocals.
@@ -91,18 +97,25 @@ __device__ __forceinline__ void warp_ldlt8(double* A, int lda, int w, double* La
       if (i >= j) a[i][j] = v.x;
       a[i + 1][j] = v.y;
     }
-  if (w < 8) {
+  auto pad = [&] {
+    if (w < 8) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
+      for (int j = 0; j < 8; ++j)
 #pragma unroll
-      for (int i = j; i < 8; ++i)
-        if (i >= w) a[i][j] = (i == j) ? 1.0 : 0.0;
-  }
+        for (int i = j; i < 8; ++i)
+          if (i >= w) a[i][j] = (i == j) ? 1.0 : 0.0;
+    }
+  };
+  pad();
+  // the block as it came, for a second pass (A is overwritten as the columns are finished)
+  Lam[g + tg * kLam8Ld] = A[g + tg * lda];
+  Lam[g + (tg + 4) * kLam8Ld] = A[g + (tg + 4) * lda];
   __syncwarp();  // every lane has read the block that lane 0 overwrites
   // Right-looking elimination of the block and of the columns tg and tg + 4 of L^-1 (x0, x1: rows 4 to 7
   // of the latter). A finished column leaves for shared memory at once (lane 0), which frees its registers.
   double x0[8], x1[4];
   const int lim = lane == 0 ? w : 0;
+  bool in_range = true;
   auto eliminate = [&](auto rcp) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) x0[i] = (i == tg) ? 1.0 : 0.0;
@@ -110,6 +123,7 @@ __device__ __forceinline__ void warp_ldlt8(double* A, int lda, int w, double* La
     for (int i = 0; i < 4; ++i) x1[i] = (i == tg) ? 1.0 : 0.0;
 #pragma unroll
     for (int p = 0; p < 8; ++p) {
+      in_range = in_range && rcp_in_range(a[p][p]);
       const double r = rcp(a[p][p]);
       if (lane == 0) di[p] = r;
       if (p < lim) A[p + p * lda] = a[p][p];
@@ -128,12 +142,17 @@ __device__ __forceinline__ void warp_ldlt8(double* A, int lda, int w, double* La
       }
     }
   };
-  // largest diagonal entry by its high word (sign off; NaN and infinity compare as large)
-  int big = 0;
+  eliminate([](double d) { return rcp_straight(d); });
+  if (!in_range) {  // every lane alike
+    __syncwarp();
 #pragma unroll
-  for (int i = 0; i < 8; ++i) big = max(big, __double2hiint(a[i][i]) & 0x7fffffff);
-  if (big < 0x7c300000) eliminate([](double d) { return rcp_straight(d); });  // |a_ii| < 2^964
-  else eliminate([](double d) { return 1.0 / d; });  // outside the range of rcp_straight
+    for (int j = 0; j < 8; ++j)
+#pragma unroll
+      for (int i = j; i < 8; ++i) a[i][j] = Lam[i + j * kLam8Ld];
+    pad();
+    eliminate([](double d) { return 1.0 / d; });
+    __syncwarp();  // the block in Lam has been read
+  }
   lam0 = x0[0];
   lam1 = 0.0;
 #pragma unroll
@@ -186,8 +205,9 @@ __device__ __forceinline__ void warp_trinv16(const double* L, int ldl, int w, do
 // trailing tiles while the pivot warp is already in the next block. What bounds it is the pivot
 // warp's chain. Lam and 1 / d are double-buffered: they are overwritten two blocks later, after a
 // barrier that every reader has passed.
-// Measured for a 64 x 64 block with its inverse, one CTA of 256 threads: 14.3 k cycles (11.6 k without the inverse); the 16-wide form it
-// replaces (one warp factoring 16 x 16 with the others waiting, three barriers per block): 32.7 k (25.5 k).
+// Measured for a 64 x 64 block with its inverse, one CTA of 256 threads: 13.3 k cycles (11.9 k without the
+// inverse); the 16-wide form it replaces (one warp factoring 16 x 16 with the others waiting, three barriers
+// per block): 32.7 k (25.5 k).
 template <bool kInv>
 __device__ __forceinline__ void cta_ldlt(double* A, int lda, int m, int kp, double* Li, int ldi, double* U, int ldu, double* ws) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;

@@ -1012,6 +1012,24 @@ void GpuFactor::check_schedule() {
                   (int)cudaErrorLaunchTimeout);
 }
 
+namespace {
+__global__ void k_reciprocal(int64_t n, const double* __restrict__ x, double* __restrict__ y) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i < n) y[i] = rcp_in_range(x[i]) ? rcp_straight(x[i]) : 1.0 / x[i];
+}
+}  // namespace
+
+void reciprocal_selftest(int64_t n, const double* x, double* y) {
+  if (n == 0) return;
+  DBuf<double> dx, dy;
+  dx.alloc(n);
+  dy.alloc(n);
+  INLA_CUDA(cudaMemcpy(dx.p, x, sizeof(double) * n, cudaMemcpyHostToDevice));
+  k_reciprocal<<<(unsigned)cdiv(n, 256), 256>>>(n, dx.p, dy.p);
+  INLA_CUDA(cudaGetLastError());
+  INLA_CUDA(cudaMemcpy(y, dy.p, sizeof(double) * n, cudaMemcpyDeviceToHost));
+}
+
 int GpuFactor::persist_wait_limit_selftest(double limit_ms) {
   if (!persist_) return -1;
   const int ns = (int)sym_.nsuper;

@@ -114,6 +114,7 @@ void release_host_maps();
 std::vector<LevelPlan> make_level_plans(const Symbolic& S, std::vector<int>& flat);
 void make_mini_plan(const Symbolic& S, const std::vector<LevelPlan>& levels, MiniPlan& pl);
 std::string check_mini_plan(const Symbolic& S, const std::vector<LevelPlan>& levels, const MiniPlan& pl);
+void reciprocal_selftest(int64_t n, const double* x, double* y);
 std::string check_selinv_launches(const Symbolic& S, const std::vector<LevelPlan>& levels, int B, int sms,
                                   int64_t* info3);
 bool make_persist_plan(const Symbolic& S, const std::vector<LevelPlan>& levels, PersistPlan& out);
