@@ -20,8 +20,6 @@ namespace inla {
 namespace {
 inline int cdiv(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }
 
-constexpr size_t kSolvePersistLevels = 8;  // see GpuFactor::solve
-
 // Panel forms of a level's large fronts (entries of the per-level schedule).
 constexpr char kFormSplit = 0, kFormFused = 1, kFormLookahead = 2, kNumForms = 3;
 // Process-wide panel form for engines built from now on: -1 the autotuner's choice per level
@@ -621,9 +619,12 @@ namespace {
 // per batch size (default), 2 persistent wherever it fits. INLA_NO_PERSIST in the environment
 // starts it at 0; inla_set_persistent_schedule changes it.
 std::atomic<int> g_persist_default{-1};
-// measured choice per (supernodal structure, batch size): true = persistent
+// measured choices per (supernodal structure, batch size): true = persistent
+struct SchedChoice {
+  bool factor, solve;
+};
 std::mutex g_sched_mu;
-std::map<std::pair<uint64_t, int>, bool> g_sched;
+std::map<std::pair<uint64_t, int>, SchedChoice> g_sched;
 }  // namespace
 
 void set_persistent_default(int mode) { g_persist_default.store(mode < 0 ? 0 : (mode > 2 ? 2 : mode)); }
@@ -954,7 +955,11 @@ void GpuFactor::run_factor_persist(int B, const int* total_override, long long l
 // Persistent or level launches for batch size B: fixed by the mode, or measured on the
 // first factorization at B (the level sequence in its tuned form and the persistent launch,
 // each after a warm-up, with CUDA events on the engine's stream) and kept for the structure
-// and B. The triangular solve follows the same choice.
+// and B. Where the factorization is persistent, the triangular solve's two schedules are timed in
+// the same way, each as the graph it runs as: which is faster depends on the tree, not on its depth alone.
+// Level launches / persistent: 13 levels (n = 900, AMD) 187 / 169 us, 28 levels (n = 10 000, AMD) 519 / 450, 3-D
+// grid of 22^3 350 / 336, but 2-D grids of 60^2 and 300^2 under nested dissection 193 / 224 and 488 / 607, binary
+// trees of dense 60-column blocks, 3 / 5 / 7 / 8 levels, 41 / 52, 69 / 83, 223 / 302, 513 / 776.
 bool GpuFactor::use_persist(int B, const std::function<void()>& fill) {
   if (!persist_) return false;
   if (persist_mode_ == 2) return true;
@@ -963,7 +968,10 @@ bool GpuFactor::use_persist(int B, const std::function<void()>& fill) {
   {
     std::lock_guard<std::mutex> lk(g_sched_mu);
     auto g = g_sched.find({struct_hash_, B});
-    if (g != g_sched.end()) return persist_at_[B] = g->second;
+    if (g != g_sched.end()) {
+      solve_persist_at_[B] = g->second.solve;
+      return persist_at_[B] = g->second.factor;
+    }
   }
   const std::vector<char>* pol = schedule(B, fill);
   cudaEvent_t e[4];
@@ -985,16 +993,67 @@ bool GpuFactor::use_persist(int B, const std::function<void()>& fill) {
   INLA_CUDA(cudaEventElapsedTime(&tl, e[0], e[1]));
   INLA_CUDA(cudaEventElapsedTime(&tp, e[2], e[3]));
   for (auto& x : e) cudaEventDestroy(x);
-  check_schedule();
   const bool pick = tp < tl;
+  bool pick_solve = false;
+  if (pick && solve_persist_) {
+    INLA_CUDA(cudaMemsetAsync(xp_.p, 0, sizeof(double) * B * sym_.n, stream_));
+    const float sl = time_graph([&] { solve_levels(B, 0); });
+    const float sp = time_graph([&] { solve_queue(B, 0); });
+    pick_solve = sp < sl;
+    if (std::getenv("INLA_DEBUG"))
+      std::fprintf(stderr, "solve B=%d: level launches %.3f ms, persistent %.3f ms -> %s\n", B, sl, sp,
+                   pick_solve ? "persistent" : "levels");
+  }
+  check_schedule();
   if (std::getenv("INLA_DEBUG"))
     std::fprintf(stderr, "schedule B=%d: level launches %.3f ms, persistent %.3f ms -> %s\n", B, tl, tp,
                  pick ? "persistent" : "levels");
   {
     std::lock_guard<std::mutex> lk(g_sched_mu);
-    g_sched[{struct_hash_, B}] = pick;
+    g_sched[{struct_hash_, B}] = {pick, pick_solve};
   }
+  solve_persist_at_[B] = pick_solve;
   return persist_at_[B] = pick;
+}
+
+// Milliseconds of a launch sequence run as a graph (after a warm-up), or launched directly where it cannot be
+// captured.
+float GpuFactor::time_graph(const std::function<void()>& body) {
+  const int64_t before = launches_;
+  cudaGraph_t g = nullptr;
+  cudaGraphExec_t ex = nullptr;
+  if (use_graphs_) {
+    INLA_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
+    bool ok = true;
+    try {
+      body();
+    } catch (...) {
+      ok = false;  // the direct run below throws it again
+    }
+    ok = cudaGetLastError() == cudaSuccess && ok;
+    if (cudaStreamEndCapture(stream_, &g) != cudaSuccess || !ok || cudaGraphInstantiate(&ex, g, 0) != cudaSuccess) {
+      ex = nullptr;
+      cudaGetLastError();  // the capture's errors are not sticky
+    }
+    if (g) cudaGraphDestroy(g);
+  }
+  auto run = [&] {
+    if (ex) INLA_CUDA(cudaGraphLaunch(ex, stream_));
+    else body();
+  };
+  cudaEvent_t e[2];
+  for (auto& x : e) INLA_CUDA(cudaEventCreate(&x));
+  run();
+  INLA_CUDA(cudaEventRecord(e[0], stream_));
+  run();
+  INLA_CUDA(cudaEventRecord(e[1], stream_));
+  INLA_CUDA(cudaStreamSynchronize(stream_));
+  float ms = 0.f;
+  INLA_CUDA(cudaEventElapsedTime(&ms, e[0], e[1]));
+  for (auto& x : e) cudaEventDestroy(x);
+  if (ex) cudaGraphExecDestroy(ex);
+  launches_ = before;
+  return ms;
 }
 
 void GpuFactor::check_schedule() {
@@ -1334,120 +1393,113 @@ void GpuFactor::factor_model(int ncomp, const double* d_comp, const double* d_co
 void GpuFactor::solve(double* d_x, int64_t xstride, int B, int slot0) {
   if (B < 1 || slot0 < 0 || slot0 + B > max_batch_) throw std::runtime_error("batch size out of range");
   const int n = (int)sym_.n;
-  const int64_t fs = ftotal_;
-  const double* Fp = F_.p + (int64_t)slot0 * fs;
   dim3 gp(cdiv(n, 256) > 1024 ? 1024 : cdiv(n, 256), B);
-  auto pa = persist_at_.find(B);
-  // Follows the factorization's choice on trees of at least kSolvePersistLevels levels, where the level
-  // launches (up to three per level and direction) cost more than the waits of the persistent sweep:
-  // 169 against 187 us on 13 levels (n = 900), 450 / 519 on 28 (n = 10 000), 514 / 585 on 18 (group
-  // 24x24x14). One level of one 902-row front: 208 against 122, the launch's one CTA per SM having
-  // twice the loads in flight.
-  const bool per = solve_persist_ && (persist_mode_ == 2 || (pa != persist_at_.end() && pa->second &&
-                                                             levels_.size() >= kSolvePersistLevels));
-  if (per) {
-    launch_cached({3, B, (int64_t)(uintptr_t)d_x, xstride, slot0, 1}, [&] {
-      const int ns = (int)sym_.nsuper;
-      k_permute_in<<<gp, 256, 0, stream_>>>(n, d_perm_.p, d_x, xstride, xp_.p);
-      INLA_CUDA(cudaMemsetAsync(d_sstate_.p + 1, 0, sizeof(int) * (1 + 2 * (size_t)B * ns), stream_));
-      SolveArgs a;
-      a.S = ds_;
-      a.F = Fp;
-      a.fstride = fs;
-      a.B = B;
-      a.ngroups = solve_groups_;
-      a.gstart = d_sgstart_.p;
-      a.task = reinterpret_cast<const PersistTask*>(d_stask_.p);
-      a.tiny_list = d_stiny_.p;
-      a.linv = linv_.p + (int64_t)slot0 * ds_.lstride;
-      a.xp = xp_.p;
-      a.ub = ub_.p;
-      a.ustride = std::max<int64_t>(usum_, 1);
-      a.progf = d_sstate_.p + 2;
-      a.progb = d_sstate_.p + 2 + (size_t)B * ns;
-      a.head = reinterpret_cast<unsigned*>(d_sstate_.p + 1);
-      a.err = d_sstate_.p;
-      a.limit_ns = persist_limit_ns_;
-      k_solve_persist<<<solve_grid_, kPersistThreads, solve_smem_, stream_>>>(a);
-      k_permute_out<<<gp, 256, 0, stream_>>>(n, d_perm_.p, xp_.p, d_x, xstride);
-      launches_ += 3;
-    });
-    return;
-  }
-  launch_cached({3, B, (int64_t)(uintptr_t)d_x, xstride, slot0}, [&] {
+  auto pa = solve_persist_at_.find(B);
+  const bool per = solve_persist_ && (persist_mode_ == 2 || (pa != solve_persist_at_.end() && pa->second));
+  launch_cached({3, B, (int64_t)(uintptr_t)d_x, xstride, slot0, per}, [&] {
     k_permute_in<<<gp, 256, 0, stream_>>>(n, d_perm_.p, d_x, xstride, xp_.p);
-    ++launches_;
-    const int64_t us = std::max<int64_t>(usum_, 1);
-    const double* Lp = linv_.p + (int64_t)slot0 * ds_.lstride;
-    // fronts of up to kSmallB rows (contiguous lists small_a, small_b) in 32-column blocks by one
-    // CTA each; larger fronts in 64-column blocks with their cached inverse blocks
-    for (size_t li = 0; li < levels_.size(); ++li) {
-      const LevelPlan& P = levels_[li];
-      if (band_at_[li] >= 0) {
-        const MiniBand& M = bands_[band_at_[li]];
-        if ((int)li != M.l0) continue;
-        k_fwd_mini<<<dim3(cdiv(M.ntask, kMiniGroups), B), kMiniThreads, 0, stream_>>>(
-            ds_, mini_tables(M.off), M.ntask, Fp, fs, xp_.p, ub_.p, us);
-        ++launches_;
-        continue;
-      }
-      if (!P.tiny.empty()) {
-        const int nt = (int)P.tiny.size();
-        k_fwd_tiny<<<dim3(cdiv(nt, kTinySweepWarps), B), 32 * kTinySweepWarps, 0, stream_>>>(
-            ds_, d_lists_.p + P.off_tiny, nt, Fp, fs, xp_.p, ub_.p, us);
-        ++launches_;
-      }
-      const int nsm = (int)(P.small_a.size() + P.small_b.size());
-      if (nsm > 0) {
-        k_fwd32<128><<<dim3((unsigned)nsm, B), 128, (std::max(P.mmax_a, P.mmax_b) + 2 + 32 * 33) * 8, stream_>>>(
-            ds_, d_lists_.p + P.off_small_a, Fp, fs, xp_.p, ub_.p, us);
-        ++launches_;
-      }
-      if (!P.large.empty()) {
-        const dim3 g((unsigned)P.large.size(), B);
-        const int sm = (P.mmax_large + 2) * 8;
-        if ((int64_t)P.large.size() * B <= num_sms_)
-          k_fwd64<256, true><<<g, 256, sm, stream_>>>(ds_, d_lists_.p + P.off_large, Fp, fs, Lp, xp_.p, ub_.p, us);
-        else
-          k_fwd64<256, false><<<g, 256, sm, stream_>>>(ds_, d_lists_.p + P.off_large, Fp, fs, Lp, xp_.p, ub_.p, us);
-        ++launches_;
-      }
-    }
-    for (int l = (int)levels_.size() - 1; l >= 0; --l) {
-      const LevelPlan& P = levels_[l];
-      if (band_at_[l] >= 0) {
-        const MiniBand& M = bands_[band_at_[l]];
-        if (l != M.l0) continue;
-        k_bwd_mini<<<dim3(cdiv(M.ntask, kMiniGroups), B), kMiniThreads, 0, stream_>>>(
-            ds_, mini_tables(M.off), M.ntask, Fp, fs, xp_.p);
-        ++launches_;
-        continue;
-      }
-      if (!P.tiny.empty()) {
-        const int nt = (int)P.tiny.size();
-        k_bwd_tiny<<<dim3(cdiv(nt, kTinySweepWarps), B), 32 * kTinySweepWarps, 0, stream_>>>(
-            ds_, d_lists_.p + P.off_tiny, nt, Fp, fs, xp_.p);
-        ++launches_;
-      }
-      const int nsm = (int)(P.small_a.size() + P.small_b.size());
-      if (nsm > 0) {
-        k_bwd32<128><<<dim3((unsigned)nsm, B), 128, (std::max(P.mmax_a, P.mmax_b) + 2 + 32 * 33) * 8, stream_>>>(
-            ds_, d_lists_.p + P.off_small_a, Fp, fs, xp_.p);
-        ++launches_;
-      }
-      if (!P.large.empty()) {
-        const dim3 g((unsigned)P.large.size(), B);
-        const int sm = (P.mmax_large + 2) * 8;
-        if ((int64_t)P.large.size() * B <= num_sms_)
-          k_bwd64<256, true><<<g, 256, sm, stream_>>>(ds_, d_lists_.p + P.off_large, Fp, fs, Lp, xp_.p);
-        else
-          k_bwd64<256, false><<<g, 256, sm, stream_>>>(ds_, d_lists_.p + P.off_large, Fp, fs, Lp, xp_.p);
-        ++launches_;
-      }
-    }
+    if (per) solve_queue(B, slot0);
+    else solve_levels(B, slot0);
     k_permute_out<<<gp, 256, 0, stream_>>>(n, d_perm_.p, xp_.p, d_x, xstride);
-    ++launches_;
+    launches_ += 2;
   });
+}
+
+void GpuFactor::solve_queue(int B, int slot0) {
+  const int ns = (int)sym_.nsuper;
+  INLA_CUDA(cudaMemsetAsync(d_sstate_.p + 1, 0, sizeof(int) * (1 + 2 * (size_t)B * ns), stream_));
+  SolveArgs a;
+  a.S = ds_;
+  a.F = F_.p + (int64_t)slot0 * ftotal_;
+  a.fstride = ftotal_;
+  a.B = B;
+  a.ngroups = solve_groups_;
+  a.gstart = d_sgstart_.p;
+  a.task = reinterpret_cast<const PersistTask*>(d_stask_.p);
+  a.tiny_list = d_stiny_.p;
+  a.linv = linv_.p + (int64_t)slot0 * ds_.lstride;
+  a.xp = xp_.p;
+  a.ub = ub_.p;
+  a.ustride = std::max<int64_t>(usum_, 1);
+  a.progf = d_sstate_.p + 2;
+  a.progb = d_sstate_.p + 2 + (size_t)B * ns;
+  a.head = reinterpret_cast<unsigned*>(d_sstate_.p + 1);
+  a.err = d_sstate_.p;
+  a.limit_ns = persist_limit_ns_;
+  k_solve_persist<<<solve_grid_, kPersistThreads, solve_smem_, stream_>>>(a);
+  ++launches_;
+}
+
+// Fronts of up to kSmallB rows (contiguous lists small_a, small_b) in 32-column blocks by one CTA each;
+// larger fronts in 64-column blocks with their cached inverse blocks.
+void GpuFactor::solve_levels(int B, int slot0) {
+  const int64_t fs = ftotal_, us = std::max<int64_t>(usum_, 1);
+  const double* Fp = F_.p + (int64_t)slot0 * fs;
+  const double* Lp = linv_.p + (int64_t)slot0 * ds_.lstride;
+  for (size_t li = 0; li < levels_.size(); ++li) {
+    const LevelPlan& P = levels_[li];
+    if (band_at_[li] >= 0) {
+      const MiniBand& M = bands_[band_at_[li]];
+      if ((int)li != M.l0) continue;
+      k_fwd_mini<<<dim3(cdiv(M.ntask, kMiniGroups), B), kMiniThreads, 0, stream_>>>(
+          ds_, mini_tables(M.off), M.ntask, Fp, fs, xp_.p, ub_.p, us);
+      ++launches_;
+      continue;
+    }
+    if (!P.tiny.empty()) {
+      const int nt = (int)P.tiny.size();
+      k_fwd_tiny<<<dim3(cdiv(nt, kTinySweepWarps), B), 32 * kTinySweepWarps, 0, stream_>>>(
+          ds_, d_lists_.p + P.off_tiny, nt, Fp, fs, xp_.p, ub_.p, us);
+      ++launches_;
+    }
+    const int nsm = (int)(P.small_a.size() + P.small_b.size());
+    if (nsm > 0) {
+      k_fwd32<128><<<dim3((unsigned)nsm, B), 128, (std::max(P.mmax_a, P.mmax_b) + 2 + 32 * 33) * 8, stream_>>>(
+          ds_, d_lists_.p + P.off_small_a, Fp, fs, xp_.p, ub_.p, us);
+      ++launches_;
+    }
+    if (!P.large.empty()) {
+      const dim3 g((unsigned)P.large.size(), B);
+      const int sm = (P.mmax_large + 2) * 8;
+      if ((int64_t)P.large.size() * B <= num_sms_)
+        k_fwd64<256, true><<<g, 256, sm, stream_>>>(ds_, d_lists_.p + P.off_large, Fp, fs, Lp, xp_.p, ub_.p, us);
+      else
+        k_fwd64<256, false><<<g, 256, sm, stream_>>>(ds_, d_lists_.p + P.off_large, Fp, fs, Lp, xp_.p, ub_.p, us);
+      ++launches_;
+    }
+  }
+  for (int l = (int)levels_.size() - 1; l >= 0; --l) {
+    const LevelPlan& P = levels_[l];
+    if (band_at_[l] >= 0) {
+      const MiniBand& M = bands_[band_at_[l]];
+      if (l != M.l0) continue;
+      k_bwd_mini<<<dim3(cdiv(M.ntask, kMiniGroups), B), kMiniThreads, 0, stream_>>>(
+          ds_, mini_tables(M.off), M.ntask, Fp, fs, xp_.p);
+      ++launches_;
+      continue;
+    }
+    if (!P.tiny.empty()) {
+      const int nt = (int)P.tiny.size();
+      k_bwd_tiny<<<dim3(cdiv(nt, kTinySweepWarps), B), 32 * kTinySweepWarps, 0, stream_>>>(
+          ds_, d_lists_.p + P.off_tiny, nt, Fp, fs, xp_.p);
+      ++launches_;
+    }
+    const int nsm = (int)(P.small_a.size() + P.small_b.size());
+    if (nsm > 0) {
+      k_bwd32<128><<<dim3((unsigned)nsm, B), 128, (std::max(P.mmax_a, P.mmax_b) + 2 + 32 * 33) * 8, stream_>>>(
+          ds_, d_lists_.p + P.off_small_a, Fp, fs, xp_.p);
+      ++launches_;
+    }
+    if (!P.large.empty()) {
+      const dim3 g((unsigned)P.large.size(), B);
+      const int sm = (P.mmax_large + 2) * 8;
+      if ((int64_t)P.large.size() * B <= num_sms_)
+        k_bwd64<256, true><<<g, 256, sm, stream_>>>(ds_, d_lists_.p + P.off_large, Fp, fs, Lp, xp_.p);
+      else
+        k_bwd64<256, false><<<g, 256, sm, stream_>>>(ds_, d_lists_.p + P.off_large, Fp, fs, Lp, xp_.p);
+      ++launches_;
+    }
+  }
 }
 
 // Launches of the products of a level whose large fronts have at most kmax pivots and rmax rows below them,

@@ -209,6 +209,9 @@ class GpuFactor {
   const std::vector<char>* schedule(int B, const std::function<void()>& fill);
   void selinv_levels(int B, int slot0);
   void plan_persist();
+  void solve_levels(int B, int slot0);  // both sweeps of xp_, by level launches
+  void solve_queue(int B, int slot0);   // the same by the persistent launch
+  float time_graph(const std::function<void()>& body);
   void run_factor_persist(int B, const int* total_override = nullptr, long long limit_ns = 0,
                           const unsigned char* active = nullptr, int nseg = 1);
   template <class Body>
@@ -252,7 +255,8 @@ class GpuFactor {
   // persistent schedule
   bool persist_ = false;
   int persist_mode_ = 1;
-  std::map<int, bool> persist_at_;  // measured choice per batch size
+  std::map<int, bool> persist_at_;        // measured choices per batch size: factorization,
+  std::map<int, bool> solve_persist_at_;  // solve
   int persist_smem_ = 0, persist_grid_ = 0, persist_groups_ = 0;
   long long persist_limit_ns_ = 2000000000LL;
   DBuf<int> d_pgstart_, d_ptask_, d_ptiny_, d_ptotal_, d_pstate_;  // pstate: err, head, prog[B][ns], dprog[B][ns]
