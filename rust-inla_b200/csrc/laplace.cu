@@ -147,9 +147,14 @@ LaplaceEngine::LaplaceEngine(const LaplaceSpec& spec, int max_batch, cudaStream_
         atv[fill[aci[a]]++] = av[a];
       }
   }
-  // columns summed by a CTA of their own (k_newton_rhs, k_spmv_at), lanes per other column: a warp
-  // where a column has more than 48 entries on average (the dense augmented form), else 8 lanes
-  wide_cols_ = nnz_ + (int64_t)aci.size() > 48 * n;
+  // Columns summed by a CTA of their own (k_newton_rhs, k_spmv_at); the others by a warp each in models whose
+  // columns have many entries on average, else by 8 lanes. A warp's strided sum is shorter, but n warps for
+  // every four problems must not crowd out one another, so the line rises with n: 16 entries up to 800
+  // columns, n / 50 beyond, 128 from 6400 on. Right-hand side, 8 lanes / a warp, at B = 1, 7 and 20: n = 300,
+  // 18 entries 3.4 / 2.5, 4.6 / 3.4, 4.7 / 3.7 us; n = 2500, 50 entries 6.0 / 3.6, 8.7 / 8.4, 11.6 / 16.9; n = 5000,
+  // 98 entries 10.3 / 8.1, 24.9 / 23.8, 41 / 49; n = 14 000, 98 entries 15.8 / 20.5, 46 / 60, 95 / 129; n = 20 000,
+  // 122 entries at B = 1 and 7 39 / 37, 86 / 95. Fewer entries: n = 2500, 18 entries 3.5 / 2.9, 5.0 / 6.4, 5.9 / 12.1.
+  wide_cols_ = nnz_ + (int64_t)aci.size() > std::max<int64_t>(16, std::min<int64_t>(128, n / 50)) * n;
   std::vector<int> longc;
   for (int64_t j = 0; j < n; ++j)
     if ((spec_.colptr[j + 1] - spec_.colptr[j]) + (spec_.identity_a ? 0 : atp[j + 1] - atp[j]) >

@@ -67,9 +67,10 @@ __global__ void k_eval_lik(int fam, int64_t nobs, const double* __restrict__ eta
 // column such a column of 24 000 entries took 10 ms while the rest of the kernel took 0.05 ms. So
 // short columns are summed by L lanes each (strided entries, shuffle tree; NT = 256) and a column of
 // more than long_col(L) entries (host list `longc`) by a CTA of kLongThreads in a launch of its own
-// (L = 0). The split of a column depends on its own length only, so its sum does not depend on the
-// batch or on the other columns. What bounds a long column is the chain index -> x per entry, hence
-// 1024 threads for it (256: 105 us for group 24x24x14); two entries in flight per thread, four spill. With 8 lanes the
+// (L = 0). The split of a column depends on its own length and on L, which the model fixes
+// (LaplaceEngine::wide_cols_), so its sum does not depend on the batch. What bounds a long column is the
+// chain index -> x per entry, hence 1024 threads for it (256: 105 us for group 24x24x14); two entries in
+// flight per thread, four spill. With 8 lanes the
 // line lies at 128 entries: at 1024 the intercepts of models with 200 to 340 observations (600 to
 // 1024 entries) stayed with 8 lanes and set the kernel's time (226 us).
 // Group 24x24x14, B = 2: 10.4 ms -> 57 us; 96 uneven models, B = 2: 5.0 ms -> 96 us; SPDE 200^2, B = 7
