@@ -887,6 +887,8 @@ void GpuFactor::plan_solve_persist() {
   solve_persist_ = true;
 }
 
+constexpr int64_t kPersistPairs = 1 << 17;  // (large front, problem) pairs
+
 void GpuFactor::plan_persist() {
   int def = g_persist_default.load();
   if (def < 0) {
@@ -901,8 +903,10 @@ void GpuFactor::plan_persist() {
   PersistPlan pl;
   if (!make_persist_plan(sym_, levels_, pl)) return;  // a front too wide for the schedule's shared memory
   const int ns = (int)sym_.nsuper;
-  // (the limit of the former block cache, kept so that the same engines stay with level launches)
-  if ((size_t)std::max(pl.nlarge, 1) * max_batch_ * kB64 * kB64 * 8 > ((size_t)4 << 30)) return;
+  // With this many large fronts every step of a level fills the GPU, and the queue only adds its waits: 4400
+  // fronts of 100 rows at B = 30 35.1 ms by level launches, 54.2 ms persistent; 600 trees of seven fronts of 150
+  // and 300 rows at B = 32 170 and 266 ms. Not worth timing both.
+  if ((int64_t)pl.nlarge * max_batch_ > kPersistPairs) return;
   persist_groups_ = (int)pl.gstart.size() - 1;
   d_pgstart_.upload(pl.gstart, stream_);
   d_ptask_.upload(pl.task, stream_);
