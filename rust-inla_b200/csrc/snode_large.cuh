@@ -955,13 +955,10 @@ __device__ __forceinline__ void si_gemm_body(const DevSym& S, int s, int b, int 
     for (int q = 0; q < 2; ++q) acc[a][q][0] = acc[a][q][1] = 0.0;
   const int nc = (t1 - t0 + 31) / 32;
   load_chunk(t0, 0);
-  if (kSiStages > 2 && nc > 1) load_chunk(t0 + 32, 1);
   for (int c = 0; c < nc; ++c) {
-    if (kSiStages > 2 && c + 1 < nc) cp_async_wait<1>();
-    else cp_async_wait<0>();
+    cp_async_wait<0>();
     __syncthreads();  // chunk c has landed, and every warp is done with chunk c - 1
-    constexpr int kAhead = kSiStages - 1;
-    if (c + kAhead < nc) load_chunk(t0 + 32 * (c + kAhead), (c + kAhead) % kSiStages);
+    if (c + 1 < nc) load_chunk(t0 + 32 * (c + 1), (c + 1) % kSiStages);
     const double* As = smem64 + (c % kSiStages) * kBuf;
     const double* Bs = As + 32 * ld;
     if (wact) {
