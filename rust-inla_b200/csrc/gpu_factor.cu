@@ -337,10 +337,8 @@ GpuFactor::GpuFactor(const Symbolic& sym, int max_batch, cudaStream_t stream)
   }
 
   // the look-ahead form needs its stream where a large front has more than one block of pivots
-  if (std::any_of(levels_.begin(), levels_.end(), [](const LevelPlan& P) { return P.kmax_large > kB64; })) {
-    INLA_CUDA(cudaStreamCreateWithFlags(&chain_stream_, cudaStreamNonBlocking));
-    for (auto& e : chain_ev_) INLA_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-  }
+  if (std::any_of(levels_.begin(), levels_.end(), [](const LevelPlan& P) { return P.kmax_large > kB64; }))
+    chain_.create();
   panel_form_ = g_panel_form.load();
   plan_persist();
   const auto ta = std::chrono::steady_clock::now();
@@ -415,9 +413,6 @@ GpuFactor::GpuFactor(const Symbolic& sym, int max_batch, cudaStream_t stream)
 }
 
 GpuFactor::~GpuFactor() {
-  for (auto& e : chain_ev_)
-    if (e) cudaEventDestroy(e);
-  if (chain_stream_) cudaStreamDestroy(chain_stream_);
   for (auto& kv : graphs_) cudaGraphExecDestroy(kv.second.exec);
 }
 
@@ -1170,15 +1165,15 @@ void GpuFactor::run_factor_levels(int B, const std::vector<char>* fuse, cudaEven
           }
           const bool next = j0 + kB64 < P.kmax_large;
           if (next) {
-            INLA_CUDA(cudaEventRecord(chain_ev_[0], stream_));
-            INLA_CUDA(cudaStreamWaitEvent(chain_stream_, chain_ev_[0], 0));
-            k_diag_next<<<dim3(nl, B), 256, kPanelSmem, chain_stream_>>>(ds_, lst, j0 + kB64, F_.p, fs, linv_.p);
-            INLA_CUDA(cudaEventRecord(chain_ev_[1], chain_stream_));
+            INLA_CUDA(cudaEventRecord(chain_.fork, stream_));
+            INLA_CUDA(cudaStreamWaitEvent(chain_.stream, chain_.fork, 0));
+            k_diag_next<<<dim3(nl, B), 256, kPanelSmem, chain_.stream>>>(ds_, lst, j0 + kB64, F_.p, fs, linv_.p);
+            INLA_CUDA(cudaEventRecord(chain_.join, chain_.stream));
             ++launches_;
           }
           k_rows64<<<dim3(nl, B, nrb), 256, kRowsSmem, stream_>>>(ds_, lst, j0, F_.p, fs, nullptr, linv_.p);
           k_update64w8<<<ug, 256, kPersistUpdSmem, stream_>>>(ds_, lst, j0, F_.p, fs, nullptr);
-          if (next) INLA_CUDA(cudaStreamWaitEvent(stream_, chain_ev_[1], 0));
+          if (next) INLA_CUDA(cudaStreamWaitEvent(stream_, chain_.join, 0));
           launches_ += 2;
           continue;
         }

@@ -79,6 +79,26 @@ struct LevelPlan {
   int off_si_tiny = 0, off_si_small = 0, off_si_large = 0, mmax_si_small = 0, kmax_si_small = 0, kmax_si_large = 0, mmax_si_large = 0, rmax_si_large = 0;
 };
 
+// A stream and the events that fork it from the engine's stream and join it (destroyed also when the engine's
+// constructor throws after create()).
+struct ChainStream {
+  cudaStream_t stream = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
+  ChainStream() = default;
+  ChainStream(const ChainStream&) = delete;
+  ChainStream& operator=(const ChainStream&) = delete;
+  ~ChainStream() {
+    if (join) cudaEventDestroy(join);
+    if (fork) cudaEventDestroy(fork);
+    if (stream) cudaStreamDestroy(stream);
+  }
+  void create() {
+    INLA_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+    INLA_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
+    INLA_CUDA(cudaEventCreateWithFlags(&join, cudaEventDisableTiming));
+  }
+};
+
 // Consecutive levels [l0, l1) whose fronts all have at most kMiniM rows: tasks off .. off + ntask of the
 // mini task table (snode_mini.cuh).
 struct MiniBand {
@@ -260,8 +280,7 @@ class GpuFactor {
   int persist_smem_ = 0, persist_grid_ = 0, persist_groups_ = 0;
   long long persist_limit_ns_ = 2000000000LL;
   DBuf<int> d_pgstart_, d_ptask_, d_ptiny_, d_ptotal_, d_pstate_;  // pstate: err, head, prog[B][ns], dprog[B][ns]
-  cudaStream_t chain_stream_ = nullptr;  // pivot chain of the look-ahead form, joined with stream_
-  cudaEvent_t chain_ev_[2] = {nullptr, nullptr};
+  ChainStream chain_;  // pivot chain of the look-ahead form, joined with stream_
   int panel_form_ = -1;  // forced panel form (set_panel_form at construction), -1 autotuned
   DBuf<int> d_fseg_;
   // persistent solve
