@@ -437,21 +437,6 @@ def factor_roofline(p, torch, B=21, reps=10):
     return {"flops_per_launch": flops * B, "ms": ms, "nnz_l": int(s.info()["nnz_l"]), "B": B}
 
 
-TRAFFIC_SUMMARY = Path(__file__).resolve().parent / "profiles" / "traffic_factor_spde200.md"
-
-
-def factor_traffic(B):
-    """DRAM bytes (read + write) of one batched factorization of B problems, from the committed
-    ncu summary (per-problem figure of a smaller capture; batch members use disjoint buffers)."""
-    try:
-        for line in TRAFFIC_SUMMARY.read_text().splitlines():
-            if line.startswith("dram_bytes_per_problem:"):
-                return int(line.split(":")[1]) * B, f"{TRAFFIC_SUMMARY.name} (per-problem DRAM bytes x {B})"
-    except OSError:
-        pass
-    return None, "no ncu traffic summary"
-
-
 def run_ours(args, ws, rank, local, dist):
     import torch
 
@@ -555,13 +540,13 @@ def run_ours(args, ws, rank, local, dist):
     fr = factor_roofline(p, torch, B=10)
     fr21 = factor_roofline(p, torch, B=21)
     achieved = fr["flops_per_launch"] / (fr["ms"] * 1e-3) / 1e12
-    traffic, tsrc = factor_traffic(fr["B"])
     roof = {"bound": "tensor",
             "kernel": "batched supernodal LDL^T at the fit's batch size (B=10 theta-points, nested dissection; "
                       "the schedule the engine picks for that size)",
             "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
             "peak_source": "cuBLAS DGEMM 8192^3 measured in this run (FP64; the measured-peaks file has no FP64 entry)",
-            "traffic": traffic, "traffic_source": tsrc, "ms_per_launch": fr["ms"],
+            "traffic": None, "traffic_source": "not measured (needs counters over every launch of the sequence)",
+            "ms_per_launch": fr["ms"],
             "flops_per_launch": fr["flops_per_launch"],
             "b21": {"ms_per_launch": fr21["ms"], "achieved": fr21["flops_per_launch"] / (fr21["ms"] * 1e-3) / 1e12,
                     "frac": fr21["flops_per_launch"] / (fr21["ms"] * 1e-3) / 1e12 / peak}}
