@@ -64,7 +64,7 @@ __device__ __forceinline__ void bar_arrive_id(int id, int threads) {
 // lies within one unit of the correctly rounded 1 / d (measured over two million mantissas: 0.03 % differ, the
 // worst is 0.506 units off). Outside the range y may be flushed; warp_ldlt8 then
 // repeats the block with 1.0 / d. With 1.0 / d throughout the 64 x 64 block of cta_ldlt takes 14.9 k cycles with
-// the inverse and 13.3 k without, with this 13.3 k and 11.9 k.
+// the inverse and 13.3 k without, with this 13.6 k and 11.4 k.
 __device__ __forceinline__ double rcp_straight(double d) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
@@ -74,6 +74,43 @@ __device__ __forceinline__ double rcp_straight(double d) {
 
 __device__ __forceinline__ bool rcp_in_range(double d) {  // by the high word of |d|
   return (unsigned)(__double2hiint(d) & 0x7fffffff) - 0x01700000u < 0x7d000000u;
+}
+
+// One warp: what warp_ldlt8 leaves in A, Lam and di, with 1.0 / d for every pivot, from the copy of the block
+// that Lam holds. Rarely taken, so it works in shared memory, lane i on row i (then on column i of L^-1),
+// and is a call: unrolled beside the fast pass it spills in k_panel64 and k_diag_next (5 to 7 % slower).
+__device__ __noinline__ void warp_ldlt8_div(double* A, int lda, int w, double* Lam, double* di) {
+  const int lane = threadIdx.x & 31;
+  if (lane < 8)
+    for (int j = 0; j <= lane; ++j)
+      if (lane >= w) Lam[lane + j * kLam8Ld] = lane == j ? 1.0 : 0.0;
+  __syncwarp();
+#pragma unroll 1
+  for (int p = 0; p < 8; ++p) {
+    const double r = 1.0 / Lam[p + p * kLam8Ld];
+    const bool below = lane > p && lane < 8;
+    const double l = below ? Lam[lane + p * kLam8Ld] * r : 0.0;
+    if (below)
+#pragma unroll 1
+      for (int j = p + 1; j <= lane; ++j) Lam[lane + j * kLam8Ld] -= l * Lam[j + p * kLam8Ld];
+    __syncwarp();
+    if (below) Lam[lane + p * kLam8Ld] = l;
+    if (lane == 0) di[p] = r;
+    if (lane >= p && lane < w) A[lane + p * lda] = lane == p ? Lam[p + p * kLam8Ld] : l;
+    __syncwarp();
+  }
+  double x[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    x[i] = i == lane ? 1.0 : 0.0;
+#pragma unroll
+    for (int p = 0; p < i; ++p) x[i] -= Lam[i + p * kLam8Ld] * x[p];
+  }
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    if (lane < 8) Lam[i + lane * kLam8Ld] = x[i];
+  __syncwarp();
 }
 
 // One warp: LDL^T and inverse of the w x w (w <= 8) leading block of A (shared memory, column-major,
@@ -97,16 +134,13 @@ __device__ __forceinline__ void warp_ldlt8(double* A, int lda, int w, double* La
       if (i >= j) a[i][j] = v.x;
       a[i + 1][j] = v.y;
     }
-  auto pad = [&] {
-    if (w < 8) {
+  if (w < 8) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j)
+    for (int j = 0; j < 8; ++j)
 #pragma unroll
-        for (int i = j; i < 8; ++i)
-          if (i >= w) a[i][j] = (i == j) ? 1.0 : 0.0;
-    }
-  };
-  pad();
+      for (int i = j; i < 8; ++i)
+        if (i >= w) a[i][j] = (i == j) ? 1.0 : 0.0;
+  }
   // the block as it came, for a second pass (A is overwritten as the columns are finished)
   Lam[g + tg * kLam8Ld] = A[g + tg * lda];
   Lam[g + (tg + 4) * kLam8Ld] = A[g + (tg + 4) * lda];
@@ -116,42 +150,36 @@ __device__ __forceinline__ void warp_ldlt8(double* A, int lda, int w, double* La
   double x0[8], x1[4];
   const int lim = lane == 0 ? w : 0;
   bool in_range = true;
-  auto eliminate = [&](auto rcp) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) x0[i] = (i == tg) ? 1.0 : 0.0;
+  for (int i = 0; i < 8; ++i) x0[i] = (i == tg) ? 1.0 : 0.0;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) x1[i] = (i == tg) ? 1.0 : 0.0;
+  for (int i = 0; i < 4; ++i) x1[i] = (i == tg) ? 1.0 : 0.0;
 #pragma unroll
-    for (int p = 0; p < 8; ++p) {
-      in_range = in_range && rcp_in_range(a[p][p]);
-      const double r = rcp(a[p][p]);
-      if (lane == 0) di[p] = r;
-      if (p < lim) A[p + p * lda] = a[p][p];
-      double l[8];
+  for (int p = 0; p < 8; ++p) {
+    in_range = in_range && rcp_in_range(a[p][p]);
+    const double r = rcp_straight(a[p][p]);
+    if (lane == 0) di[p] = r;
+    if (p < lim) A[p + p * lda] = a[p][p];
+    double l[8];
 #pragma unroll
-      for (int i = p + 1; i < 8; ++i) l[i] = a[i][p] * r;
+    for (int i = p + 1; i < 8; ++i) l[i] = a[i][p] * r;
 #pragma unroll
-      for (int j = p + 1; j < 8; ++j)
+    for (int j = p + 1; j < 8; ++j)
 #pragma unroll
-        for (int i = j; i < 8; ++i) a[i][j] -= l[i] * a[j][p];
+      for (int i = j; i < 8; ++i) a[i][j] -= l[i] * a[j][p];
 #pragma unroll
-      for (int i = p + 1; i < 8; ++i) {
-        if (i < lim) A[i + p * lda] = l[i];
-        x0[i] -= l[i] * x0[p];
-        if (p >= 4) x1[i - 4] -= l[i] * x1[p - 4];
-      }
+    for (int i = p + 1; i < 8; ++i) {
+      if (i < lim) A[i + p * lda] = l[i];
+      x0[i] -= l[i] * x0[p];
+      if (p >= 4) x1[i - 4] -= l[i] * x1[p - 4];
     }
-  };
-  eliminate([](double d) { return rcp_straight(d); });
+  }
   if (!in_range) {  // every lane alike
     __syncwarp();
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-#pragma unroll
-      for (int i = j; i < 8; ++i) a[i][j] = Lam[i + j * kLam8Ld];
-    pad();
-    eliminate([](double d) { return 1.0 / d; });
-    __syncwarp();  // the block in Lam has been read
+    warp_ldlt8_div(A, lda, w, Lam, di);
+    lam0 = Lam[g + tg * kLam8Ld];
+    lam1 = Lam[g + (tg + 4) * kLam8Ld];
+    return;
   }
   lam0 = x0[0];
   lam1 = 0.0;
@@ -205,7 +233,7 @@ __device__ __forceinline__ void warp_trinv16(const double* L, int ldl, int w, do
 // trailing tiles while the pivot warp is already in the next block. What bounds it is the pivot
 // warp's chain. Lam and 1 / d are double-buffered: they are overwritten two blocks later, after a
 // barrier that every reader has passed.
-// Measured for a 64 x 64 block with its inverse, one CTA of 256 threads: 13.3 k cycles (11.9 k without the
+// Measured for a 64 x 64 block with its inverse, one CTA of 256 threads: 13.6 k cycles (11.4 k without the
 // inverse); the 16-wide form it replaces (one warp factoring 16 x 16 with the others waiting, three barriers
 // per block): 32.7 k (25.5 k).
 template <bool kInv>
