@@ -952,10 +952,13 @@ void GpuFactor::run_factor_persist(int B, const int* total_override, long long l
 }
 
 // Persistent or level launches for batch size B: fixed by the mode, or measured on the
-// first factorization at B (the level sequence in its tuned form and the persistent launch,
-// each after a warm-up, with CUDA events on the engine's stream) and kept for the structure
-// and B. Where the factorization is persistent, the triangular solve's two schedules are timed in
-// the same way, each as the graph it runs as: which is faster depends on the tree, not on its depth alone.
+// first factorization at B (the level sequence in its tuned form and the persistent launch, with their
+// value fills, each after a warm-up as the graph it runs as, with CUDA events on the engine's stream) and
+// kept for the structure and B. Launched directly, a level sequence takes longer than its graph: the grouped
+// model 24x24x14 at B = 2 1.69 ms against 1.67 persistent, and the evaluation 22.0 ms persistent, 21.2 by
+// level launches; binary trees of dense blocks lost up to 13 % by that.
+// Where the factorization is persistent, the triangular solve's two schedules are timed in
+// the same way: which is faster depends on the tree, not on its depth alone.
 // Level launches / persistent: 13 levels (n = 900, AMD) 187 / 169 us, 28 levels (n = 10 000, AMD) 519 / 450, 3-D
 // grid of 22^3 350 / 336, but 2-D grids of 60^2 and 300^2 under nested dissection 193 / 224 and 488 / 607, binary
 // trees of dense 60-column blocks, 3 / 5 / 7 / 8 levels, 41 / 52, 69 / 83, 223 / 302, 513 / 776.
@@ -973,25 +976,14 @@ bool GpuFactor::use_persist(int B, const std::function<void()>& fill) {
     }
   }
   const std::vector<char>* pol = schedule(B, fill);
-  cudaEvent_t e[4];
-  for (auto& x : e) INLA_CUDA(cudaEventCreate(&x));
-  fill();
-  run_factor_levels(B, pol);  // warm-up
-  fill();
-  INLA_CUDA(cudaEventRecord(e[0], stream_));
-  run_factor_levels(B, pol);
-  INLA_CUDA(cudaEventRecord(e[1], stream_));
-  fill();
-  run_factor_persist(B);  // warm-up
-  fill();
-  INLA_CUDA(cudaEventRecord(e[2], stream_));
-  run_factor_persist(B);
-  INLA_CUDA(cudaEventRecord(e[3], stream_));
-  INLA_CUDA(cudaStreamSynchronize(stream_));
-  float tl = 0.f, tp = 0.f;
-  INLA_CUDA(cudaEventElapsedTime(&tl, e[0], e[1]));
-  INLA_CUDA(cudaEventElapsedTime(&tp, e[2], e[3]));
-  for (auto& x : e) cudaEventDestroy(x);
+  const float tl = time_graph([&] {
+    fill();
+    run_factor_levels(B, pol);
+  });
+  const float tp = time_graph([&] {
+    fill();
+    run_factor_persist(B);
+  });
   const bool pick = tp < tl;
   bool pick_solve = false;
   if (pick && solve_persist_) {
